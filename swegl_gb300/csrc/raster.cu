@@ -107,14 +107,12 @@ __global__ void k_world(SceneDev s)
     const float4 q = s.nrm_v[g];
     const V3 w = transform3(mk3(p.x, p.y, p.z), M);
     const V3 nw = normalize3(normalize3(rotate_n(mk3(q.x, q.y, q.z), RS)));
-    s.wpos[g] = make_float4(w.x, w.y, w.z, 0.0f);
-    s.wnrm[g] = make_float4(nw.x, nw.y, nw.z, 0.0f);
-    s.uv[g] = make_float2(p.w, q.w);
+    s.wpos[g] = make_float4(w.x, w.y, w.z, p.w);
+    s.wnrm[g] = make_float4(nw.x, nw.y, nw.z, q.w);
 }
 
 // k_world for one posed request: the same transforms under the request's
-// node matrices, into its own arrays (texture coordinates are pose-free and
-// stay the scene's).
+// node matrices, into its own arrays.
 __global__ void k_pose(SceneDev s, const float *node_world, const float *node_rs, float4 *wpos, float4 *wnrm)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -125,8 +123,8 @@ __global__ void k_pose(SceneDev s, const float *node_world, const float *node_rs
     const float4 q = s.nrm_v[g];
     const V3 w = transform3(mk3(p.x, p.y, p.z), node_world + 16 * n);
     const V3 nw = normalize3(normalize3(rotate_n(mk3(q.x, q.y, q.z), node_rs + 16 * n)));
-    wpos[g] = make_float4(w.x, w.y, w.z, 0.0f);
-    wnrm[g] = make_float4(nw.x, nw.y, nw.z, 0.0f);
+    wpos[g] = make_float4(w.x, w.y, w.z, p.w);
+    wnrm[g] = make_float4(nw.x, nw.y, nw.z, q.w);
 }
 
 // The box of each primitive's world positions (a warp per primitive), for the
@@ -1677,10 +1675,9 @@ __device__ __forceinline__ void load_tv(const ItemDev &it, uint32_t g, TV &o)
     o.world = mk3(w.x, w.y, w.z);
     const float4 nv = it.s.nrm_v[g];
     o.normal = mk3(nv.x, nv.y, nv.z);
-    const float2 uv = it.s.uv[g];
-    o.uv = mk2(uv.x, uv.y);
     const float4 nw = it.s.wnrm[g];
     o.nworld = mk3(nw.x, nw.y, nw.z);
+    o.uv = mk2(w.w, nw.w);
 }
 
 // world_to_viewport (vertex_shaders.hpp:54-59) of a near-clip vertex
@@ -1915,19 +1912,10 @@ __device__ __forceinline__ void bind_material(const SceneDev &s, uint32_t prim, 
     sh.shininess = (int)c.y;
 }
 
-// prepare_for_upper/lower_triangle, prepare_for_scanline and shade for the
-// winner's progress values (renderer.cpp:433-493)
-template <bool ALL_MODES = true>
-__device__ __forceinline__ uint32_t shade_winner(Shader &sh, const LightsDev &L, const ViewDev &v, float4 rec)
+// Whether a pixel shader's light is per triangle (pixel_shader_lights_flat).
+__device__ __forceinline__ bool flat_mode(int shader)
 {
-    const uint32_t bits = __float_as_uint(rec.w);
-    const bool llr = (bits & kBitLLR) != 0u;
-    if (bits & kBitLower)
-        sh_prepare_lower(sh, llr);
-    else
-        sh_prepare_upper(sh, llr);
-    sh_prepare_scanline(sh, rec.y, rec.z);
-    return sh_shade<ALL_MODES>(sh, L, v, rec.x);
+    return shader == SGL_SHADER_FLAT_BILINEAR || shader == SGL_SHADER_FLAT_NEAREST || shader == SGL_SHADER_FLAT;
 }
 
 // A winner of a near-clipped triangle: the clip vertices are rebuilt exactly
@@ -1944,18 +1932,24 @@ __device__ __noinline__ uint32_t shade_clip_rec(const ItemDev &it, uint32_t slot
         if (p1->vp.y < p0->vp.y) { t = p0; p0 = p1; p1 = t; }
         if (p2->vp.y < p1->vp.y) { t = p1; p1 = p2; p2 = t; }
         if (p1->vp.y < p0->vp.y) { t = p0; p0 = p1; p1 = t; }
-        const V3 sw[3] = {p0->world, p1->world, p2->world};
-        const V3 sn[3] = {p0->nworld, p1->nworld, p2->nworld};
-        const V2 su[3] = {p0->uv, p1->uv, p2->uv};
         bind_material(it.s, it.s.tris[slot >> 1].w, sh);
-        sh_prepare_triangle(sh, sw, sn, su, !ffv);
-        if (it.v.shader == SGL_SHADER_FLAT_BILINEAR || it.v.shader == SGL_SHADER_FLAT_NEAREST ||
-            it.v.shader == SGL_SHADER_FLAT)
+        const uint32_t bits = __float_as_uint(rec.w);
+        const bool lower = (bits & kBitLower) != 0u;
+        uint32_t is, il, ir;
+        sh_edge_ends(lower, (bits & kBitLLR) != 0u, 0u, 1u, 2u, is, il, ir);
+        auto vert = [&](uint32_t k) {
+            const TV *p = k == 0u ? p0 : (k == 1u ? p1 : p2);
+            return SVert{p->world, p->nworld, p->uv};
+        };
+        sh_fragment(sh, vert(is), vert(il), vert(ir), lower, !ffv, rec.y, rec.z, rec.x);
+        if (flat_mode(it.v.shader)) {
+            const V3 sw[3] = {p0->world, p1->world, p2->world};
             sh.flat_light = flat_light(sw, !ffv, *it.s.lights, it.v, sh.shininess);
+        }
         done = true;
     };
     clip_triangle(it, slot >> 1, emit);
-    return done ? shade_winner(sh, *it.s.lights, it.v, rec) : 0u;
+    return done ? sh_shade(sh, *it.s.lights, it.v) : 0u;
 }
 
 __device__ __forceinline__ uint32_t shade_clip_px(const ItemDev &it, uint32_t i, uint32_t slot)
@@ -2024,6 +2018,12 @@ __device__ __forceinline__ uint32_t shade_winner_impl(const BatchDev *b, uint32_
     return shade_rec<ALL_MODES>(it, q7, flags, rec);
 }
 
+__device__ __forceinline__ SVert load_svert(const ItemDev &it, uint32_t g)
+{
+    const float4 w = it.s.wpos[g], n = it.s.wnrm[g];
+    return SVert{mk3(w.x, w.y, w.z), mk3(n.x, n.y, n.z), mk2(w.w, n.w)};
+}
+
 // The colour of a fragment of a set-up triangle (vertices and primitive
 // `q7`, TriRec flags `flags`) at the progress values `rec`.
 template <bool ALL_MODES>
@@ -2032,20 +2032,19 @@ __device__ __forceinline__ uint32_t shade_rec(const ItemDev &it, uint4 q7, uint3
     const ViewDev &v = it.v;
     Shader sh;
     bind_material(it.s, q7.w, sh);
-    const float4 w0 = it.s.wpos[q7.x], w1 = it.s.wpos[q7.y], w2 = it.s.wpos[q7.z];
-    const float4 n0 = it.s.wnrm[q7.x], n1 = it.s.wnrm[q7.y], n2 = it.s.wnrm[q7.z];
-    const float2 u0 = it.s.uv[q7.x], u1 = it.s.uv[q7.y], u2 = it.s.uv[q7.z];
-    const V3 sw[3] = {mk3(w0.x, w0.y, w0.z), mk3(w1.x, w1.y, w1.z), mk3(w2.x, w2.y, w2.z)};
-    const V3 sn[3] = {mk3(n0.x, n0.y, n0.z), mk3(n1.x, n1.y, n1.z), mk3(n2.x, n2.y, n2.z)};
-    const V2 su[3] = {mk2(u0.x, u0.y), mk2(u1.x, u1.y), mk2(u2.x, u2.y)};
-    sh_prepare_triangle(sh, sw, sn, su, (flags & kRecFFV) == 0u);
-    if (ALL_MODES &&
-        (v.shader == SGL_SHADER_FLAT_BILINEAR || v.shader == SGL_SHADER_FLAT_NEAREST || v.shader == SGL_SHADER_FLAT))
-        sh.flat_light = flat_light(sw, (flags & kRecFFV) == 0u, *it.s.lights, v, sh.shininess);
-    return shade_winner<ALL_MODES>(sh, *it.s.lights, v, rec);
+    const uint32_t bits = __float_as_uint(rec.w);
+    const bool lower = (bits & kBitLower) != 0u, llr = (bits & kBitLLR) != 0u, inverted = (flags & kRecFFV) == 0u;
+    uint32_t is, il, ir;
+    sh_edge_ends(lower, llr, q7.x, q7.y, q7.z, is, il, ir);
+    const SVert s = load_svert(it, is), l = load_svert(it, il), r = load_svert(it, ir);
+    sh_fragment(sh, s, l, r, lower, inverted, rec.y, rec.z, rec.x);
+    if (ALL_MODES && flat_mode(v.shader)) {
+        const V3 v1 = llr ? l.p : r.p, o = llr ? r.p : l.p;
+        const V3 sw[3] = {lower ? o : s.p, v1, lower ? s.p : o};
+        sh.flat_light = flat_light(sw, inverted, *it.s.lights, v, sh.shininess);
+    }
+    return sh_shade<ALL_MODES>(sh, *it.s.lights, v);
 }
-
-
 
 // Per pixel: the background of viewport_t::clear (viewport.cpp:88-113) or the
 // colour of the winning fragment, and its depth.  A block takes TILE x TILE

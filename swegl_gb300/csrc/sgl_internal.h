@@ -74,9 +74,8 @@ struct SceneDev {
     const float *node_world; // 16 floats per node
     const float *node_rs;    // 16 floats per node
     const LightsDev *lights;
-    float4 *wpos;            // v_world
-    float4 *wnrm;            // normal_world
-    float2 *uv;              // tex_coords
+    float4 *wpos;            // v_world, and tex_coords u in w
+    float4 *wnrm;            // normal_world, and tex_coords v in w
     const uint4 *pgeo;       // draw-order primitives: first vertex, vertex count, first triangle, triangle count
     const PrimShade *pshade; // draw-order primitives: material and texture as the pixel shader binds them
     uint32_t n_vertices;

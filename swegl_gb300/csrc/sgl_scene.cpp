@@ -406,7 +406,6 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     CUDA_TRY(upload(d_pshade, pshade.data(), pshade.size()));
     CUDA_TRY(d_wpos.ensure(sizeof(float4) * std::max<size_t>(n_vertices, 1)));
     CUDA_TRY(d_wnrm.ensure(sizeof(float4) * std::max<size_t>(n_vertices, 1)));
-    CUDA_TRY(d_uv.ensure(sizeof(float2) * std::max<size_t>(n_vertices, 1)));
     dev = SceneDev{};
     dev.pos_u = (const float4 *)d_pos_u.ptr;
     dev.nrm_v = (const float4 *)d_nrm_v.ptr;
@@ -417,7 +416,6 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     dev.texs = (const TexDesc *)d_texs.ptr;
     dev.wpos = (float4 *)d_wpos.ptr;
     dev.wnrm = (float4 *)d_wnrm.ptr;
-    dev.uv = (float2 *)d_uv.ptr;
     dev.pgeo = (const uint4 *)d_pgeo.ptr;
     dev.pshade = (const PrimShade *)d_pshade.ptr;
     dev.n_prims = (uint32_t)pgeo.size();
@@ -461,7 +459,7 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     if (st != SGL_OK)
         return st;
     device_bytes = d_pos_u.bytes + d_nrm_v.bytes + d_vnode.bytes + d_tris.bytes + d_prims.bytes + d_mats.bytes +
-                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_uv.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes;
+                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes;
     return SGL_OK;
 }
 

@@ -12,99 +12,74 @@
 
 namespace sgl {
 
-// The state of pixel_shader_light_and_texture<lights_phong, texture_bilinear>
-// (swegl/render/pixel_shaders.hpp:76-97,125-150,121-179).
+// What the pixel shaders read at one fragment: the state that
+// pixel_shader_light_and_texture<lights_phong, texture_bilinear>
+// (swegl/render/pixel_shaders.hpp:76-97,125-150,121-179) carries along a span,
+// evaluated at the fragment (sh_fragment), and what bind_material binds.
 struct Shader {
-    V3 v0, v1, v2, n0, n1, n2;
-    V3 vleft, vright, vleftdir, vrightdir, nleft, nright, nleftdir, nrightdir;
-    V3 v, vdir, n, ndir;
-    V2 t0, t1, t2, side_long_t_dir, side_short_t, side_short_t_dir, t_left, t_dir;
-    bool llr;
+    V3 center, n; // position, and normal before its normalisation
+    V2 t;         // texture coordinates in texels
     const uint32_t *tex;
     uint32_t color;
     int tw, th, shininess;
     int flat_light; // pixel_shader_lights_flat::light as shade() returns it
 };
 
-// pixel_shader_*::prepare_for_triangle (src/render/pixel_shaders.cpp:88-105,304-318)
-__device__ __forceinline__ void sh_prepare_triangle(Shader &sh, const V3 w[3], const V3 n[3], const V2 uv[3],
-                                                    bool inverted)
+// One vertex as the pixel shaders read it.
+struct SVert {
+    V3 p, n;
+    V2 uv;
+};
+
+// Which of a triangle's vertices (v0, v1, v2 in fill_triangle_2's order) the
+// two edges of a span of half `lower` run between: both edges share vertex s
+// (v0 in the upper half, v2 in the lower one); the other end of the left edge
+// is l, of the right edge r.  The long edge v0 -> v2 is the right one when
+// `llr`.
+__device__ __forceinline__ void sh_edge_ends(bool lower, bool llr, uint32_t g0, uint32_t g1, uint32_t g2, uint32_t &s,
+                                             uint32_t &l, uint32_t &r)
 {
-    sh.v0 = w[0];
-    sh.v1 = w[1];
-    sh.v2 = w[2];
-    if (!inverted) {
-        sh.n0 = n[0];
-        sh.n1 = n[1];
-        sh.n2 = n[2];
-    } else {
-        sh.n0 = neg3(n[0]);
-        sh.n1 = neg3(n[1]);
-        sh.n2 = neg3(n[2]);
+    s = lower ? g2 : g0;
+    const uint32_t o = lower ? g0 : g2; // the long edge's other end
+    l = llr ? g1 : o;
+    r = llr ? o : g1;
+}
+
+__device__ __forceinline__ V3 sel3(bool c, V3 a, V3 b) { return mk3(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z); }
+__device__ __forceinline__ V2 sel2(bool c, V2 a, V2 b) { return mk2(c ? a.x : b.x, c ? a.y : b.y); }
+
+// prepare_for_triangle, prepare_for_upper/lower_triangle, prepare_for_scanline
+// (src/render/pixel_shaders.cpp:88-158,304-346) and the interpolation of
+// shade(): position, normal and texture coordinates run along the left edge
+// to progress pl, along the right edge to pr, and between the two to
+// `progress`, each as start + (end - start) * progress.  Both lower edges end
+// at s, both upper ones start there.  The reference negates the three normals
+// of an `inverted` triangle before interpolating; every step commutes with
+// that sign, so it is taken at the end.
+__device__ __forceinline__ void sh_fragment(Shader &sh, const SVert &s, const SVert &l, const SVert &r, bool lower,
+                                            bool inverted, float pl, float pr, float progress)
+{
+    {
+        const V3 a = sel3(lower, l.p, s.p), b = sel3(lower, s.p, l.p);
+        const V3 c = sel3(lower, r.p, s.p), d = sel3(lower, s.p, r.p);
+        const V3 v = add3(a, mul3(sub3(b, a), pl));
+        sh.center = add3(v, mul3(sub3(add3(c, mul3(sub3(d, c), pr)), v), progress));
     }
-    const float tw = (float)sh.tw, th = (float)sh.th;
-    sh.t0 = mk2(uv[0].x * tw, uv[0].y * th);
-    sh.t1 = mk2(uv[1].x * tw, uv[1].y * th);
-    sh.t2 = mk2(uv[2].x * tw, uv[2].y * th);
-    sh.side_long_t_dir = sub2(sh.t2, sh.t0);
-}
-
-// pixel_shaders.cpp:106-126,320-325
-__device__ __forceinline__ void sh_prepare_upper(Shader &sh, bool llr)
-{
-    sh.vleft = sh.v0;
-    sh.vright = sh.v0;
-    sh.vleftdir = llr ? sub3(sh.v1, sh.v0) : sub3(sh.v2, sh.v0);
-    sh.vrightdir = llr ? sub3(sh.v2, sh.v0) : sub3(sh.v1, sh.v0);
-    sh.nleft = sh.n0;
-    sh.nright = sh.n0;
-    sh.nleftdir = llr ? sub3(sh.n1, sh.n0) : sub3(sh.n2, sh.n0);
-    sh.nrightdir = llr ? sub3(sh.n2, sh.n0) : sub3(sh.n1, sh.n0);
-    sh.llr = llr;
-    sh.side_short_t = sh.t0;
-    sh.side_short_t_dir = sub2(sh.t1, sh.t0);
-}
-
-// pixel_shaders.cpp:127-151,327-332
-__device__ __forceinline__ void sh_prepare_lower(Shader &sh, bool llr)
-{
-    if (llr) {
-        sh.vright = sh.v0;
-        sh.vrightdir = sub3(sh.v2, sh.v0);
-        sh.vleft = sh.v1;
-        sh.vleftdir = sub3(sh.v2, sh.v1);
-        sh.nright = sh.n0;
-        sh.nrightdir = sub3(sh.n2, sh.n0);
-        sh.nleft = sh.n1;
-        sh.nleftdir = sub3(sh.n2, sh.n1);
-    } else {
-        sh.vleft = sh.v0;
-        sh.vleftdir = sub3(sh.v2, sh.v0);
-        sh.vright = sh.v1;
-        sh.vrightdir = sub3(sh.v2, sh.v1);
-        sh.nleft = sh.n0;
-        sh.nleftdir = sub3(sh.n2, sh.n0);
-        sh.nright = sh.n1;
-        sh.nrightdir = sub3(sh.n2, sh.n1);
+    {
+        const V3 a = sel3(lower, l.n, s.n), b = sel3(lower, s.n, l.n);
+        const V3 c = sel3(lower, r.n, s.n), d = sel3(lower, s.n, r.n);
+        const V3 v = add3(a, mul3(sub3(b, a), pl));
+        const V3 n = add3(v, mul3(sub3(add3(c, mul3(sub3(d, c), pr)), v), progress));
+        sh.n = sel3(inverted, neg3(n), n);
     }
-    sh.llr = llr;
-    sh.side_short_t = sh.t1;
-    sh.side_short_t_dir = sub2(sh.t2, sh.t1);
-}
-
-// pixel_shaders.cpp:152-158,334-346
-__device__ __forceinline__ void sh_prepare_scanline(Shader &sh, float pl, float pr)
-{
-    sh.v = add3(sh.vleft, mul3(sh.vleftdir, pl));
-    sh.vdir = sub3(add3(sh.vright, mul3(sh.vrightdir, pr)), sh.v);
-    sh.n = add3(sh.nleft, mul3(sh.nleftdir, pl));
-    sh.ndir = sub3(add3(sh.nright, mul3(sh.nrightdir, pr)), sh.n);
-    if (sh.llr) {
-        sh.t_left = add2(sh.side_short_t, mul2(sh.side_short_t_dir, pl));
-        sh.t_dir = sub2(add2(sh.t0, mul2(sh.side_long_t_dir, pr)), sh.t_left);
-    } else {
-        sh.t_left = add2(sh.t0, mul2(sh.side_long_t_dir, pl));
-        sh.t_dir = sub2(add2(sh.side_short_t, mul2(sh.side_short_t_dir, pr)), sh.t_left);
+    {
+        const float tw = (float)sh.tw, th = (float)sh.th;
+        const V2 ts = mk2(s.uv.x * tw, s.uv.y * th), tl = mk2(l.uv.x * tw, l.uv.y * th),
+                 tr = mk2(r.uv.x * tw, r.uv.y * th);
+        const V2 a = sel2(lower, tl, ts), b = sel2(lower, ts, tl);
+        const V2 c = sel2(lower, tr, ts), d = sel2(lower, ts, tr);
+        const V2 v = add2(a, mul2(sub2(b, a), pl));
+        sh.t = add2(v, mul2(sub2(add2(c, mul2(sub2(d, c), pr)), v), progress));
     }
 }
 
@@ -134,6 +109,7 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
     else
         face_sun = face_sun * L.sun_intensity;
     float dyn = 0.0f;
+    const float fp = (float)shininess;
     for (int l = 0; l < L.n; l++) {
         const float4 pl = L.pl[l];
         V3 ld = sub3(center, mk3(pl.x, pl.y, pl.z));
@@ -152,9 +128,9 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
         diffuse = diffuse * alignment;
         const V3 reflection = add3(ld, mul3(normal, alignment * 2.0f));
         float specular = dot3(reflection, camvec);
-        if (specular > 0.0f) {
+        if (specular > 0.0f && !(fp * log2_approx(specular) < log2_approx(diffuse * d2) - 36.0f)) {
             specular = spec_pow(specular, shininess);
-            specular = specular * (float)shininess / 2.0f;
+            specular = specular * fp / 2.0f;
             dyn = dyn + (diffuse + specular / d2);
         } else {
             dyn = dyn + diffuse;
@@ -164,12 +140,11 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
 }
 
 // pixel_shader_lights_phong::shade (src/render/pixel_shaders.cpp:159-205)
-__device__ __forceinline__ int sh_phong(const Shader &sh, const LightsDev &L, const ViewDev &v, float progress)
+__device__ __forceinline__ int sh_phong(const Shader &sh, const LightsDev &L, const ViewDev &v)
 {
-    const V3 center = add3(sh.v, mul3(sh.vdir, progress));
-    const V3 normal = normalize3(add3(sh.n, mul3(sh.ndir, progress)));
-    const V3 camvec = normalize3(sub3(mk3(v.campos[0], v.campos[1], v.campos[2]), center));
-    return f2i(65536.0f * light_sum(L, center, normal, camvec, sh.shininess));
+    const V3 normal = normalize3(sh.n);
+    const V3 camvec = normalize3(sub3(mk3(v.campos[0], v.campos[1], v.campos[2]), sh.center));
+    return f2i(65536.0f * light_sum(L, sh.center, normal, camvec, sh.shininess));
 }
 
 // pixel_shader_lights_flat::prepare_for_triangle (src/render/pixel_shaders.cpp:
@@ -194,9 +169,9 @@ __device__ __forceinline__ int flat_light(const V3 w[3], bool inverted, const Li
 // pixel_shader_texture::shade (src/render/pixel_shaders.cpp:276-281): the
 // texel at (int)t % size, the int converted to unsigned by the unsigned width
 // and height.
-__device__ __forceinline__ uint32_t sh_nearest(const Shader &sh, float progress)
+__device__ __forceinline__ uint32_t sh_nearest(const Shader &sh)
 {
-    const V2 t = add2(sh.t_left, mul2(sh.t_dir, progress));
+    const V2 t = sh.t;
     const uint32_t tw = (uint32_t)sh.tw, th = (uint32_t)sh.th;
     const uint32_t u = (uint32_t)f2i(t.x) % tw;
     const uint32_t vv = (uint32_t)f2i(t.y) % th;
@@ -205,12 +180,34 @@ __device__ __forceinline__ uint32_t sh_nearest(const Shader &sh, float progress)
     return sh.tex ? __ldg(sh.tex + vv * tw + u) : sh.color; // untextured: 1x1 of the colour
 }
 
+// The remainder of `i + n` by n as the reference's int arithmetic gives it
+// (it keeps the sign of a negative dividend), without the division while i
+// is in [-n, n).
+__device__ __forceinline__ int wrap_texel(int i, int n)
+{
+    int m = i < 0 ? i + n : i;
+    if ((uint32_t)m >= (uint32_t)n)
+        m = (n & (n - 1)) == 0 && i >= 0 ? i & (n - 1) : (i + n) % n;
+    return m;
+}
+
+// A sum of weighted bytes, 0 <= x < 2^22, rounded half away from zero
+// (roundf): adding 2^23 rounds to the nearest integer with ties to even, and
+// a tie that went down leaves a remainder of exactly 0.5.
+__device__ __forceinline__ uint32_t round_byte(float x)
+{
+    const float t = x + 8388608.0f;
+    return (__float_as_uint(t) + (x - (t - 8388608.0f) == 0.5f ? 1u : 0u)) & 0xFFu;
+}
+
 // pixel_shader_texture_bilinear::shade (src/render/pixel_shaders.cpp:348-384)
 // with the pixel_colors_f sums of src/render/colors.cpp:11-30.  v comes from
-// t.x and u from t.y, as in the reference.
-__device__ __forceinline__ uint32_t sh_bilinear(const Shader &sh, float progress)
+// t.x and u from t.y, as in the reference.  FAST: both coordinates are below
+// 2^22 in magnitude, so their conversions are in range, the weights lie in
+// [0, 1] and the sums are bytes.
+template <bool FAST>
+__device__ __forceinline__ uint32_t bilinear_at(const uint32_t *tex, int tw, int th, uint32_t color, V2 t)
 {
-    const V2 t = add2(sh.t_left, mul2(sh.t_dir, progress));
     float v = t.x;
     float u = t.y;
     // (float)(u - 0.5) in double equals u - 0.5f in float: 0.5 is exact and
@@ -218,45 +215,44 @@ __device__ __forceinline__ uint32_t sh_bilinear(const Shader &sh, float progress
     const float u1 = u - 0.5f, u2 = u + 0.5f, v1 = v - 0.5f, v2 = v + 0.5f;
     u = floorf(u2);
     v = floorf(v2);
-    const int tw = sh.tw, th = sh.th;
-    int v1m = (f2i(v1) + th) % th;
+    int v1m = FAST ? wrap_texel(__float2int_rz(v1), th) : (f2i(v1) + th) % th;
     int v2m = v1m + 1;
     if (v2m == th)
         v2m = 0;
-    v1m *= tw;
-    v2m *= tw;
-    const int u1m = (f2i(u1) + tw) % tw;
+    const int u1m = FAST ? wrap_texel(__float2int_rz(u1), tw) : (f2i(u1) + tw) % tw;
     int u2m = u1m + 1;
     if (u2m == tw)
         u2m = 0;
-    const long long n = (long long)tw * th;
-    const long long i11 = (long long)v1m + u1m, i21 = (long long)v2m + u1m, i12 = (long long)v1m + u2m,
-                    i22 = (long long)v2m + u2m;
-    if (i11 < 0 || i11 >= n || i21 < 0 || i21 >= n || i12 < 0 || i12 >= n || i22 < 0 || i22 >= n)
-        return 0u; // the reference reads outside the texture here
     const float w11 = (u - u1) * (v - v1), w21 = (u - u1) * (v2 - v), w12 = (u2 - u) * (v - v1),
                 w22 = (u2 - u) * (v2 - v);
-    uint32_t c11 = sh.color, c21 = sh.color, c12 = sh.color, c22 = sh.color; // untextured: 1x1 of the colour
-    if (sh.tex) {
+    uint32_t c11 = color, c21 = color, c12 = color, c22 = color; // untextured: 1x1 of the colour
+    const long long row1 = (long long)v1m * tw, row2 = (long long)v2m * tw;
+    if (!FAST || (v1m | u1m) < 0) { // (a negative remainder)
+        const long long n = (long long)tw * th, i11 = row1 + u1m, i21 = row2 + u1m, i12 = row1 + u2m, i22 = row2 + u2m;
+        if (i11 < 0 || i11 >= n || i21 < 0 || i21 >= n || i12 < 0 || i12 >= n || i22 < 0 || i22 >= n)
+            return 0u; // the reference reads outside the texture here
+    }
+    if (tex) {
         // the two texels of a row are neighbours unless the column wraps: one
         // 8-byte load when the pair starts on an even texel (textures start
         // 256-byte aligned), else two 4-byte loads
+        const uint32_t *r1 = tex + row1, *r2 = tex + row2;
         const bool pair = u2m == u1m + 1;
-        if (pair && (i11 & 1) == 0) {
-            const uint2 t = __ldg(reinterpret_cast<const uint2 *>(sh.tex + i11));
-            c11 = t.x;
-            c12 = t.y;
+        if (pair && ((uintptr_t)(r1 + u1m) & 7) == 0) {
+            const uint2 q = __ldg(reinterpret_cast<const uint2 *>(r1 + u1m));
+            c11 = q.x;
+            c12 = q.y;
         } else {
-            c11 = __ldg(sh.tex + i11);
-            c12 = __ldg(sh.tex + i12);
+            c11 = __ldg(r1 + u1m);
+            c12 = __ldg(r1 + u2m);
         }
-        if (pair && (i21 & 1) == 0) {
-            const uint2 t = __ldg(reinterpret_cast<const uint2 *>(sh.tex + i21));
-            c21 = t.x;
-            c22 = t.y;
+        if (pair && ((uintptr_t)(r2 + u1m) & 7) == 0) {
+            const uint2 q = __ldg(reinterpret_cast<const uint2 *>(r2 + u1m));
+            c21 = q.x;
+            c22 = q.y;
         } else {
-            c21 = __ldg(sh.tex + i21);
-            c22 = __ldg(sh.tex + i22);
+            c21 = __ldg(r2 + u1m);
+            c22 = __ldg(r2 + u2m);
         }
     }
     uint32_t out = 0;
@@ -267,38 +263,52 @@ __device__ __forceinline__ uint32_t sh_bilinear(const Shader &sh, float progress
         acc = acc + (float)((c21 >> sft) & 0xFFu) * w21;
         acc = acc + (float)((c12 >> sft) & 0xFFu) * w12;
         acc = acc + (float)((c22 >> sft) & 0xFFu) * w22;
-        out |= ((uint32_t)f2i(roundf(acc)) & 0xFFu) << sft;
+        out |= (FAST ? round_byte(acc) : (uint32_t)f2i(roundf(acc)) & 0xFFu) << sft;
     }
     return out;
+}
+
+// texture coordinates of 2^22 texels and more, infinities and NaNs
+__device__ __noinline__ uint32_t bilinear_far(const uint32_t *tex, int tw, int th, uint32_t color, float tx, float ty)
+{
+    return bilinear_at<false>(tex, tw, th, color, mk2(tx, ty));
+}
+
+__device__ __forceinline__ uint32_t sh_bilinear(const Shader &sh)
+{
+    if (!(fabsf(sh.t.x) < 4194304.0f && fabsf(sh.t.y) < 4194304.0f))
+        return bilinear_far(sh.tex, sh.tw, sh.th, sh.color, sh.t.x, sh.t.y);
+    return bilinear_at<true>(sh.tex, sh.tw, sh.th, sh.color, sh.t);
 }
 
 // The view's pixel shader (SGL_SHADER_*, include/sgl.h); the combinations are
 // pixel_shader_light_and_texture::shade (swegl/render/pixel_shaders.hpp:159-178).
 // ALL_MODES = false compiles the default Phong + bilinear shader alone.
 template <bool ALL_MODES = true>
-__device__ __forceinline__ uint32_t sh_shade(const Shader &sh, const LightsDev &L, const ViewDev &v, float progress)
+__device__ __forceinline__ uint32_t sh_shade(const Shader &sh, const LightsDev &L, const ViewDev &v)
 {
     const int mode = ALL_MODES ? v.shader : SGL_SHADER_PHONG_BILINEAR;
     if (mode >= SGL_SHADER_COLOR) {
         switch (mode) {
         case SGL_SHADER_COLOR: return sh.color;
-        case SGL_SHADER_BILINEAR: return sh_bilinear(sh, progress);
-        case SGL_SHADER_NEAREST: return sh_nearest(sh, progress);
-        case SGL_SHADER_PHONG: return (uint32_t)sh_phong(sh, L, v, progress);
+        case SGL_SHADER_BILINEAR: return sh_bilinear(sh);
+        case SGL_SHADER_NEAREST: return sh_nearest(sh);
+        case SGL_SHADER_PHONG: return (uint32_t)sh_phong(sh, L, v);
         default: return (uint32_t)sh.flat_light; // SGL_SHADER_FLAT
         }
     }
     const bool nearest = mode == SGL_SHADER_PHONG_NEAREST || mode == SGL_SHADER_FLAT_NEAREST;
     const bool flat = mode == SGL_SHADER_FLAT_BILINEAR || mode == SGL_SHADER_FLAT_NEAREST;
-    uint32_t color = nearest ? sh_nearest(sh, progress) : sh_bilinear(sh, progress);
+    uint32_t color = nearest ? sh_nearest(sh) : sh_bilinear(sh);
     // (float)(i / 65536.0): the int rounded to float, then an exact power-of-two scale
-    float light = __int2float_rn(flat ? sh.flat_light : sh_phong(sh, L, v, progress)) * (1.0f / 65536.0f);
+    float light = __int2float_rn(flat ? sh.flat_light : sh_phong(sh, L, v)) * (1.0f / 65536.0f);
     uint32_t out = color & 0xFF000000u;
     if (light < 1.0f) {
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const uint32_t c = (color >> (8 * k)) & 0xFFu;
-            out |= ((uint32_t)f2i((float)c * light) & 0xFFu) << (8 * k);
+            // (|light| <= 2^15: the conversion is in range)
+            out |= ((uint32_t)__float2int_rz((float)c * light) & 0xFFu) << (8 * k);
         }
     } else {
         light = sqrtf(light);
@@ -306,7 +316,7 @@ __device__ __forceinline__ uint32_t sh_shade(const Shader &sh, const LightsDev &
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const uint32_t c = (color >> (8 * k)) & 0xFFu;
-            const uint32_t q = (uint32_t)f2i((float)(255u - c) / light) & 0xFFu;
+            const uint32_t q = (uint32_t)__float2int_rz((float)(255u - c) / light) & 0xFFu;
             out |= ((255u - q) & 0xFFu) << (8 * k);
         }
     }
