@@ -7,11 +7,11 @@
 //
 //   k_vertex      world -> view -> projection, |z'| divide      (vertex_shaders.hpp:35-52)
 //   k_flags       visibility flags of triangles                  (renderer.cpp:86-185)
-//   k_compact     drawable triangles -> the walk list / the near-clip list
-//   k_setup       per walk-list triangle: its scanline set-up (TriRec)
-//   k_walk        rows of each 32 set-ups dealt across a warp's lanes,
-//                 fragment keys folded with an atomic min; then the warp's
-//                 share of the near-clip triangles and of the tall triangles
+//   k_compact     drawable triangles -> the walk, tall or near-clip list
+//   k_walk        scanline set-ups (TriRec) of 32 walk-list triangles, their
+//                 rows dealt across a warp's lanes, fragment keys folded with
+//                 an atomic min; then the warp's share of the near-clip
+//                 triangles and of the tall triangles
 //   k_spans       long spans binned by the walk, one warp each
 //   k_winners     winner records of binned spans and near-clip triangles
 //                 (every span after a bin overflow)
@@ -81,11 +81,11 @@ __device__ __forceinline__ void key_min(unsigned long long *p, unsigned long lon
     asm volatile("red.global.min.u64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
 }
 
-// Asynchronous 4-byte global -> shared copies (cp.async), committed as groups.
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem)
+// Asynchronous global -> shared copies of BYTES (cp.async), committed as groups.
+template <int BYTES> __device__ __forceinline__ void cp_async(void *smem, const void *gmem)
 {
     const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sa), "l"(gmem), "n"(BYTES) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -421,9 +421,36 @@ __device__ __forceinline__ unsigned long long reserve_lists(const BatchDev *b, u
     return atomicAdd(b->counters + C_LIST / 2, ((unsigned long long)n1 << 32) | n0);
 }
 
+// The rows a triangle whose screen y range is lo_y .. hi_y walks in a view of
+// rows y .. y_end are more than kTallRows (the first test settles most).
+__device__ __forceinline__ bool tall_rows(float lo_y, float hi_y, int y, int y_end)
+{
+    if (hi_y - lo_y < kTallRows - 0.5f)
+        return false;
+    const int a = max(f2i(ceilf(lo_y)), y), z = min(f2i(ceilf(hi_y)), y_end);
+    return z > a && z - a > kTallRows;
+}
+
+// Batch triangles r of the lanes that ask for it into the tall list, one
+// atomic per warp.  Every lane of the warp calls it.
+__device__ __forceinline__ void list_tall(const BatchDev *b, bool want, uint32_t r)
+{
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, want);
+    if (!m)
+        return;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    uint32_t at = 0;
+    if (lane == leader)
+        at = atomicAdd(counter32(b, C_TALL), (uint32_t)__popc(m));
+    at = __shfl_sync(0xFFFFFFFFu, at, leader) + __popc(m & ((1u << lane) - 1u));
+    if (want && in_bounds(at < b->list_cap, CHK_REC, at))
+        b->tall[at] = r;
+}
+
 // Drawable triangles (all three vertices flagged, renderer.cpp:248-253) into
-// the walk list; triangles crossing the near plane go to their own list and
-// are marked in the record map.  One global atomic per list per block.
+// the walk list, or the tall list when they have many rows; triangles crossing
+// the near plane go to their own list and are marked in the record map.  One
+// global atomic per list per block.
 constexpr int kCompactBlock = 512;
 __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
 {
@@ -443,7 +470,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
             cnt[threadIdx.x] = 0;
         __syncthreads();
         const uint32_t g = g0 + threadIdx.x;
-        int list = -1;
+        int list = -1; // 0 walk list, 1 clip list, 2 tall list
         bool xsliver = false;
         uint32_t t = 0;
         if (g < total) {
@@ -501,12 +528,15 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
                                 xsliver = true;
                                 if (b->slot_flags)
                                     b->slot_flags[2 * t] = 1;
+                            } else if (tall_rows(lo_y, hi_y, it.v.y, it.v.y + it.v.h)) {
+                                list = 2;
                             }
                         }
                     }
                 }
             }
         }
+        list_tall(b, list == 2, list == 2 ? __ldg(b->tri_base + item) + t : 0u);
         acc.add(b, (uint32_t)item, 1ull, 0ull, xsliver);
         uint32_t pos = 0;
 #pragma unroll
@@ -571,8 +601,8 @@ struct GeomShared {
     uint32_t clip[kGeomPass][kGeomWarps][kGeomTG]; // ... of the clip list
     uint32_t cnt[kGeomPass][kGeomWarps][2];        // entries of each list, then their first positions
     uint32_t nx[kGeomPass][kGeomWarps];            // drawable triangles without a pixel column
-    float view[kGeomWarps][28];                    // the warp's copy of the item in hand: view and
-                                                   // projection rows 0-2, vm00, vm03, vm11, vm13
+    float view[kGeomWarps][30];                    // the warp's copy of the item in hand: view and projection
+                                                   // rows 0-2, vm00, vm03, vm11, vm13, first and end row
 };
 static_assert(kFuseVerts <= 256, "local vertex indices are bytes");
 constexpr size_t kGeomSmem = sizeof(GeomShared);
@@ -674,6 +704,8 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                         vw[25] = it.v.vm03;
                         vw[26] = it.v.vm11;
                         vw[27] = it.v.vm13;
+                        vw[28] = __int_as_float(it.v.y);
+                        vw[29] = __int_as_float(it.v.y + it.v.h);
                     }
                     float4 *ndc = it.ndc + gq.x;
                     __syncwarp();
@@ -724,7 +756,7 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                     const float vm00 = vw[24], vm03 = vw[25], vm11 = vw[26], vm13 = vw[27];
                     for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
                         const uint32_t t = t0 + lane;
-                        int d = 0; // 0 none, 1 walk list, 2 clip list, 3 no pixel column
+                        int d = 0; // 0 none, 1 walk list, 2 clip list, 3 no pixel column, 4 tall list
                         if (t < gq.w) {
                             const uint32_t tp = t < 32 ? tr0 : (t < 64 ? tr1 : geom_tri(tris, gq, t));
                             const uint32_t ia = tp & 0xFFu, ib = (tp >> 8) & 0xFFu, ic = tp >> 16;
@@ -754,12 +786,17 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                                                 d = 3; // no pixel column
                                                 if (b->slot_flags)
                                                     b->slot_flags[2 * (gq.z + t)] = 1;
+                                            } else if (tall_rows(lo_y, hi_y, __float_as_int(vw[28]),
+                                                                 __float_as_int(vw[29]))) {
+                                                d = 4;
                                             }
                                         }
                                     }
                                 }
                             }
                         }
+                        if (__any_sync(0xFFFFFFFFu, d == 4))
+                            list_tall(b, d == 4, __ldg(b->tri_base + item) + gq.z + t);
                         const unsigned m1 = __ballot_sync(0xFFFFFFFFu, d == 1);
                         const unsigned m2 = __ballot_sync(0xFFFFFFFFu, d == 2);
                         const unsigned m3 = __ballot_sync(0xFFFFFFFFu, d == 3);
@@ -1059,29 +1096,43 @@ struct WinnerVisitor {
 // from the set-up; the divisions of a row (edge progress, span set-up) and of
 // its pixels then run wherever that row is.  A warp takes 32 triangles, each
 // lane makes its triangle's set-up (the TriRec), and the warp's rows are
-// dealt out across the lanes.  Triangles with more than kTallRows rows are
-// walked by the whole warp, 32 rows at a time, and every one of their spans
-// goes to the long-span kernels.
+// dealt out across the lanes.  Triangles with more than kTallRows rows have
+// a list of their own (the geometry passes know their rows): each is walked
+// by a whole warp, 32 rows at a time, and every one of its spans goes to the
+// long-span kernels.
+//
+// The set-up is made here, in the shared memory that the rows are read from.
+// As a pass of its own it spent its time on the stores of its records (51 MB
+// on the 1080p frame) and the walk on reading them back; made here, only the
+// records of triangles with fragments are stored, for the shade, as whole
+// lines: set-up and walk 49.0 -> 37.4 us (1080p), 854 -> 682 us (64 views).
+// Both were bound by latency and issue (20 % and 48 % of the issue slots).
 
 constexpr int kWalkWarps = 4;
 #ifndef SGL_WALK_MIN_BLOCKS
-#define SGL_WALK_MIN_BLOCKS 6 // resident blocks per SM the walk is compiled for (caps its registers)
+#define SGL_WALK_MIN_BLOCKS 5 // resident blocks per SM the walk is compiled for (caps its registers: 4, 5, 6 and 7
+                              // blocks walk the 1080p frame in 39.5, 37.4, 40.2 and 51.5 us)
 #endif
-// Per-warp shared copy of the lanes' set-ups, sm[field][lane]: fields 0-31 are
-// the words of TriRec in order, so the warp can store whole records; the row
-// is padded to 33 words so that both the per-lane and the per-record accesses
-// are free of bank conflicts.
+// Per-warp set-ups in shared memory, S[field][lane]: fields 0-31 are the
+// words of TriRec in order; the row is padded to 33 words so that both the
+// per-lane and the per-record accesses are free of bank conflicts.
 enum {
     F_LX, F_LT, F_LB, F_LR, F_LTS, F_LBS, // long edge: x, top, bottom, ratio, tstep, bstep
+    F_Z0, F_Z2,
     F_UX, F_UT, F_UB, F_UR, F_UTS, F_UBS, // upper short edge
+    F_SLOT, F_ITEM,
     F_DX, F_DT, F_DB, F_DR, F_DTS, F_DBS, // lower short edge
-    F_Z0, F_Z1, F_Z2, F_YS, F_YL, F_NU, F_ND, F_FLAGS, F_SLOT, F_ITEM, F_G0, F_G1, F_G2, F_PRIM,
+    F_YL, F_ND,
+    F_Z1, F_YS, F_NU, F_FLAGS, F_G0, F_G1, F_G2, F_PRIM,
     F_FRAGS, // fragments of the lane's triangle (shared atomics of the lanes walking its rows)
     F_INCL,  // inclusive prefix of the rows dealt out, per lane
     kWalkFields
 };
 constexpr int kWalkPitch = 33;
 static_assert(F_PRIM == 31 && sizeof(TriRec) == 32 * sizeof(uint32_t), "shared set-up fields follow TriRec");
+static_assert(offsetof(TriRec, slot) == 4 * F_SLOT && offsetof(TriRec, dx) == 4 * F_DX &&
+                  offsetof(TriRec, flags) == 4 * F_FLAGS,
+              "shared set-up fields follow TriRec");
 
 // interpolator_g<1>::InitSelf then DisplaceStartingPoint (interpolator.hpp:
 // 60-84), with 1/z1 and 1/z2 passed in (the same divisions, made once per
@@ -1307,119 +1358,79 @@ __device__ __forceinline__ void smem_row_in(RowIn &r, const WalkRow *S, int o, i
            S[F_FLAGS][o]);
 }
 
-// Set-up of triangle t of `item` (list entry i): fill_triangle's z sort
-// (renderer.cpp:264-279), fill_triangle_2's y sort, edges and halves
-// (:375-460), into the TriRec of batch triangle r (t = r - tri_base[item]).
-// Returns whether the triangle reached scanline set-up (y0 != y2); the record
-// of one that did not has no rows.
-__device__ __forceinline__ bool tri_setup(const BatchDev *b, uint32_t r, uint32_t item, bool &tall)
+// Set-up of triangle t (vertices `tri`, projected n0, n1, n2) of `item`:
+// fill_triangle's z sort (renderer.cpp:264-279), fill_triangle_2's y sort,
+// edges and halves (:375-460), into column `c` of the warp's set-ups.  Returns
+// whether the triangle reached scanline set-up (y0 != y2); one that did not
+// has no rows.
+__device__ __forceinline__ bool tri_setup(const BatchDev *b, const ViewDev &v, uint32_t item, uint32_t t, uint4 tri,
+                                          float4 n0, float4 n1, float4 n2, uint32_t extra_flags, WalkRow *S, int c)
 {
-    tall = false;
-    const uint32_t t = r - __ldg(b->tri_base + item);
-    const ItemDev &it = b->items[item];
-    const ViewDev &v = it.v;
-    const uint4 tri = it.s.tris[t];
-    V3 a = load_vp(it, tri.x), c1 = load_vp(it, tri.y), c2 = load_vp(it, tri.z);
+    auto put = [&](int f, float x) { S[f][c] = __float_as_uint(x); };
+    auto vp = [&](float4 n) { return mk3(v.vm00 * n.x + v.vm03, v.vm11 * n.y + v.vm13, n.z); }; // as load_vp
+    V3 a = vp(n0), c1 = vp(n1), c2 = vp(n2);
     const bool ffv = cross_z_negative(sub3(c1, a), sub3(c2, a));
     int pa = 0, pb = 1, pc = 2;
     sort_z_desc(a, c1, c2, pa, pb, pc);
     sort_y_asc(a, c1, c2, pa, pb, pc);
     const V3 v0 = a, v1 = c1, v2 = c2;
     const int y0 = f2i(ceilf(v0.y)), y1 = f2i(ceilf(v1.y)), y2 = f2i(ceilf(v2.y));
-    if (!in_bounds(r < b->list_cap, CHK_REC, r))
+    S[F_ITEM][c] = item;
+    S[F_SLOT][c] = 2 * t;
+    S[F_NU][c] = 0;
+    S[F_ND][c] = 0;
+    S[F_FLAGS][c] = extra_flags;
+    if (y0 == y2)
         return false;
-    float4 *dst = reinterpret_cast<float4 *>(b->recs + r);
-    if (y0 == y2) {
-        // no rows: n_u = n_d = 0
-        dst[5] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
-        dst[6] = make_float4(__int_as_float(0), 0.0f, 0.0f, __uint_as_float(item));
-        return false;
-    }
-    const uint32_t slot = 2 * t;
     if (b->slot_flags)
-        b->slot_flags[slot] = 1;
+        b->slot_flags[2 * t] = 1;
+    S[F_G0][c] = pa == 0 ? tri.x : (pa == 1 ? tri.y : tri.z);
+    S[F_G1][c] = pb == 0 ? tri.x : (pb == 1 ? tri.y : tri.z);
+    S[F_G2][c] = pc == 0 ? tri.x : (pc == 1 ? tri.y : tri.z);
+    S[F_PRIM][c] = tri.w;
+    put(F_Z0, v0.z);
+    put(F_Z1, v1.z);
+    put(F_Z2, v2.z);
     const float rz0 = 1.0f / v0.z, rz1 = 1.0f / v1.z, rz2 = 1.0f / v2.z;
     const int ys = y0 < v.y ? v.y : y0;
-    float ltop, lbot, lts, lbs;
+    S[F_YS][c] = (uint32_t)ys;
     const float lmove = (float)ys - v0.y;
     const float lratio = (v2.x - v0.x) / (v2.y - v0.y);
-    edge_init(v2.y - v0.y, rz0, rz2, lmove, ltop, lbot, lts, lbs);
-    const float lx = v0.x + lratio * lmove;
-    uint32_t flags = ffv ? kRecFFV : 0u;
-    int n_u = 0, n_d = 0, y_l = 0;
-    float ux = 0.0f, utop = 0.0f, ubot = 0.0f, uratio = 0.0f, uts = 0.0f, ubs = 0.0f;
-    float dx = 0.0f, dtop = 0.0f, dbot = 0.0f, dratio = 0.0f, dts = 0.0f, dbs = 0.0f;
+    float top, bot, ts, bs;
+    auto edge = [&](int f, float x, float ratio) {
+        put(f, x);
+        put(f + 1, top);
+        put(f + 2, bot);
+        put(f + 3, ratio);
+        put(f + 4, ts);
+        put(f + 5, bs);
+    };
+    edge_init(v2.y - v0.y, rz0, rz2, lmove, top, bot, ts, bs);
+    edge(F_LX, v0.x + lratio * lmove, lratio);
+    uint32_t flags = extra_flags | (ffv ? kRecFFV : 0u);
     if (y1 >= v.y) {
-        uratio = (v1.x - v0.x) / (v1.y - v0.y);
+        const float ratio = (v1.x - v0.x) / (v1.y - v0.y);
         const int yend = y1 < v.y + v.h ? y1 : v.y + v.h;
-        edge_init(v1.y - v0.y, rz0, rz1, lmove, utop, ubot, uts, ubs);
-        ux = v0.x + uratio * lmove;
-        if (lratio > uratio)
+        edge_init(v1.y - v0.y, rz0, rz1, lmove, top, bot, ts, bs);
+        edge(F_UX, v0.x + ratio * lmove, ratio);
+        if (lratio > ratio)
             flags |= kRecLLRUpper;
-        n_u = yend > ys ? yend - ys : 0;
+        S[F_NU][c] = yend > ys ? (uint32_t)(yend - ys) : 0u;
     }
     if (y1 < v.y + v.h) {
-        dratio = (v2.x - v1.x) / (v2.y - v1.y);
+        const float ratio = (v2.x - v1.x) / (v2.y - v1.y);
         const int y = y1 > v.y ? y1 : v.y;
         const int yend = y2 < v.y + v.h ? y2 : v.y + v.h;
         const float move = (float)y - v1.y;
-        edge_init(v2.y - v1.y, rz1, rz2, move, dtop, dbot, dts, dbs);
-        dx = v1.x + dratio * move;
-        if (lratio < dratio)
+        edge_init(v2.y - v1.y, rz1, rz2, move, top, bot, ts, bs);
+        edge(F_DX, v1.x + ratio * move, ratio);
+        if (lratio < ratio)
             flags |= kRecLLRLower;
-        y_l = y;
-        n_d = yend > y ? yend - y : 0;
+        S[F_YL][c] = (uint32_t)y;
+        S[F_ND][c] = yend > y ? (uint32_t)(yend - y) : 0u;
     }
-    if (n_u + n_d > kTallRows) {
-        flags |= kRecTall;
-        tall = true;
-    }
-    const uint32_t g0 = pa == 0 ? tri.x : (pa == 1 ? tri.y : tri.z);
-    const uint32_t g1 = pb == 0 ? tri.x : (pb == 1 ? tri.y : tri.z);
-    const uint32_t g2 = pc == 0 ? tri.x : (pc == 1 ? tri.y : tri.z);
-    dst[0] = make_float4(lx, ltop, lbot, lratio);
-    dst[1] = make_float4(lts, lbs, ux, utop);
-    dst[2] = make_float4(ubot, uratio, uts, ubs);
-    dst[3] = make_float4(dx, dtop, dbot, dratio);
-    dst[4] = make_float4(dts, dbs, v0.z, v1.z);
-    dst[5] = make_float4(v2.z, __int_as_float(ys), __int_as_float(y_l), __int_as_float(n_u));
-    dst[6] = make_float4(__int_as_float(n_d), __uint_as_float(flags), __uint_as_float(slot), __uint_as_float(item));
-    dst[7] = make_float4(__uint_as_float(g0), __uint_as_float(g1), __uint_as_float(g2), __uint_as_float(tri.w));
+    S[F_FLAGS][c] = flags;
     return true;
-}
-
-// Set-up of every walk list entry, one thread each.
-__global__ void __launch_bounds__(256) k_setup(const BatchDev *b)
-{
-    const uint32_t n_raw = *counter32(b, C_LIST);
-    const uint32_t n = n_raw < b->list_cap ? n_raw : b->list_cap;
-    ItemAcc acc;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    // the loop runs the same number of times on every lane of a warp
-    for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; i0 < n; i0 += stride) {
-        const uint32_t i = i0 + (threadIdx.x & 31);
-        bool drawn = false, tall = false;
-        uint32_t item = 0, r = 0;
-        if (i < n) {
-            const uint2 e = b->list[i];
-            r = e.x;
-            item = e.y;
-            drawn = tri_setup(b, r, item, tall);
-        }
-        // tall triangles are walked by a whole warp each, in k_walk_rare
-        const unsigned tm = __ballot_sync(0xFFFFFFFFu, tall);
-        if (tm) {
-            const int lane = threadIdx.x & 31, leader = __ffs(tm) - 1;
-            uint32_t tb = 0;
-            if (lane == leader)
-                tb = atomicAdd(counter32(b, C_TALL), (uint32_t)__popc(tm));
-            tb = __shfl_sync(0xFFFFFFFFu, tb, leader);
-            if (tall)
-                b->tall[tb + __popc(tm & ((1u << lane) - 1u))] = r;
-        }
-        acc.add(b, item, drawn ? 1ull : 0ull, 0ull, i < n);
-    }
-    acc.flush(b);
 }
 
 // One row of triangle `slot` of `item` on this lane; every lane of the warp
@@ -1472,64 +1483,84 @@ __device__ __forceinline__ int walk_row(const BatchDev *b, WalkView &v, uint32_t
     return has ? sp.x2 - sp.x1 : 0;
 }
 
-// A tall triangle (list entry i), walked by the whole warp: for each 32 rows
-// every lane runs the 32 edge steps and keeps the state of its own row, so
-// no lane repeats more than 32 steps per row it walks.  Every span is binned.
-// Returns this lane's fragments.
+// n <= 31 repeated additions x += d of three chains; every lane takes its own
+// n.  The additions of a chain are all alike, so a lane's n of them can be
+// taken in any grouping: 16, 8, 4, 2, 1 by the bits of n.
+__device__ __forceinline__ void step3(float &x, float &t, float &b, float dx, float dt, float db, int n)
+{
+#pragma unroll
+    for (int bit = 16; bit; bit >>= 1)
+        if (n & bit) {
+#pragma unroll
+            for (int k = 0; k < bit; k++) {
+                x = x + dx;
+                t = t + dt;
+                b = b + db;
+            }
+        }
+}
+__device__ __forceinline__ void step2(float &t, float &b, float dt, float db, int n)
+{
+#pragma unroll
+    for (int bit = 16; bit; bit >>= 1)
+        if (n & bit) {
+#pragma unroll
+            for (int k = 0; k < bit; k++) {
+                t = t + dt;
+                b = b + db;
+            }
+        }
+}
+
+// A tall triangle (set-up in column 0 of S), walked by the whole warp 32 rows
+// at a time: each lane takes its own row's steps from the state of the first
+// of the 32, and lane 31's state after one more step is the next 32 rows'.
+// Every span is binned.  Returns this lane's fragments.
 template <bool FRAGS>
-__device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, uint32_t i)
+__device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, const WalkRow *S)
 {
     const int lane = threadIdx.x & 31;
-    const float4 *q = reinterpret_cast<const float4 *>(b->recs + i);
-    const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5], q6 = q[6];
-    const float lg[6] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
-    const float up[6] = {q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
-    const float dn[6] = {q3.x, q3.y, q3.z, q3.w, q4.x, q4.y};
-    const float z0 = q4.z, z1 = q4.w, z2 = q5.x;
-    const int y_s = __float_as_int(q5.y), y_l = __float_as_int(q5.z), n_u = __float_as_int(q5.w);
-    const int n_d = __float_as_int(q6.x);
-    const uint32_t flags = __float_as_uint(q6.y), slot = __float_as_uint(q6.z), item = __float_as_uint(q6.w);
-    const int n = n_u + n_d;
+    const int n_u = (int)S[F_NU][0], n = n_u + (int)S[F_ND][0];
+    const uint32_t slot = S[F_SLOT][0], item = S[F_ITEM][0];
     uint32_t frags = 0;
     WalkView v;
     v.load(b, item);
     v.inline_span = b->inline_span;
-    float lx = lg[0], lt = lg[1], lb = lg[2];
-    float sx = up[0], st = up[1], sb = up[2];
+    float lx = smf(S, F_LX, 0), lt = smf(S, F_LT, 0), lb = smf(S, F_LB, 0);
+    int sf = n_u > 0 ? F_UX : F_DX; // the short edge in hand
+    float sx = smf(S, sf, 0), st = smf(S, sf + 1, 0), sb = smf(S, sf + 2, 0);
     for (int r0 = 0; r0 < n; r0 += 32) {
-        float mlx = 0.0f, mlt = 0.0f, mlb = 0.0f, msx = 0.0f, mst = 0.0f, msb = 0.0f;
-        for (int k = 0; k < 32; k++) {
-            const int rr = r0 + k;
-            if (rr == n_u) { // the lower half starts on its own short edge
-                sx = dn[0];
-                st = dn[1];
-                sb = dn[2];
-            }
-            if (k == lane) {
-                mlx = lx; mlt = lt; mlb = lb;
-                msx = sx; mst = st; msb = sb;
-            }
-            lx = lx + lg[3];
-            lt = lt + lg[4];
-            lb = lb + lg[5];
-            if (rr < n_u) {
-                sx = sx + up[3];
-                st = st + up[4];
-                sb = sb + up[5];
-            } else {
-                sx = sx + dn[3];
-                st = st + dn[4];
-                sb = sb + dn[5];
-            }
-        }
         const int k = r0 + lane;
         const bool act = k < n;
         RowIn r;
-        row_in(r, act ? k : 0, lg, (act && k >= n_u) ? dn : up, z0, z1, z2, y_s, y_l, n_u, flags);
-        r.lx = mlx; r.lt = mlt; r.lb = mlb; // already stepped to the row
-        r.sx = msx; r.st = mst; r.sb = msb;
+        smem_row_in(r, S, 0, act ? k : 0);
+        r.lx = lx; r.lt = lt; r.lb = lb;
+        step3(r.lx, r.lt, r.lb, r.lr, r.lts, r.lbs, lane);
+        // rows of the half in hand continue its chain; a row beyond it starts
+        // on the lower short edge (smem_row_in's state)
+        const bool cont = (k < n_u) == (sf == F_UX);
+        if (cont) {
+            r.sx = sx; r.st = st; r.sb = sb;
+        }
+        step3(r.sx, r.st, r.sb, r.sr, r.sts, r.sbs, cont ? lane : k - n_u);
         r.ls = 0;
         r.ss = 0;
+        // the state of row r0 + 32, if lane 31 has a row
+        if (r0 + 32 < n) {
+            lx = __shfl_sync(0xFFFFFFFFu, r.lx + r.lr, 31);
+            lt = __shfl_sync(0xFFFFFFFFu, r.lt + r.lts, 31);
+            lb = __shfl_sync(0xFFFFFFFFu, r.lb + r.lbs, 31);
+            const int half = r0 + 31 < n_u ? F_UX : F_DX; // lane 31's half
+            sx = __shfl_sync(0xFFFFFFFFu, r.sx + r.sr, 31);
+            st = __shfl_sync(0xFFFFFFFFu, r.st + r.sts, 31);
+            sb = __shfl_sync(0xFFFFFFFFu, r.sb + r.sbs, 31);
+            sf = r0 + 32 < n_u ? F_UX : F_DX;
+            if (sf != half) { // row r0 + 32 is the first of the lower half
+                sx = smf(S, F_DX, 0);
+                st = smf(S, F_DT, 0);
+                sb = smf(S, F_DB, 0);
+            }
+        }
         frags += (uint32_t)walk_row<FRAGS>(b, v, item, slot, r, act, true);
     }
     return frags;
@@ -1538,18 +1569,33 @@ __device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, uint32_t i)
 // the rare depth walks, defined with the near-clip code below
 __device__ __noinline__ void walk_clip_depth(const BatchDev *b, ItemAcc &acc);
 template <bool FRAGS>
-__device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc);
+__device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc, WalkRow *S);
 
-// Depth walk of the drawable triangles wholly in front of the near plane
-// (fill_triangle's normal case, renderer.cpp:281-285: one sub-triangle, slot
-// 2t).  Each warp takes groups of 32 list entries (warp-strided), loads their
-// set-ups into shared memory (one 128-byte record per load) and deals their
-// rows across its lanes.  FRAGS: the fragment capture of a layered view (the
-// near-clipped triangles are captured by k_frags).
+// One warp's shared memory: the set-ups of the group in hand, and what is
+// copied in ahead for the next groups: list entries (three ahead), their
+// triangles (two ahead) and the triangles' projected vertices (one ahead).
+// Each lane reads only what it copied itself, except the entries' batch
+// triangles.
+struct WalkShared {
+    WalkRow S[kWalkFields];
+    __align__(16) float4 ndc[3][32];
+    uint4 tri[2][32];
+    uint2 entry[4][32];
+};
+
+// Set-up and depth walk of the drawable triangles wholly in front of the near
+// plane (fill_triangle's normal case, renderer.cpp:281-285: one sub-triangle,
+// slot 2t).  Each warp takes groups of 32 list entries (warp-strided): a lane
+// makes its entry's set-up in shared memory, the group's rows are dealt across
+// the lanes, and the set-ups with fragments are stored as whole records for
+// the shade.  FRAGS: the fragment capture of a layered view (the near-clipped
+// triangles are captured by k_frags).
 template <bool FRAGS, bool STRIDED>
 __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(const BatchDev *b)
 {
-    __shared__ WalkRow sm[kWalkWarps][2][kWalkFields];
+    __shared__ WalkShared shared[kWalkWarps];
+    WalkShared &W = shared[threadIdx.x >> 5];
+    WalkRow *S = W.S;
     const int lane = threadIdx.x & 31;
     const uint32_t n_raw = *counter32(b, C_LIST);
     const uint32_t n = n_raw < b->list_cap ? n_raw : b->list_cap;
@@ -1561,59 +1607,67 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
     // batch of several views a strided group would mix the views' triangles,
     // whose view parameters each row then reloads (serving: 5.5 -> 12.3 us
     // per request), so there group g holds entries 32 g + j.
-    auto entry = [&](uint32_t g, uint32_t j) -> uint32_t { return STRIDED ? g + j * n_groups : 32 * g + j; };
-    auto count = [&](uint32_t g) -> uint32_t {
-        if (STRIDED)
-            return min(32u, (n - g + n_groups - 1) / n_groups);
-        return n - 32 * g < 32u ? n - 32 * g : 32u;
+    auto index = [&](uint32_t g) -> uint32_t { return STRIDED ? g + (uint32_t)lane * n_groups : 32 * g + (uint32_t)lane; };
+    // the copies of group g's entries, triangles and vertices (q: the group's
+    // place in this warp's sequence, which picks the buffers)
+    auto fetch_entry = [&](uint32_t g, int q) {
+        if (g < n_groups && index(g) < n)
+            cp_async<8>(&W.entry[q & 3][lane], b->list + index(g));
     };
-    // the record (batch triangle) of entry `lane` of group g; loaded one
-    // group ahead of its fetch, so that the copies do not wait for it
-    auto rec_of = [&](uint32_t g) -> uint32_t {
-        const uint32_t i = entry(g, (uint32_t)lane);
-        return g < n_groups && i < n ? b->list[i].x : 0u;
+    auto fetch_tri = [&](uint32_t g, int q) {
+        if (g < n_groups && index(g) < n) {
+            const uint2 e = W.entry[q & 3][lane];
+            cp_async<16>(&W.tri[q & 1][lane], b->items[e.y].s.tris + (e.x - __ldg(b->tri_base + e.y)));
+        }
     };
-    // record j of group g -> word `lane` of field row `lane`, column j
-    auto fetch = [&](uint32_t g, uint32_t rec, WalkRow *D) {
-        if (g < n_groups) {
-            const uint32_t cnt = count(g);
-#pragma unroll 8
-            for (uint32_t j = 0; j < cnt; j++) {
-                const uint32_t rj = __shfl_sync(0xFFFFFFFFu, rec, j);
-                if (in_bounds(rj < b->list_cap, CHK_REC, rj))
-                    cp_async4(&D[lane][j], reinterpret_cast<const uint32_t *>(b->recs + rj) + lane);
+    auto fetch_ndc = [&](uint32_t g, int q) {
+        if (g < n_groups && index(g) < n) {
+            const ItemDev &it = b->items[W.entry[q & 3][lane].y];
+            const uint4 t = W.tri[q & 1][lane];
+            if (in_bounds(t.x < it.s.n_vertices && t.y < it.s.n_vertices && t.z < it.s.n_vertices, CHK_NDC, t.x)) {
+                cp_async<16>(&W.ndc[0][lane], it.ndc + t.x);
+                cp_async<16>(&W.ndc[1][lane], it.ndc + t.y);
+                cp_async<16>(&W.ndc[2][lane], it.ndc + t.z);
             }
         }
-        cp_async_commit();
     };
     ItemAcc acc;
     WalkView view;
     view.item = 0xFFFFFFFFu;
     view.inline_span = b->inline_span;
-    // Warps take groups g, g + W, g + 2W, ... (W warps in the grid; work
-    // queues were measured slower: 41 -> 48 us on the 1080p frame).  While
-    // group g is walked, the records of the next one are copied in and the
-    // list entries of the one after are loaded.
-    const uint32_t W = (gridDim.x * blockDim.x) >> 5;
+    // Warps take groups g, g + G, g + 2G, ... (G warps in the grid; work
+    // queues were measured slower: 41 -> 48 us on the 1080p frame).
+    const uint32_t G = (gridDim.x * blockDim.x) >> 5;
     uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t g_next = g + W;
-    int buf = 0;
-    fetch(g, rec_of(g), sm[threadIdx.x >> 5][0]);
-    uint32_t rec_next = rec_of(g_next);
-    while (g < n_groups) {
-        fetch(g_next, rec_next, sm[threadIdx.x >> 5][buf ^ 1]);
-        const uint32_t g_after = g_next + W;
-        rec_next = rec_of(g_after);
-        cp_async_wait<1>(); // this group's copies are done
-        WalkRow *S = sm[threadIdx.x >> 5][buf];
-        const uint32_t cnt = count(g);
+    if (g < n_groups) {
+        fetch_entry(g, 0);
+        fetch_entry(g + G, 1);
+        fetch_entry(g + 2 * G, 2);
+        cp_async_commit();
+        cp_async_wait<0>();
+        fetch_tri(g, 0);
+        fetch_tri(g + G, 1);
+        cp_async_commit();
+        cp_async_wait<0>();
+        fetch_ndc(g, 0);
+        cp_async_commit();
+    }
+    for (int q = 0; g < n_groups; q++, g += G) {
+        cp_async_wait<0>();
+        const bool valid = index(g) < n;
+        bool drawn = false;
         S[F_FRAGS][lane] = 0;
-        __syncwarp();
-        const bool valid = (uint32_t)lane < cnt;
-        const int n_u = valid ? (int)S[F_NU][lane] : 0, n_d = valid ? (int)S[F_ND][lane] : 0;
-        const bool tall = valid && (S[F_FLAGS][lane] & kRecTall) != 0u; // walked by k_walk_rare
-        // rows of the non-tall triangles, dealt across the lanes
-        int incl = tall ? 0 : n_u + n_d;
+        if (valid) {
+            const uint2 e = W.entry[q & 3][lane];
+            const float4 n0 = W.ndc[0][lane], n1 = W.ndc[1][lane], n2 = W.ndc[2][lane];
+            drawn = tri_setup(b, b->items[e.y].v, e.y, e.x - __ldg(b->tri_base + e.y), W.tri[q & 1][lane], n0, n1, n2,
+                              0u, S, lane);
+        } else {
+            S[F_NU][lane] = 0;
+            S[F_ND][lane] = 0;
+        }
+        // rows dealt across the lanes
+        int incl = (int)(S[F_NU][lane] + S[F_ND][lane]);
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
@@ -1622,6 +1676,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
         }
         S[F_INCL][lane] = (uint32_t)incl;
         __syncwarp();
+        // the vertices, triangles and entries of the groups ahead (this
+        // group's are consumed)
+        fetch_ndc(g + G, q + 1);
+        fetch_tri(g + 2 * G, q + 2);
+        fetch_entry(g + 3 * G, q + 3);
+        cp_async_commit();
         const int total = (int)S[F_INCL][31];
         for (int p0 = 0; p0 < total; p0 += 32) {
             const int p = p0 + lane;
@@ -1642,17 +1702,28 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
                 atomicAdd(&S[F_FRAGS][o], (uint32_t)fr);
         }
         __syncwarp();
-        acc.add(b, valid ? S[F_ITEM][lane] : 0u, 0ull, valid ? (unsigned long long)S[F_FRAGS][lane] : 0ull, valid);
+        acc.add(b, valid ? S[F_ITEM][lane] : 0u, drawn ? 1ull : 0ull, (unsigned long long)S[F_FRAGS][lane], valid);
+        // the records with fragments, four per round (a 128-byte line by eight
+        // lanes): written by one lane each, as eight 16-byte stores to its own
+        // line, the stores' 32 lines per instruction throttled the set-up
+        // (20 us at 20 % issue on the 1080p frame)
+#pragma unroll
+        for (int j0 = 0; j0 < 32; j0 += 4) {
+            const int j = j0 + (lane >> 3), w = 4 * (lane & 7);
+            if (S[F_FRAGS][j]) {
+                const uint32_t r = W.entry[q & 3][j].x;
+                if (in_bounds(r < b->list_cap, CHK_REC, r))
+                    reinterpret_cast<uint4 *>(b->recs + r)[lane & 7] =
+                        make_uint4(S[w][j], S[w + 1][j], S[w + 2][j], S[w + 3][j]);
+            }
+        }
         __syncwarp();
-        g = g_next;
-        g_next = g_after;
-        buf ^= 1;
     }
     cp_async_wait<0>();
     // then this warp's share of the near-clip and the tall triangles
     if (!FRAGS)
         walk_clip_depth(b, acc);
-    walk_tall_all<FRAGS>(b, acc);
+    walk_tall_all<FRAGS>(b, acc, S);
     acc.flush(b);
 }
 
@@ -1782,18 +1853,28 @@ __device__ __noinline__ void walk_clip_depth(const BatchDev *b, ItemAcc &acc)
     }
 }
 
-// Depth walk (or fragment capture) of the tall triangles, one warp each
-// (warp-strided).
+// Set-up and depth walk (or fragment capture) of the tall triangles, one warp
+// each (warp-strided).
 template <bool FRAGS>
-__device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc)
+__device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc, WalkRow *S)
 {
     const uint32_t nt_raw = *counter32(b, C_TALL);
     const uint32_t nt = nt_raw < b->list_cap ? nt_raw : b->list_cap;
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t k = gw; k < nt; k += n_warps) {
-        const uint32_t i = b->tall[k];
-        const uint32_t fr = walk_tall<FRAGS>(b, i);
-        acc.add(b, b->recs[i].item, 0ull, fr, true);
+        const uint32_t r = b->tall[k];
+        const uint32_t item = (uint32_t)find_item(b->tri_base, b->n_items, r), t = r - __ldg(b->tri_base + item);
+        const ItemDev &it = b->items[item];
+        const uint4 tri = it.s.tris[t];
+        __syncwarp();
+        // (every lane writes the same values)
+        const bool drawn = tri_setup(b, it.v, item, t, tri, it.ndc[tri.x], it.ndc[tri.y], it.ndc[tri.z], kRecTall, S, 0);
+        __syncwarp();
+        if (in_bounds(r < b->list_cap, CHK_REC, r))
+            reinterpret_cast<uint32_t *>(b->recs + r)[lane] = S[lane][0];
+        const uint32_t fr = walk_tall<FRAGS>(b, S);
+        acc.add(b, item, drawn && lane == 0 ? 1ull : 0ull, fr, true);
     }
 }
 
@@ -1821,12 +1902,13 @@ __device__ __noinline__ void winner_clip(const BatchDev *b, bool overflow)
 
 __device__ __noinline__ void winner_overflow(const BatchDev *b)
 {
-    const uint32_t n_raw = *counter32(b, C_LIST);
-    const uint32_t n = n_raw < b->list_cap ? n_raw : b->list_cap;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint2 e = b->list[i];
-        const ItemDev &it = b->items[e.y];
-        const uint32_t t = e.x - __ldg(b->tri_base + e.y);
+    const uint32_t n_raw = *counter32(b, C_LIST), nt_raw = *counter32(b, C_TALL);
+    const uint32_t n = n_raw < b->list_cap ? n_raw : b->list_cap, nt = nt_raw < b->list_cap ? nt_raw : b->list_cap;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n + nt; i += gridDim.x * blockDim.x) {
+        const uint32_t r = i < n ? b->list[i].x : b->tall[i - n];
+        const uint32_t item = i < n ? b->list[i].y : (uint32_t)find_item(b->tri_base, b->n_items, r);
+        const ItemDev &it = b->items[item];
+        const uint32_t t = r - __ldg(b->tri_base + item);
         WinnerVisitor vis{&it, 2 * t, b->inline_span, true};
         const uint4 tri = it.s.tris[t];
         V3 a = load_vp(it, tri.x), c1 = load_vp(it, tri.y), c2 = load_vp(it, tri.z);
@@ -1868,14 +1950,10 @@ __device__ __forceinline__ void spans_pass(const BatchDev *b, bool winner)
         float top = r.top, bottom = r.bottom;
         for (int x0 = r.x1; x0 < r.x2; x0 += 32) {
             float mt = top, mb = bottom;
-#pragma unroll
-            for (int k = 0; k < 32; k++) {
-                if (k == lane) {
-                    mt = top;
-                    mb = bottom;
-                }
-                top = top + r.tstep;
-                bottom = bottom + r.bstep;
+            step2(mt, mb, r.tstep, r.bstep, lane);
+            if (x0 + 32 < r.x2) {
+                top = __shfl_sync(0xFFFFFFFFu, mt + r.tstep, 31);
+                bottom = __shfl_sync(0xFFFFFFFFu, mb + r.bstep, 31);
             }
             const int x = x0 + lane;
             if (x >= r.x2)
@@ -1957,30 +2035,41 @@ __device__ __forceinline__ uint32_t shade_clip_px(const ItemDev &it, uint32_t i,
     return shade_clip_rec(it, slot, it.prec[i]);
 }
 
+// A 32-byte quarter of a record, one load.
+struct Quarter {
+    uint32_t w[8];
+};
+__device__ __forceinline__ Quarter load_quarter(const TriRec *rp, int k)
+{
+    Quarter q;
+    asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(q.w[0]), "=r"(q.w[1]), "=r"(q.w[2]), "=r"(q.w[3]), "=r"(q.w[4]), "=r"(q.w[5]), "=r"(q.w[6]), "=r"(q.w[7])
+        : "l"(reinterpret_cast<const char *>(rp) + 32 * k));
+    return q;
+}
+
 // The progress values of pixel (X, Y) (surface coordinates) from its winning
-// triangle's set-up: the row's edges after their steps, the span and the
+// triangle's set-up (`d`: the record's last quarter): the row's edges after their steps, the span and the
 // qpixel chain up to X (renderer.cpp:474-493).  False when the span was wide
 // enough to be binned (its winners were recorded by the span kernels).
-__device__ __forceinline__ bool rec_replay(const TriRec *rp, const ViewDev &v, int inline_span, int X, int Y,
-                                           float4 &out)
+__device__ __forceinline__ bool rec_replay(const TriRec *rp, const Quarter &d, const ViewDev &v, int inline_span,
+                                           int X, int Y, float4 &out)
 {
-    const float4 *q = reinterpret_cast<const float4 *>(rp);
-    const float4 q5 = q[5], q6 = q[6];
-    const int y_s = __float_as_int(q5.y), y_l = __float_as_int(q5.z), n_u = __float_as_int(q5.w);
-    const uint32_t flags = __float_as_uint(q6.y);
-    const int k = (Y >= y_s && Y < y_s + n_u) ? Y - y_s : n_u + (Y - y_l);
-    const float4 q0 = q[0], q1 = q[1], q4 = q[4];
-    const float lg[6] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
-    float sh[6];
-    if (k < n_u) {
-        const float4 q2 = q[2];
-        sh[0] = q1.z; sh[1] = q1.w; sh[2] = q2.x; sh[3] = q2.y; sh[4] = q2.z; sh[5] = q2.w;
-    } else {
-        const float4 q3 = q[3];
-        sh[0] = q3.x; sh[1] = q3.y; sh[2] = q3.z; sh[3] = q3.w; sh[4] = q4.x; sh[5] = q4.y;
+    const Quarter a = load_quarter(rp, 0);
+    const int y_s = (int)d.w[1], n_u = (int)d.w[2];
+    const uint32_t flags = d.w[3];
+    const bool upper = Y >= y_s && Y < y_s + n_u;
+    const Quarter s = load_quarter(rp, upper ? 1 : 2);
+    const int y_l = (int)s.w[6]; // (read in the lower half)
+    const int k = upper ? Y - y_s : n_u + (Y - y_l);
+    float lg[6], sh[6];
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+        lg[f] = __uint_as_float(a.w[f]);
+        sh[f] = __uint_as_float(s.w[f]);
     }
     RowIn r;
-    row_in(r, k, lg, sh, q4.z, q4.w, q5.x, y_s, y_l, n_u, flags);
+    row_in(r, k, lg, sh, __uint_as_float(a.w[6]), __uint_as_float(d.w[0]), __uint_as_float(a.w[7]), y_s, y_l, n_u, flags);
     RowSpan sp;
     row_span(r, v.x, v.w, sp);
     if (sp.x2 - sp.x1 > inline_span)
@@ -2006,16 +2095,15 @@ __device__ __forceinline__ uint32_t shade_winner_impl(const BatchDev *b, uint32_
     if (!in_bounds(r < b->list_cap, CHK_REC, r))
         return 0u;
     const TriRec *rp = b->recs + r;
-    const uint4 q6 = reinterpret_cast<const uint4 *>(rp)[6];
-    const uint4 q7 = reinterpret_cast<const uint4 *>(rp)[7];
-    const uint32_t flags = q6.y;
+    const Quarter d = load_quarter(rp, 3);
+    const uint32_t flags = d.w[3];
     if (flags == kRecClip)
         return shade_clip_px(it, i, slot);
     const int y = (int)(i / (uint32_t)v.w), x = (int)(i - (uint32_t)y * (uint32_t)v.w);
     float4 rec;
-    if (overflow || (flags & kRecTall) || !rec_replay(rp, v, b->inline_span, x + v.x, y + v.y, rec))
+    if (overflow || (flags & kRecTall) || !rec_replay(rp, d, v, b->inline_span, x + v.x, y + v.y, rec))
         rec = it.prec[i]; // recorded by the span kernels (or the overflow winner walk)
-    return shade_rec<ALL_MODES>(it, q7, flags, rec);
+    return shade_rec<ALL_MODES>(it, make_uint4(d.w[4], d.w[5], d.w[6], d.w[7]), flags, rec);
 }
 
 __device__ __forceinline__ SVert load_svert(const ItemDev &it, uint32_t g)
@@ -2053,10 +2141,14 @@ __device__ __forceinline__ uint32_t shade_rec(const ItemDev &it, uint4 q7, uint3
 // are reset to empty for the next launch sequence (unless kept for debug).
 constexpr int kShadeThreads = 256;
 #ifndef SGL_SHADE_MIN_BLOCKS
-#define SGL_SHADE_MIN_BLOCKS 5 // resident blocks per SM the shade is compiled for
+#define SGL_SHADE_MIN_BLOCKS 5 // resident blocks per SM the winner-list shade is compiled for
+#endif
+#ifndef SGL_TILE_MIN_BLOCKS
+#define SGL_TILE_MIN_BLOCKS 6 // ... and the tiled shade, which also hides its key loads and barriers with them (64
+                              // views: 511, 451 and 433 us at 4, 5 and 6 blocks)
 #endif
 template <int TILE, bool ALL_MODES>
-__global__ void __launch_bounds__(kShadeThreads, SGL_SHADE_MIN_BLOCKS) k_shade(const BatchDev *b)
+__global__ void __launch_bounds__(kShadeThreads, SGL_TILE_MIN_BLOCKS) k_shade(const BatchDev *b)
 {
     __shared__ uint4 queue[2 * kShadeThreads];
     __shared__ int qn;
@@ -2692,14 +2784,10 @@ __global__ void __launch_bounds__(256) k_frag_spans(const BatchDev *b)
         float top = r.top, bottom = r.bottom;
         for (int x0 = r.x1; x0 < r.x2; x0 += 32) {
             float mt = top, mb = bottom;
-#pragma unroll
-            for (int k = 0; k < 32; k++) {
-                if (k == lane) {
-                    mt = top;
-                    mb = bottom;
-                }
-                top = top + r.tstep;
-                bottom = bottom + r.bstep;
+            step2(mt, mb, r.tstep, r.bstep, lane);
+            if (x0 + 32 < r.x2) {
+                top = __shfl_sync(0xFFFFFFFFu, mt + r.tstep, 31);
+                bottom = __shfl_sync(0xFFFFFFFFu, mb + r.bstep, 31);
             }
             const int x = x0 + lane;
             if (x >= r.x2)
@@ -2738,11 +2826,10 @@ template <bool ALL_MODES>
 __device__ __forceinline__ uint32_t shade_frag(const BatchDev *b, const ItemDev &it, uint32_t item, uint32_t slot,
                                                float4 rec)
 {
-    const uint4 *q = reinterpret_cast<const uint4 *>(b->recs + __ldg(b->tri_base + item) + (slot >> 1));
-    const uint4 q6 = q[6];
-    if (q6.y == kRecClip)
+    const Quarter d = load_quarter(b->recs + __ldg(b->tri_base + item) + (slot >> 1), 3);
+    if (d.w[3] == kRecClip)
         return shade_clip_rec(it, slot, rec);
-    return shade_rec<ALL_MODES>(it, q[7], q6.y, rec);
+    return shade_rec<ALL_MODES>(it, make_uint4(d.w[4], d.w[5], d.w[6], d.w[7]), d.w[3], rec);
 }
 
 // One pixel with fragments: the opaque winner to the screen and the depth
@@ -2961,8 +3048,8 @@ cudaError_t launch_pose(const SceneDev &s, const float *node_world, const float 
 
 const char *prof_kernel_name(int k)
 {
-    static const char *names[kProfKernels] = {"k_geom",    "k_vertex",  "k_flags",  "k_compact", "k_setup",
-                                              "k_walk",    "k_spans",   "k_winners", "k_shade",  "k_dof",
+    static const char *names[kProfKernels] = {"k_geom",    "k_vertex",  "k_flags",  "k_compact", "k_walk",
+                                                 "k_spans",   "k_winners", "k_shade",  "k_dof",
                                               "k_frags",   "k_layers",  "k_flatten", "k_copy_layer"};
     return (k >= 0 && k < kProfKernels) ? names[k] : "?";
 }
@@ -3082,10 +3169,6 @@ cudaError_t launch_batch(const BatchDev *b, int tile, int flags, cudaStream_t st
         mark(PK_FLAGS);
         mark(PK_COMPACT);
     }
-    mark(PK_SETUP);
-    k_setup<<<sms * 8, 256, 0, st>>>(b);
-    ran(PK_SETUP);
-    n++;
     if (flags & kSeqLayers) {
         for (int k = PK_WALK; k <= PK_DOF; k++)
             mark(k);
@@ -3139,7 +3222,7 @@ cudaError_t launch_batch(const BatchDev *b, int tile, int flags, cudaStream_t st
     mark(PK_SHADE);
     // the kernel with every pixel shader only when a view asks for another
     // than the default, which then keeps all the registers
-    const unsigned sg = sms * SGL_SHADE_MIN_BLOCKS;
+    const unsigned sg = sms * ((flags & kSeqWinList) ? SGL_SHADE_MIN_BLOCKS : SGL_TILE_MIN_BLOCKS);
     if (flags & kSeqWinList) {
         k_classify<<<sms * 8, 256, 0, st>>>(b);
         if (flags & kSeqShaders)

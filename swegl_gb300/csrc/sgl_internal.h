@@ -193,29 +193,30 @@ static_assert(sizeof(SpanRec) == 52, "SpanRec layout");
 constexpr uint32_t kBitLower = 1u << 30; // span of the lower half-triangle
 constexpr uint32_t kBitLLR = 1u << 31;   // long_line_on_right
 constexpr uint32_t kYMask = (1u << 30) - 1u;
-constexpr int kTallRows = 16; // triangles walking more rows bin every span
+constexpr int kTallRows = 16; // triangles with more rows in the view are walked a warp each and bin every span
 
 // The scanline set-up of one drawable triangle (fill_triangle_2,
-// src/render/renderer.cpp:361-460), written by the walk and read back by the
-// shade kernel, which replays a winner's row and pixel steps from it instead
-// of repeating the set-up.  Vertices are in fill_triangle_2's y order
-// (v0, v1, v2).  Each edge is an interpolator_g<1> with its x, after the
-// displacement to the first row the walk visits: the long edge v0 -> v2 and
-// the upper short edge v0 -> v1 at row y_s, the lower short edge v1 -> v2 at
-// row y_l.  Row k of the walk (k < n_u: upper half, else lower half) sees the
-// long edge after k steps and its short edge after k (or k - n_u) steps.
-struct __align__(16) TriRec {
-    float lx, ltop, lbot, lratio;  // long edge
-    float ltstep, lbstep, ux, utop; // ... upper short edge
-    float ubot, uratio, utstep, ubstep;
-    float dx, dtop, dbot, dratio;   // lower short edge
-    float dtstep, dbstep, z0, z1;   // z' of v0, v1, v2
-    float z2;
-    int y_s, y_l, n_u;
-    int n_d;
-    uint32_t flags;                 // kRecLLRUpper | kRecLLRLower | kRecFFV | kRecTall
+// src/render/renderer.cpp:361-460), made by the walk and, when the triangle
+// has fragments, written for the shade kernel, which replays a winner's row
+// and pixel steps from it instead of repeating the set-up.  Vertices are in
+// fill_triangle_2's y order (v0, v1, v2).  Each edge is an interpolator_g<1>
+// with its x, after the displacement to the first row the walk visits: the
+// long edge v0 -> v2 and the upper short edge v0 -> v1 at row y_s, the lower
+// short edge v1 -> v2 at row y_l.  Row k of the walk (k < n_u: upper half,
+// else lower half) sees the long edge after k steps and its short edge after
+// k (or k - n_u) steps.  A shaded fragment reads the first, the last and one
+// of the two middle 32-byte quarters.
+struct __align__(32) TriRec {
+    float lx, ltop, lbot, lratio, ltstep, lbstep; // long edge
+    float z0, z2;                                 // z' of v0, v2
+    float ux, utop, ubot, uratio, utstep, ubstep; // upper short edge
     uint32_t slot, item;
-    uint32_t g0, g1, g2, prim;      // vertices of v0, v1, v2; draw-order primitive
+    float dx, dtop, dbot, dratio, dtstep, dbstep; // lower short edge
+    int y_l, n_d;
+    float z1; // z' of v1
+    int y_s, n_u;
+    uint32_t flags;            // kRecLLRUpper | kRecLLRLower | kRecFFV | kRecTall
+    uint32_t g0, g1, g2, prim; // vertices of v0, v1, v2; draw-order primitive
 };
 static_assert(sizeof(TriRec) == 128, "TriRec layout");
 constexpr uint32_t kRecLLRUpper = 1u; // long_line_on_right in the upper half
@@ -225,7 +226,7 @@ constexpr uint32_t kRecTall = 8u;     // every span was binned (winners recorded
 // The flags word of the record slot of a near-clipped triangle (written by the
 // geometry passes; such a triangle gets no set-up record).
 constexpr uint32_t kRecClip = 0xFFFFFFFFu;
-constexpr int kRecFlagsWord = 25; // 32-bit word of TriRec::flags
+constexpr int kRecFlagsWord = 27; // 32-bit word of TriRec::flags
 static_assert(offsetof(TriRec, flags) == 4 * kRecFlagsWord, "TriRec::flags word");
 
 // Batch counters (32-bit words); the drawn-triangle and fragment counts are
@@ -261,9 +262,9 @@ struct BatchDev {
     uint32_t list_cap;
     uint2 *clip;               // drawable triangles crossing the near plane {t, item}: entry j at clip[clip_cap - 1 - j]
     uint32_t clip_cap;
-    TriRec *recs;              // per batch triangle (tri_base[item] + t): the scanline set-up of a walk-list
-                               // triangle, or flags kRecClip for a near-clipped one (others: stale)
-    uint32_t *tall;            // batch triangles of the tall set-ups (list_cap entries)
+    TriRec *recs;              // per batch triangle (tri_base[item] + t): the scanline set-up of a walked
+                               // triangle with fragments, or flags kRecClip for a near-clipped one (others: stale)
+    uint32_t *tall;            // batch triangles walked a warp each (list_cap entries; not in `list`)
     int keep_keys;             // leave the depth keys for the caller (debug); else the shade resets them
     unsigned long long *key_pool; // the items' depth keys: batch pixel px_base[item] + i at key_pool[...]
     uint2 *wins;               // kSeqWinList: pixels with a winner {batch pixel, draw slot}, in pixel order
@@ -278,9 +279,9 @@ struct BatchDev {
 
 // Optional per-kernel timing: CUDA events recorded on the launching stream
 // around each stage of a launch sequence (enabled with sgl_profile).
-constexpr int kProfKernels = 14;
+constexpr int kProfKernels = 13;
 enum ProfKernel {
-    PK_GEOM = 0, PK_VERTEX, PK_FLAGS, PK_COMPACT, PK_SETUP, PK_WALK, PK_SPANS, PK_WINNER, PK_SHADE, PK_DOF,
+    PK_GEOM = 0, PK_VERTEX, PK_FLAGS, PK_COMPACT, PK_WALK, PK_SPANS, PK_WINNER, PK_SHADE, PK_DOF,
     PK_FRAGS, PK_LAYERS, PK_FLATTEN, PK_COPY
 };
 struct Profiler {
