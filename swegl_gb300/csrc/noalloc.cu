@@ -202,7 +202,7 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     off += dof ? up256(8 * px) : 0;
     const size_t o_spans = off;
     const size_t min_spans = 4096;
-    const size_t need = o_spans + min_spans * sizeof(SpanRec);
+    const size_t need = o_spans + min_spans * kSpanBytes;
     if (need > kNoAllocScratchBytes || px >= (1ull << 32) || tiles >= (1ull << 32)) {
         ctx->fail("sgl_render_noalloc: this view of scene %d needs %zu bytes of scratch; the static scratch "
                   "holds %zu bytes (use sgl_render, or a smaller view or scene)",
@@ -215,7 +215,7 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
         ctx->fail("sgl_render_noalloc: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
         return SGL_ERR_CUDA;
     }
-    const uint32_t span_cap = (uint32_t)((kNoAllocScratchBytes - o_spans) / sizeof(SpanRec));
+    const uint32_t span_cap = (uint32_t)((kNoAllocScratchBytes - o_spans) / kSpanBytes);
     ItemDev it{};
     it.s = s->dev;
     it.v = make_view(v);
@@ -254,8 +254,8 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     const bool split = !fused || s->dev.mixed != 0; // the general passes run (all, or the larger primitives)
     // prefixes of one item (vertices, triangles, pixels, tiles, depth-of-field
     // tiles, the general geometry pass's vertices and triangles), then the
-    // fused pass's one group: its chunks, its items, the item
-    const uint32_t chunks = fused ? (s->dev.n_prims + kGeomWarps - 1) / kGeomWarps : 0u;
+    // fused pass's one group: its units, its items, the item
+    const uint32_t chunks = fused ? geom_units(s->dev.n_prims, 1) : 0u;
     const NoAllocBases bases = {{0u, (uint32_t)nv,              0u, (uint32_t)nt,
                                  0u, (uint32_t)px,              0u, (uint32_t)tiles,
                                  0u, dof_tiles,                 0u, split ? (uint32_t)nv : 0u,
@@ -291,7 +291,7 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     b.keep_keys = 0;
     b.key_pool = (unsigned long long *)(base + o_key);
     b.wins = win_list ? (uint2 *)(base + o_wins) : nullptr;
-    b.spans = (SpanRec *)(base + o_spans);
+    b.spans = base + o_spans;
     b.span_cap = span_cap;
     b.counters = (unsigned long long *)(base + o_counters);
     b.item_counters = (unsigned long long *)(base + o_item_counters);

@@ -235,12 +235,12 @@ __global__ void __launch_bounds__(256) k_vertex(const BatchDev *b)
 }
 
 // inside_camera_frustum (src/render/renderer.cpp:58-70)
+// (a >= k || b >= k || c >= k is max(a, b, c) >= k, NaNs ignored alike)
 __device__ __forceinline__ bool inside_frustum(V3 a, V3 b, V3 c)
 {
-    return (a.x >= -1.0f || b.x >= -1.0f || c.x >= -1.0f) && (a.y >= -1.0f || b.y >= -1.0f || c.y >= -1.0f) &&
-           (a.x < 1.0f || b.x < 1.0f || c.x < 1.0f) && (a.y < 1.0f || b.y < 1.0f || c.y < 1.0f) &&
-           (at_or_past_near(a.z) || at_or_past_near(b.z) || at_or_past_near(c.z)) && (a.x != b.x || a.x != c.x) &&
-           (a.y != b.y || a.y != c.y);
+    return fmaxf(fmaxf(a.x, b.x), c.x) >= -1.0f && fmaxf(fmaxf(a.y, b.y), c.y) >= -1.0f &&
+           fminf(fminf(a.x, b.x), c.x) < 1.0f && fminf(fminf(a.y, b.y), c.y) < 1.0f &&
+           at_or_past_near(fmaxf(fmaxf(a.z, b.z), c.z)) && (a.x != b.x || a.x != c.x) && (a.y != b.y || a.y != c.y);
 }
 
 __device__ __forceinline__ V3 ld3(const float4 *a, uint32_t i)
@@ -333,68 +333,23 @@ __device__ __forceinline__ V3 load_vp(const ItemDev &it, uint32_t g)
     return mk3(it.v.vm00 * n.x + it.v.vm03, it.v.vm11 * n.y + it.v.vm13, n.z);
 }
 
-// Per-item counters of a warp: lanes grouped by item, one atomic per group.
-__device__ __forceinline__ void item_add(unsigned long long *dst, uint32_t item, unsigned long long v, bool valid)
+// The lanes' counts added to their items' counters (item_counters[2 item +
+// which]: 0 drawn triangles, 1 fragments), one atomic per distinct item.
+// Every lane of the warp calls it.
+__device__ __forceinline__ void item_add(const BatchDev *b, int which, uint32_t item, unsigned long long n, bool valid)
 {
-    const unsigned act = __ballot_sync(0xFFFFFFFFu, valid);
-    if (!valid)
+    const unsigned act = __ballot_sync(0xFFFFFFFFu, valid && n);
+    if (!(valid && n))
         return;
+    if (__any_sync(act, n >> 26)) { // the sum of 32 might not fit
+        atomicAdd(b->item_counters + 2 * (size_t)item + which, n);
+        return;
+    }
     const unsigned grp = __match_any_sync(act, item);
-    unsigned long long sum = 0;
-    for (unsigned m = grp; m; m &= m - 1)
-        sum += __shfl_sync(grp, v, __ffs(m) - 1);
-    if ((threadIdx.x & 31) == __ffs(grp) - 1 && sum)
-        atomicAdd(dst + 2 * (size_t)item, sum);
+    const uint32_t sum = __reduce_add_sync(grp, (uint32_t)n);
+    if ((threadIdx.x & 31) == __ffs(grp) - 1)
+        atomicAdd(b->item_counters + 2 * (size_t)item + which, (unsigned long long)sum);
 }
-
-__device__ __forceinline__ void warp_add(unsigned long long *dst, unsigned long long v)
-{
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-    if ((threadIdx.x & 31) == 0 && v)
-        atomicAdd(dst, v);
-}
-
-// Per-item counters (drawn triangles, fragments) of a warp, summed in
-// registers while all of the warp's lanes work on one item and added to the
-// item's counters when the item changes (one atomic per counter then); an
-// iteration whose lanes span several items adds per item at once.  Every
-// lane of the warp calls add() and flush().
-struct ItemAcc {
-    uint32_t item = 0xFFFFFFFFu;
-    unsigned long long v0 = 0, v1 = 0;
-
-    __device__ __forceinline__ void flush(const BatchDev *b)
-    {
-        if (item != 0xFFFFFFFFu) {
-            warp_add(b->item_counters + 2 * (size_t)item, v0);
-            warp_add(b->item_counters + 2 * (size_t)item + 1, v1);
-        }
-        item = 0xFFFFFFFFu;
-        v0 = v1 = 0;
-    }
-    __device__ __forceinline__ void add(const BatchDev *b, uint32_t it, unsigned long long a0, unsigned long long a1,
-                                        bool valid)
-    {
-        const unsigned act = __ballot_sync(0xFFFFFFFFu, valid);
-        if (!act)
-            return;
-        const uint32_t first = __shfl_sync(0xFFFFFFFFu, it, __ffs(act) - 1);
-        if (__all_sync(0xFFFFFFFFu, !valid || it == first)) {
-            if (first != item) {
-                flush(b);
-                item = first;
-            }
-            if (valid) {
-                v0 += a0;
-                v1 += a1;
-            }
-        } else {
-            item_add(b->item_counters, it, a0, valid);
-            item_add(b->item_counters + 1, it, a1, valid);
-        }
-    }
-};
 
 // The record slot of a near-clipped batch triangle: flags = kRecClip.
 __device__ __forceinline__ void mark_clip(const BatchDev *b, uint32_t r)
@@ -462,7 +417,6 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
     const uint8_t *yes = nullptr;
     const uint8_t *psmall = nullptr; // a mixed scene: primitives of the fused pass
     const uint32_t total = b->total_gtri;
-    ItemAcc acc; // triangles counted as drawn here (no pixel column)
     // every thread of the block runs the same number of iterations (barriers inside)
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t g0 = blockIdx.x * blockDim.x; g0 < total; g0 += stride) {
@@ -471,7 +425,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
         __syncthreads();
         const uint32_t g = g0 + threadIdx.x;
         int list = -1; // 0 walk list, 1 clip list, 2 tall list
-        bool xsliver = false;
+        bool counted = false; // reached fill_triangle_2's set-up
         uint32_t t = 0;
         if (g < total) {
             if (g < lo || g >= hi) {
@@ -506,6 +460,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
                             // the set-up or the walk, and is not counted
                             list = -1;
                         } else {
+                            counted = true;
                             // No pixel column either: every row's span [ceil(xl),
                             // ceil(xr)) is empty when the triangle's x range, widened
                             // by the walk's rounding, holds no integer boundary.  The
@@ -525,7 +480,6 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
                             const float hi_x = fmaxf(x0, fmaxf(x1, x2)) + eps;
                             if (ceilf(lo_x) == ceilf(hi_x)) {
                                 list = -1;
-                                xsliver = true;
                                 if (b->slot_flags)
                                     b->slot_flags[2 * t] = 1;
                             } else if (tall_rows(lo_y, hi_y, it.v.y, it.v.y + it.v.h)) {
@@ -537,7 +491,7 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
             }
         }
         list_tall(b, list == 2, list == 2 ? __ldg(b->tri_base + item) + t : 0u);
-        acc.add(b, (uint32_t)item, 1ull, 0ull, xsliver);
+        item_add(b, 0, (uint32_t)item, 1u, counted);
         uint32_t pos = 0;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
@@ -570,7 +524,6 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
         }
         __syncthreads();
     }
-    acc.flush(b);
 }
 
 // The geometry of fused scenes (every primitive within kFuseVerts vertices
@@ -583,28 +536,41 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
 //
 // Items are taken in groups that read the same vertex data (the views of one
 // scene in the batch; the reference likewise transforms a scene to world
-// space once for all the viewports of a render call, renderer.hpp:27-34).
-// A block takes a chunk of kGeomWarps consecutive primitives of a group and
-// runs each warp's primitive for every item of the group: the primitive's
-// first 64 triangles stay in registers as local vertex indices and its world
-// positions are read again per item (from L1 after the first).  The items go
-// in passes of kGeomPass: per item the warp records its walk-list and
-// clip-list decisions as ballot masks, and after the pass one global atomic
-// reserves both lists for all the pass's items and warps (reserve_lists).
-constexpr int kGeomPass = 8;            // items per list reservation
+// space once for all the viewports of a render call, renderer.hpp:27-34).  A
+// block takes kGeomWarps consecutive primitives and up to kGeomItems items of
+// a group and runs each warp's primitive for each of the items: the primitive's first 64 triangles stay in registers as local vertex
+// indices and its world positions are read again per item (from L1 after the
+// first).  Per item the warp records its walk-list and clip-list decisions as
+// ballot masks, and at the end one global atomic reserves both lists for all
+// the unit's items and warps (reserve_lists).
+//
+// The pass is bound by instruction issue and by the latency of its load chain
+// (about 1,000 instructions a primitive and view before, at 49 % issue).  So a
+// vertex is one 16-byte word of shared memory with its flags in w, the
+// unit's cameras are staged once for the block, a primitive without a
+// visible triangle (about half of a closed mesh's) stops after the visibility
+// test, and projected vertices are stored only for primitives with an entry
+// in a list, which are all that the later passes read: 64 views 691 -> 573 us,
+// of 200 spheres.
+constexpr int kGeomVerts = 2;           // vertices of a lane with loads in flight (four spill registers: 683 us for 573)
 constexpr int kGeomTG = kFuseTris / 32; // groups of 32 triangles
 constexpr int kGeomBlocks = 4;          // resident blocks per SM the pass is compiled for
+// words of an item's camera in shared memory: view and projection rows 0-2, then
+enum { GV_VM00 = 24, GV_VM03, GV_VM11, GV_VM13, GV_Y, GV_YEND, GV_ITEM, GV_TRI, kGeomViewWords };
+static_assert(kGeomViewWords == 32, "a warp stages an item's camera, a word per lane");
 struct GeomShared {
-    float pos[kGeomWarps][3 * kFuseVerts];         // x, y, z' of each vertex (for the item in hand)
-    uint8_t yes[kGeomWarps][kFuseVerts];
-    uint32_t walk[kGeomPass][kGeomWarps][kGeomTG]; // per 32 triangles: ballot of the walk list
-    uint32_t clip[kGeomPass][kGeomWarps][kGeomTG]; // ... of the clip list
-    uint32_t cnt[kGeomPass][kGeomWarps][2];        // entries of each list, then their first positions
-    uint32_t nx[kGeomPass][kGeomWarps];            // drawable triangles without a pixel column
-    float view[kGeomWarps][30];                    // the warp's copy of the item in hand: view and projection
-                                                   // rows 0-2, vm00, vm03, vm11, vm13, first and end row
+    float4 pos[kGeomWarps][kFuseVerts];             // x, y, z' and flags of each vertex (for the item in hand)
+    float view[kGeomItems][kGeomViewWords];         // the unit's cameras
+    float4 *ndc[kGeomItems];                        // ... and projected vertices
+    uint32_t walk[kGeomItems][kGeomWarps][kGeomTG]; // per 32 triangles: ballot of the walk list
+    uint32_t clip[kGeomItems][kGeomWarps][kGeomTG]; // ... of the clip list
+    uint32_t cnt[kGeomItems * kGeomWarps];          // entries: walk list | clip list << 16
+    uint32_t off[kGeomItems * kGeomWarps];          // ... of the items and warps before
+    uint32_t nx[kGeomItems];                        // triangles that reach fill_triangle_2's set-up
+    uint32_t base[2];                               // the block's first position in each list
 };
 static_assert(kFuseVerts <= 256, "local vertex indices are bytes");
+static_assert(kGeomItems * kGeomWarps == 64 && 64 * kFuseTris < 65536, "a warp scans the counts, two a lane, in 16 bits");
 constexpr size_t kGeomSmem = sizeof(GeomShared);
 
 // The local vertex indices of triangle t of a fused primitive (a | b << 8 | c << 16).
@@ -633,7 +599,7 @@ __device__ __forceinline__ uint32_t geom_unseen(const BatchDev *b, const float4 
     const unsigned m = __ballot_sync(0xFFFFFFFFu, out);
     uint32_t u = 0;
 #pragma unroll
-    for (int i = 0; i < kGeomPass; i++)
+    for (int i = 0; i < kGeomItems; i++)
         u |= ((m >> (4 * i)) & 15u) ? 1u << i : 0u;
     return u;
 }
@@ -645,27 +611,55 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
     const int warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    float *pos = S.pos[warp];
-    uint8_t *sy = S.yes[warp];
-    float *vw = S.view[warp];
-    int g = -1;
-    uint32_t c_lo = 0, c_hi = 0;
+    float4 *pos = S.pos[warp];
+    uint32_t c_lo = 0, c_hi = 0, g_lo = 0, g_n = 0, passes = 1, i_lo = 0xFFFFFFFFu;
+    int nv = 0;
     const uint32_t total = b->total_chunks;
     // every thread of the block runs the same iterations (barriers inside)
     for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
+        __syncthreads(); // the previous unit's masks and cameras are read
         if (c < c_lo || c >= c_hi) {
-            g = find_item(b->grp_chunk_base, b->n_groups, c);
+            const int g = find_item(b->grp_chunk_base, b->n_groups, c);
             c_lo = __ldg(b->grp_chunk_base + g);
             c_hi = __ldg(b->grp_chunk_base + g + 1);
+            g_lo = __ldg(b->grp_item_base + g);
+            g_n = __ldg(b->grp_item_base + g + 1) - g_lo;
+            passes = (g_n + kGeomItems - 1) / kGeomItems;
         }
-        const uint32_t i_lo = __ldg(b->grp_item_base + g), i_hi = __ldg(b->grp_item_base + g + 1);
+        const uint32_t chunk = passes == 1 ? c - c_lo : (c - c_lo) / passes, first = (c - c_lo - chunk * passes) * kGeomItems;
+        if (g_lo + first != i_lo) {
+            i_lo = g_lo + first;
+            nv = (int)min((uint32_t)kGeomItems, g_n - first);
+            // warp vi stages item vi's camera (kGeomItems <= kGeomWarps)
+            if (warp < nv) {
+                const uint32_t item = __ldg(b->grp_items + i_lo + warp);
+                const ItemDev &it = b->items[item];
+                float x;
+                if (lane < 12)
+                    x = it.v.view[lane];
+                else if (lane < 24)
+                    x = it.v.proj[lane - 12];
+                else if (lane < GV_Y)
+                    x = (&it.v.vm00)[lane - GV_VM00];
+                else
+                    x = __uint_as_float(lane == GV_Y      ? (uint32_t)it.v.y
+                                        : lane == GV_YEND ? (uint32_t)(it.v.y + it.v.h)
+                                        : lane == GV_ITEM ? item
+                                                          : __ldg(b->tri_base + item));
+                S.view[warp][lane] = x;
+                if (lane == 0)
+                    S.ndc[warp] = it.ndc;
+            }
+        }
+        if (threadIdx.x < kGeomItems)
+            S.nx[threadIdx.x] = 0;
         const SceneDev &sc = b->items[__ldg(b->grp_items + i_lo)].s; // vertex data shared by the group
-        const uint32_t q = (c - c_lo) * kGeomWarps + warp;             // this warp's primitive
+        const uint32_t q = chunk * kGeomWarps + warp;                  // this warp's primitive
         const bool has = q < sc.n_prims && (!sc.psmall || sc.psmall[q]); // (a mixed scene's larger ones: general passes)
         uint4 gq = make_uint4(0u, 0u, 0u, 0u); // first vertex, vertex count, first triangle, triangle count
         bool ds = false;
         uint32_t tr0 = 0, tr1 = 0; // the first 64 triangles, local vertex indices
-        uint32_t unseen = 0; // bit vi: item vi of the pass in hand sees none of the primitive
+        uint32_t unseen = 0;       // bit vi: item vi sees none of the primitive
         const float4 *wpos = sc.wpos;
         const uint4 *tris = sc.tris;
         if (has) {
@@ -677,106 +671,93 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
             if (lane + 32 < gq.w)
                 tr1 = geom_tri(tris, gq, lane + 32);
             ds = sc.pshade[q].double_sided != 0;
+            if (sc.pbox)
+                unseen = geom_unseen(b, sc.pbox, q, i_lo, (uint32_t)nv, lane);
         }
-        for (uint32_t v0 = i_lo; v0 < i_hi; v0 += kGeomPass) {
-            const int nv = (int)min((uint32_t)kGeomPass, i_hi - v0);
-            if (has && sc.pbox)
-                unseen = geom_unseen(b, sc.pbox, q, v0, (uint32_t)nv, lane);
-            for (int vi = 0; vi < nv; vi++) {
-                uint32_t c0 = 0, c1 = 0, nx = 0;
-                const bool seen = has && !((unseen >> vi) & 1u);
-                if (!seen && has) {
-                    // the item sees none of the primitive's triangles
-                    if (lane < (uint32_t)kGeomTG) {
-                        S.walk[vi][warp][lane] = 0u;
-                        S.clip[vi][warp][lane] = 0u;
-                    }
-                }
-                if (seen) {
-                    const uint32_t item = __ldg(b->grp_items + v0 + vi);
-                    const ItemDev &it = b->items[item];
-                    __syncwarp(); // the previous item's reads of pos, sy and vw are done
-                    if (lane < 12) {
-                        vw[lane] = it.v.view[lane];
-                        vw[12 + lane] = it.v.proj[lane];
-                    } else if (lane == 12) {
-                        vw[24] = it.v.vm00;
-                        vw[25] = it.v.vm03;
-                        vw[26] = it.v.vm11;
-                        vw[27] = it.v.vm13;
-                        vw[28] = __int_as_float(it.v.y);
-                        vw[29] = __int_as_float(it.v.y + it.v.h);
-                    }
-                    float4 *ndc = it.ndc + gq.x;
-                    __syncwarp();
-                    // world_to_camera_or_frustum (vertex_shaders.hpp:35-52), as
-                    // k_vertex; 128 vertices per round, their loads issued first
-                    for (uint32_t i0 = 0; i0 < gq.y; i0 += 128) {
-                        float4 w[4];
+        wpos += gq.x;
+        __syncthreads(); // the cameras are staged
+        for (int vi = 0; vi < nv; vi++) {
+            uint32_t entries = 0;
+            if (has && !((unseen >> vi) & 1u)) {
+                const float *vw = S.view[vi];
+                __syncwarp(); // the previous item's reads of pos are done
+                // world_to_camera_or_frustum (vertex_shaders.hpp:35-52), as
+                // k_vertex; kGeomVerts vertices a lane and round, their loads issued first
+                bool behind = false;
+                {
+                    float m[24];
 #pragma unroll
-                        for (int k = 0; k < 4; k++)
+                    for (int k = 0; k < 6; k++)
+                        reinterpret_cast<float4 *>(m)[k] = reinterpret_cast<const float4 *>(vw)[k];
+                    for (uint32_t i0 = 0; i0 < gq.y; i0 += 32 * kGeomVerts) {
+                        float4 w[kGeomVerts];
+#pragma unroll
+                        for (int k = 0; k < kGeomVerts; k++)
                             if (i0 + lane + 32 * k < gq.y)
-                                w[k] = wpos[gq.x + i0 + lane + 32 * k];
+                                w[k] = wpos[i0 + lane + 32 * k];
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
+                        for (int k = 0; k < kGeomVerts; k++) {
                             const uint32_t i = i0 + lane + 32 * k;
                             if (i < gq.y) {
-                                V3 v = transform3(mk3(w[k].x, w[k].y, w[k].z), vw);
-                                v = transform3(v, vw + 12);
+                                V3 v = transform3(mk3(w[k].x, w[k].y, w[k].z), m);
+                                v = transform3(v, m + 12);
                                 if (v.z != 0.0f) {
                                     v.x = v.x / fabsf(v.z);
                                     v.y = v.y / fabsf(v.z);
                                 }
-                                if (in_bounds(gq.x + i < sc.n_vertices, CHK_NDC, gq.x + i))
-                                    ndc[i] = make_float4(v.x, v.y, v.z, 0.0f);
-                                pos[3 * i] = v.x;
-                                pos[3 * i + 1] = v.y;
-                                pos[3 * i + 2] = v.z;
-                                sy[i] = below_near(v.z) ? kYesBehind : 0;
+                                const bool near = below_near(v.z);
+                                behind |= near;
+                                pos[i] = make_float4(v.x, v.y, v.z, __uint_as_float(near ? kYesBehind : 0u));
                             }
                         }
                     }
-                    __syncwarp();
-                    // visibility flags (renderer.cpp:86-185), as k_flags; every
-                    // store to a vertex writes the same value
-                    for (uint32_t t = lane; t < gq.w; t += 32) {
-                        const uint32_t tp = t < 32 ? tr0 : (t < 64 ? tr1 : geom_tri(tris, gq, t));
-                        const uint32_t ia = tp & 0xFFu, ib = (tp >> 8) & 0xFFu, ic = tp >> 16;
-                        const V3 a = mk3(pos[3 * ia], pos[3 * ia + 1], pos[3 * ia + 2]);
-                        const V3 c1v = mk3(pos[3 * ib], pos[3 * ib + 1], pos[3 * ib + 2]);
-                        const V3 c2v = mk3(pos[3 * ic], pos[3 * ic + 1], pos[3 * ic + 2]);
-                        if (inside_frustum(a, c1v, c2v) && (ds || cross_z_positive(sub3(c1v, a), sub3(c2v, a)))) {
-                            sy[ia] = kYesDrawn | (below_near(a.z) ? kYesBehind : 0);
-                            sy[ib] = kYesDrawn | (below_near(c1v.z) ? kYesBehind : 0);
-                            sy[ic] = kYesDrawn | (below_near(c2v.z) ? kYesBehind : 0);
-                        }
+                }
+                behind = __any_sync(0xFFFFFFFFu, behind);
+                // visibility flags (renderer.cpp:86-185), as k_flags; every
+                // store to a vertex writes the same value
+                bool any = false;
+                for (uint32_t t = lane; t < gq.w; t += 32) {
+                    const uint32_t tp = t < 32 ? tr0 : (t < 64 ? tr1 : geom_tri(tris, gq, t));
+                    float4 &pa = pos[tp & 0xFFu], &pb = pos[(tp >> 8) & 0xFFu], &pc = pos[tp >> 16];
+                    const float4 fa = pa, fb = pb, fc = pc;
+                    const V3 a = mk3(fa.x, fa.y, fa.z), c1 = mk3(fb.x, fb.y, fb.z), c2 = mk3(fc.x, fc.y, fc.z);
+                    if (inside_frustum(a, c1, c2) && (ds || cross_z_positive(sub3(c1, a), sub3(c2, a)))) {
+                        any = true;
+                        pa.w = __uint_as_float(__float_as_uint(fa.w) | kYesDrawn);
+                        pb.w = __uint_as_float(__float_as_uint(fb.w) | kYesDrawn);
+                        pc.w = __uint_as_float(__float_as_uint(fc.w) | kYesDrawn);
                     }
+                }
+                if (__any_sync(0xFFFFFFFFu, any)) {
                     __syncwarp();
                     // the compaction's decisions, as k_compact
-                    const float vm00 = vw[24], vm03 = vw[25], vm11 = vw[26], vm13 = vw[27];
+                    const float vm00 = vw[GV_VM00], vm03 = vw[GV_VM03], vm11 = vw[GV_VM11], vm13 = vw[GV_VM13];
+                    uint32_t nx = 0;
+                    bool listed = false;
                     for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
                         const uint32_t t = t0 + lane;
                         int d = 0; // 0 none, 1 walk list, 2 clip list, 3 no pixel column, 4 tall list
+                        bool counted = false;
                         if (t < gq.w) {
                             const uint32_t tp = t < 32 ? tr0 : (t < 64 ? tr1 : geom_tri(tris, gq, t));
-                            const uint32_t ia = tp & 0xFFu, ib = (tp >> 8) & 0xFFu, ic = tp >> 16;
-                            const uint32_t ya = sy[ia], yb = sy[ib], yc = sy[ic];
+                            const float4 fa = pos[tp & 0xFFu], fb = pos[(tp >> 8) & 0xFFu], fc = pos[tp >> 16];
+                            const uint32_t ya = __float_as_uint(fa.w), yb = __float_as_uint(fb.w),
+                                           yc = __float_as_uint(fc.w);
                             if (ya & yb & yc & kYesDrawn) {
-                                if ((ya | yb | yc) & kYesBehind) {
+                                if (behind && ((ya | yb | yc) & kYesBehind)) {
                                     d = 2;
                                 } else {
                                     d = 1;
-                                    const float y0 = vm11 * pos[3 * ia + 1] + vm13;
-                                    const float y1 = vm11 * pos[3 * ib + 1] + vm13;
-                                    const float y2 = vm11 * pos[3 * ic + 1] + vm13;
+                                    const float y0 = vm11 * fa.y + vm13, y1 = vm11 * fb.y + vm13,
+                                                y2 = vm11 * fc.y + vm13;
                                     const float lo_y = fminf(y0, fminf(y1, y2)), hi_y = fmaxf(y0, fmaxf(y1, y2));
                                     if (y0 == y0 && y1 == y1 && y2 == y2) {
                                         if (f2i(ceilf(lo_y)) == f2i(ceilf(hi_y))) {
                                             d = 0; // no row
                                         } else {
-                                            const float x0 = vm00 * pos[3 * ia] + vm03;
-                                            const float x1 = vm00 * pos[3 * ib] + vm03;
-                                            const float x2 = vm00 * pos[3 * ic] + vm03;
+                                            counted = true;
+                                            const float x0 = vm00 * fa.x + vm03, x1 = vm00 * fb.x + vm03,
+                                                        x2 = vm00 * fc.x + vm03;
                                             const float mx = fmaxf(fabsf(x0), fmaxf(fabsf(x1), fabsf(x2)));
                                             const float rows = ceilf(hi_y) - ceilf(lo_y);
                                             const float eps = (rows + 32.0f) * 0x1p-23f * (mx + 1.0f);
@@ -786,8 +767,8 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                                                 d = 3; // no pixel column
                                                 if (b->slot_flags)
                                                     b->slot_flags[2 * (gq.z + t)] = 1;
-                                            } else if (tall_rows(lo_y, hi_y, __float_as_int(vw[28]),
-                                                                 __float_as_int(vw[29]))) {
+                                            } else if (tall_rows(lo_y, hi_y, __float_as_int(vw[GV_Y]),
+                                                                 __float_as_int(vw[GV_YEND]))) {
                                                 d = 4;
                                             }
                                         }
@@ -795,77 +776,83 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                                 }
                             }
                         }
-                        if (__any_sync(0xFFFFFFFFu, d == 4))
-                            list_tall(b, d == 4, __ldg(b->tri_base + item) + gq.z + t);
+                        if (__any_sync(0xFFFFFFFFu, d == 4)) {
+                            list_tall(b, d == 4, __float_as_uint(vw[GV_TRI]) + gq.z + t);
+                            listed = true;
+                        }
                         const unsigned m1 = __ballot_sync(0xFFFFFFFFu, d == 1);
-                        const unsigned m2 = __ballot_sync(0xFFFFFFFFu, d == 2);
-                        const unsigned m3 = __ballot_sync(0xFFFFFFFFu, d == 3);
+                        const unsigned m2 = behind ? __ballot_sync(0xFFFFFFFFu, d == 2) : 0u;
+                        const unsigned m3 = __ballot_sync(0xFFFFFFFFu, counted);
                         if (lane == 0) {
                             S.walk[vi][warp][t0 >> 5] = m1;
                             S.clip[vi][warp][t0 >> 5] = m2;
                         }
-                        c0 += __popc(m1);
-                        c1 += __popc(m2);
+                        entries += __popc(m1) | (__popc(m2) << 16);
                         nx += __popc(m3);
                     }
-                }
-                if (lane == 0) {
-                    S.cnt[vi][warp][0] = c0;
-                    S.cnt[vi][warp][1] = c1;
-                    S.nx[vi][warp] = nx;
+                    // the later passes read the projected vertices of listed
+                    // triangles alone
+                    if (listed || entries) {
+                        float4 *ndc = S.ndc[vi] + gq.x;
+                        for (uint32_t i = lane; i < gq.y; i += 32)
+                            if (in_bounds(gq.x + i < sc.n_vertices, CHK_NDC, gq.x + i))
+                                ndc[i] = pos[i];
+                    }
+                    if (lane == 0 && nx)
+                        atomicAdd(&S.nx[vi], nx);
                 }
             }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                // first positions per item and warp, one reservation for the pass
-                uint32_t n0 = 0, n1 = 0;
-                for (int vi = 0; vi < nv; vi++) {
-                    uint32_t x = 0;
-                    for (int w = 0; w < kGeomWarps; w++) {
-                        const uint32_t a0 = S.cnt[vi][w][0], a1 = S.cnt[vi][w][1];
-                        S.cnt[vi][w][0] = n0;
-                        S.cnt[vi][w][1] = n1;
-                        n0 += a0;
-                        n1 += a1;
-                        x += S.nx[vi][w];
-                    }
-                    // triangles counted as drawn here: they reached fill_triangle_2's set-up
-                    if (x)
-                        atomicAdd(b->item_counters + 2 * (size_t)__ldg(b->grp_items + v0 + vi), (unsigned long long)x);
-                }
-                const unsigned long long old = reserve_lists(b, n0, n1);
-                const uint32_t g0 = (uint32_t)old, g1 = (uint32_t)(old >> 32);
-                for (int vi = 0; vi < nv; vi++)
-                    for (int w = 0; w < kGeomWarps; w++) {
-                        S.cnt[vi][w][0] += g0;
-                        S.cnt[vi][w][1] += g1;
-                    }
+            if (lane == 0)
+                S.cnt[vi * kGeomWarps + warp] = entries;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // first positions per item and warp (two a lane), one reservation
+            const int k = 2 * (int)lane;
+            const uint32_t a = k < nv * kGeomWarps ? S.cnt[k] : 0u, z = k < nv * kGeomWarps ? S.cnt[k + 1] : 0u;
+            uint32_t incl = a + z;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if ((int)lane >= d)
+                    incl += u;
             }
-            __syncthreads();
-            if (has) {
-                for (int vi = 0; vi < nv; vi++) {
-                    uint32_t o0 = S.cnt[vi][warp][0], o1 = S.cnt[vi][warp][1];
-                    const uint32_t item = __ldg(b->grp_items + v0 + vi);
-                    const uint32_t tlo = __ldg(b->tri_base + item);
-                    for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
-                        const unsigned m1 = S.walk[vi][warp][t0 >> 5], m2 = S.clip[vi][warp][t0 >> 5];
-                        const uint32_t t = t0 + lane;
-                        if ((m1 >> lane) & 1u) {
-                            const uint32_t j = o0 + __popc(m1 & below);
-                            if (j < b->list_cap)
-                                b->list[j] = make_uint2(tlo + gq.z + t, item);
-                        } else if ((m2 >> lane) & 1u) {
-                            const uint32_t j = o1 + __popc(m2 & below);
-                            if (j < b->clip_cap)
-                                b->clip[b->clip_cap - 1 - j] = make_uint2(gq.z + t, item); // from the end
-                            mark_clip(b, tlo + gq.z + t);
-                        }
-                        o0 += __popc(m1);
-                        o1 += __popc(m2);
+            S.off[k] = incl - a - z;
+            S.off[k + 1] = incl - z;
+            if (lane == 31) {
+                const unsigned long long old = reserve_lists(b, incl & 0xFFFFu, incl >> 16);
+                S.base[0] = (uint32_t)old;
+                S.base[1] = (uint32_t)(old >> 32);
+            }
+            if ((int)lane < nv && S.nx[lane])
+                atomicAdd(b->item_counters + 2 * (size_t)__float_as_uint(S.view[lane][GV_ITEM]),
+                          (unsigned long long)S.nx[lane]);
+        }
+        __syncthreads();
+        if (has) {
+            for (int vi = 0; vi < nv; vi++) {
+                if (!S.cnt[vi * kGeomWarps + warp])
+                    continue;
+                const uint32_t off = S.off[vi * kGeomWarps + warp];
+                uint32_t o0 = S.base[0] + (off & 0xFFFFu), o1 = S.base[1] + (off >> 16);
+                const uint32_t item = __float_as_uint(S.view[vi][GV_ITEM]), tlo = __float_as_uint(S.view[vi][GV_TRI]);
+                for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
+                    const unsigned m1 = S.walk[vi][warp][t0 >> 5], m2 = S.clip[vi][warp][t0 >> 5];
+                    const uint32_t t = t0 + lane;
+                    if ((m1 >> lane) & 1u) {
+                        const uint32_t j = o0 + __popc(m1 & below);
+                        if (j < b->list_cap)
+                            b->list[j] = make_uint2(tlo + gq.z + t, item);
+                    } else if ((m2 >> lane) & 1u) {
+                        const uint32_t j = o1 + __popc(m2 & below);
+                        if (j < b->clip_cap)
+                            b->clip[b->clip_cap - 1 - j] = make_uint2(gq.z + t, item); // from the end
+                        mark_clip(b, tlo + gq.z + t);
                     }
+                    o0 += __popc(m1);
+                    o1 += __popc(m2);
                 }
             }
-            __syncthreads(); // the counts and masks are rewritten by the next pass
         }
     }
 }
@@ -996,6 +983,37 @@ __device__ __forceinline__ unsigned long long make_key(float z, uint32_t slot)
     return ((unsigned long long)__float_as_uint(z) << 32) | slot;
 }
 
+// The span bins: span i's interpolator, edge values and place as three
+// 16-byte words in arrays of span_cap entries, then its item, with
+// kSpanRecorded when the shade cannot replay its pixels and their winners are
+// recorded (a capture span: its first pool entry).
+constexpr uint32_t kSpanRecorded = 1u << 31; // (a batch has at most 4,096 items)
+struct SpanRec {
+    float4 q; // the qpixel interpolator of fill_half_triangle after its displacement to x1: top, tstep, bottom, bstep
+    float4 e; // ... v0, dv; the row's edge progress progL, progR (prepare_for_scanline)
+    uint4 at; // slot, y | kBitLower | kBitLLR, x1, x2
+};
+__device__ __forceinline__ void store_span(const BatchDev *b, uint32_t i, uint32_t item, uint32_t slot, uint32_t y_bits,
+                                           int x1, int x2, const Interp &q, float pl, float pr)
+{
+    float4 *p = static_cast<float4 *>(b->spans) + i;
+    const size_t cap = b->span_cap;
+    p[0] = make_float4(q.top, q.tstep, q.bottom, q.bstep);
+    p[cap] = make_float4(q.v0, q.dv, pl, pr);
+    reinterpret_cast<uint4 *>(p)[2 * cap] = make_uint4(slot, y_bits, (uint32_t)x1, (uint32_t)x2);
+    reinterpret_cast<uint32_t *>(static_cast<float4 *>(b->spans) + 3 * cap)[i] = item;
+}
+__device__ __forceinline__ SpanRec load_span(const BatchDev *b, uint32_t i)
+{
+    const float4 *p = static_cast<const float4 *>(b->spans) + i;
+    const size_t cap = b->span_cap;
+    return SpanRec{p[0], p[cap], reinterpret_cast<const uint4 *>(p)[2 * cap]};
+}
+__device__ __forceinline__ uint32_t load_span_item(const BatchDev *b, uint32_t i)
+{
+    return reinterpret_cast<const uint32_t *>(static_cast<const float4 *>(b->spans) + 3 * (size_t)b->span_cap)[i];
+}
+
 // Bin a long span: the qpixel state after its displacement to x1.
 __device__ __forceinline__ bool bin_span(const BatchDev *b, uint32_t item, uint32_t slot, int y, int x1, int x2,
                                          const Side &Ls, const Side &Rs, uint32_t bits)
@@ -1008,21 +1026,7 @@ __device__ __forceinline__ bool bin_span(const BatchDev *b, uint32_t item, uint3
     Interp q;
     q.init_self(Rs.x - Ls.x, Ls.it.value(), Rs.it.value());
     q.displace((float)x1 - Ls.x);
-    SpanRec r;
-    r.slot = slot;
-    r.y_bits = (uint32_t)y | bits;
-    r.x1 = x1;
-    r.x2 = x2;
-    r.top = q.top;
-    r.tstep = q.tstep;
-    r.bottom = q.bottom;
-    r.bstep = q.bstep;
-    r.v0 = q.v0;
-    r.dv = q.dv;
-    r.progL = Ls.it.alpha;
-    r.progR = Rs.it.alpha;
-    r.item = item;
-    b->spans[i] = r;
+    store_span(b, i, item | kSpanRecorded, slot, (uint32_t)y | bits, x1, x2, q, Ls.it.alpha, Rs.it.alpha);
     return true;
 }
 
@@ -1033,7 +1037,8 @@ struct DepthVisitor {
     uint32_t slot;
     int inline_span;
     bool bin_all; // tall triangle: every span goes to the bins
-    unsigned long long drawn_n, fragments;
+    uint32_t drawn_n;
+    unsigned long long fragments;
 
     __device__ __forceinline__ bool active() const { return true; }
     __device__ __forceinline__ void drawn()
@@ -1126,7 +1131,8 @@ enum {
     F_Z1, F_YS, F_NU, F_FLAGS, F_G0, F_G1, F_G2, F_PRIM,
     F_FRAGS, // fragments of the lane's triangle (shared atomics of the lanes walking its rows)
     F_INCL,  // inclusive prefix of the rows dealt out, per lane
-    kWalkFields
+    F_VX, F_VW, F_KEY, // the item's view: x, w and its key pointer (two words), in batches of several views
+    kWalkFields = F_KEY + 2
 };
 constexpr int kWalkPitch = 33;
 static_assert(F_PRIM == 31 && sizeof(TriRec) == 32 * sizeof(uint32_t), "shared set-up fields follow TriRec");
@@ -1150,6 +1156,9 @@ __device__ __forceinline__ void edge_init(float dist, float rz1, float rz2, floa
     top = top + ts * move;
     bot = bot + bs * move;
 }
+
+// f2i(ceilf(x)) in one conversion where it is in range.
+__device__ __forceinline__ int ceil_i(float x) { return fabsf(x) < 2147483520.0f ? __float2int_ru(x) : f2i(ceilf(x)); }
 
 // The inputs of one walked row: both edges at the half's first row with
 // their constants, the steps to take, the row and its span bits.
@@ -1214,10 +1223,10 @@ __device__ __forceinline__ void row_span(RowIn &r, int vx, int vw, RowSpan &o)
         o.Lx = r.lx; o.Lt = r.lt; o.Lb = r.lb; o.Lz = r.lz; o.Ldv = r.ldv;
         o.Rx = r.sx; o.Rt = r.st; o.Rb = r.sb; o.Rz = r.sz; o.Rdv = r.sdv;
     }
-    o.x1 = f2i(ceilf(o.Lx));
+    o.x1 = ceil_i(o.Lx);
     if (o.x1 < vx)
         o.x1 = vx;
-    o.x2 = f2i(ceilf(o.Rx));
+    o.x2 = ceil_i(o.Rx);
     if (o.x2 > vx + vw)
         o.x2 = vx + vw;
 }
@@ -1264,54 +1273,119 @@ __device__ __forceinline__ bool bin_span_warp(const BatchDev *b, bool want, uint
         atomicExch(counter32(b, C_OVERFLOW), 1u);
         return false;
     }
-    SpanRec r;
-    r.slot = slot;
-    r.y_bits = (uint32_t)y | bits;
-    r.x1 = o.x1;
-    r.x2 = o.x2;
-    r.top = q.top;
-    r.tstep = q.tstep;
-    r.bottom = q.bottom;
-    r.bstep = q.bstep;
-    r.v0 = q.v0;
-    r.dv = q.dv;
-    r.progL = pl;
-    r.progR = pr;
-    r.item = item;
-    b->spans[i] = r;
+    store_span(b, i, item, slot, (uint32_t)y | bits, o.x1, o.x2, q, pl, pr);
     return true;
 }
 
 // One span's pixels into the depth keys (the opaque branch of
 // fill_half_triangle, renderer.cpp:484-499, as a key reduction).
-// The view fields the walk needs, kept in registers while the item stays.
+// The view fields the walk needs of an item.
 struct WalkView {
-    uint32_t item;
-    int x, y, w, h;
-    unsigned long long *key;
-    int inline_span;
-    __device__ __forceinline__ void load(const BatchDev *b, uint32_t i)
+    int x, w;
+    long long origin;         // of the view's pixels, y * w + x of its top left: pixel (X, Y) is Y * w + X - origin
+    unsigned long long *key;  // depth keys less `origin`
+    __device__ __forceinline__ void load(const ItemDev &it)
     {
-        const ItemDev &it = b->items[i];
-        item = i;
         x = it.v.x;
-        y = it.v.y;
         w = it.v.w;
-        h = it.v.h;
-        key = it.key;
+        origin = (long long)it.v.y * w + x;
+        key = it.key - origin;
     }
 };
 
-__device__ __forceinline__ void span_depth(const WalkView &v, int y, uint32_t slot, int x1, int x2, Interp q)
+__device__ __forceinline__ bool key_in_view(const BatchDev *b, uint32_t item, int x, int y)
 {
-    unsigned long long *row = v.key + ((long long)(y - v.y) * v.w - v.x);
-    for (int x = x1; x < x2; x++, q.step()) {
-        const float z = q.value();
-        if (below_near(z) || __float_as_uint(z) >= kMaxZBits)
-            continue;
-        if (in_bounds(x >= v.x && x < v.x + v.w && y >= v.y && y < v.y + v.h, CHK_KEY,
-                      (unsigned long long)(uint32_t)y << 32 | (uint32_t)x))
-            key_min(row + x, make_key(z, slot));
+#ifdef SGL_BOUNDS_CHECK
+    const ViewDev &v = b->items[item].v;
+    return in_bounds(x >= v.x && x < v.x + v.w && y >= v.y && y < v.y + v.h, CHK_KEY,
+                     (unsigned long long)(uint32_t)y << 32 | (uint32_t)x);
+#else
+    return true;
+#endif
+}
+
+// One pixel of a span at the interpolator's top and bottom.
+__device__ __forceinline__ void pixel_depth(const BatchDev *b, uint32_t item, unsigned long long *row, int x, int y,
+                                            uint32_t slot, float top, float bottom, float v0, float dv)
+{
+    const float z = v0 + dv * (top / bottom);
+    if (!below_near(z) && __float_as_uint(z) < kMaxZBits && key_in_view(b, item, x, y))
+        key_min(row + x, make_key(z, slot));
+}
+
+__device__ __forceinline__ void span_depth(const BatchDev *b, const WalkView &v, uint32_t item, int y, uint32_t slot,
+                                           int x1, int x2, const Interp &q)
+{
+    unsigned long long *row = v.key + (long long)y * v.w;
+    float top = q.top, bottom = q.bottom;
+    for (int x = x1; x < x2; x++) {
+        pixel_depth(b, item, row, x, y, slot, top, bottom, q.v0, q.dv);
+        top = top + q.tstep;
+        bottom = bottom + q.bstep;
+    }
+}
+
+// A span's pixels by eight lanes, the `sub`-th of them pixels x1 + sub, + 8, ...:
+// each lane repeats the chain's additions up to its own pixels.  (Eight lanes
+// rather than 32: the additions a lane repeats are 8 per 8 pixels instead of
+// 32 per 32, so that four spans side by side take a third of the instructions
+// of one after another.)
+constexpr int kSpanLanes = 8;
+template <class Op>
+__device__ __forceinline__ void span_by_eight(int x1, int x2, int sub, float top, float tstep, float bottom, float bstep,
+                                              Op &&op)
+{
+#pragma unroll
+    for (int bit = kSpanLanes / 2; bit; bit >>= 1)
+        if (sub & bit) {
+#pragma unroll
+            for (int k = 0; k < bit; k++) {
+                top = top + tstep;
+                bottom = bottom + bstep;
+            }
+        }
+    for (int x = x1 + sub; x < x2; x += kSpanLanes) {
+        op(x, top, bottom);
+#pragma unroll
+        for (int k = 0; k < kSpanLanes; k++) {
+            top = top + tstep;
+            bottom = bottom + bstep;
+        }
+    }
+}
+
+// The spans of the lanes that ask for it, four at a time by eight lanes each.
+// Every lane of the warp calls it.
+__device__ __forceinline__ void spans_depth_warp(const BatchDev *b, bool want, const WalkView &v, uint32_t item, int y,
+                                                 uint32_t slot, int x1, int x2, const Interp &q)
+{
+    unsigned m = __ballot_sync(0xFFFFFFFFu, want);
+    if (!m)
+        return;
+    const int lane = threadIdx.x & 31, sub = lane & (kSpanLanes - 1);
+    unsigned long long *row = v.key + (long long)y * v.w;
+    while (m) {
+        unsigned mine = m; // this lane's span: the (lane / 8)-th of those left
+#pragma unroll
+        for (int k = 0; k < 32 / kSpanLanes - 1; k++)
+            if (lane >= kSpanLanes * (k + 1))
+                mine &= mine - 1;
+        const int src = mine ? __ffs(mine) - 1 : 0;
+        const float top = __shfl_sync(0xFFFFFFFFu, q.top, src), tstep = __shfl_sync(0xFFFFFFFFu, q.tstep, src);
+        const float bottom = __shfl_sync(0xFFFFFFFFu, q.bottom, src), bstep = __shfl_sync(0xFFFFFFFFu, q.bstep, src);
+        const float v0 = __shfl_sync(0xFFFFFFFFu, q.v0, src), dv = __shfl_sync(0xFFFFFFFFu, q.dv, src);
+        const int xa = __shfl_sync(0xFFFFFFFFu, x1, src), xb = __shfl_sync(0xFFFFFFFFu, x2, src);
+        const int ys = __shfl_sync(0xFFFFFFFFu, y, src);
+        const uint32_t sl = __shfl_sync(0xFFFFFFFFu, slot, src), si = __shfl_sync(0xFFFFFFFFu, item, src);
+        unsigned long long *rs = reinterpret_cast<unsigned long long *>(
+            __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(row), src));
+        if (mine)
+            span_by_eight(xa, xb, sub, top, tstep, bottom, bstep, [&](int x, float t, float bt) {
+                pixel_depth(b, si, rs, x, ys, sl, t, bt, v0, dv);
+            });
+#pragma unroll
+        for (int k = 0; k < 32 / kSpanLanes; k++)
+            m &= m - 1;
     }
 }
 
@@ -1360,9 +1434,9 @@ __device__ __forceinline__ void smem_row_in(RowIn &r, const WalkRow *S, int o, i
 
 // Set-up of triangle t (vertices `tri`, projected n0, n1, n2) of `item`:
 // fill_triangle's z sort (renderer.cpp:264-279), fill_triangle_2's y sort,
-// edges and halves (:375-460), into column `c` of the warp's set-ups.  Returns
-// whether the triangle reached scanline set-up (y0 != y2); one that did not
-// has no rows.
+// edges and halves (:375-460), into column `c` of the warp's set-ups.  A
+// triangle that does not reach scanline set-up (y0 == y2) has no rows.
+// Returns whether it did and was not counted by the geometry pass (a NaN y).
 __device__ __forceinline__ bool tri_setup(const BatchDev *b, const ViewDev &v, uint32_t item, uint32_t t, uint4 tri,
                                           float4 n0, float4 n1, float4 n2, uint32_t extra_flags, WalkRow *S, int c)
 {
@@ -1371,10 +1445,12 @@ __device__ __forceinline__ bool tri_setup(const BatchDev *b, const ViewDev &v, u
     V3 a = vp(n0), c1 = vp(n1), c2 = vp(n2);
     const bool ffv = cross_z_negative(sub3(c1, a), sub3(c2, a));
     int pa = 0, pb = 1, pc = 2;
-    sort_z_desc(a, c1, c2, pa, pb, pc);
+    // (the order by z' decides only where the order by y leaves a tie)
+    if (!(a.y < c1.y || a.y > c1.y) || !(a.y < c2.y || a.y > c2.y) || !(c1.y < c2.y || c1.y > c2.y))
+        sort_z_desc(a, c1, c2, pa, pb, pc);
     sort_y_asc(a, c1, c2, pa, pb, pc);
     const V3 v0 = a, v1 = c1, v2 = c2;
-    const int y0 = f2i(ceilf(v0.y)), y1 = f2i(ceilf(v1.y)), y2 = f2i(ceilf(v2.y));
+    const int y0 = ceil_i(v0.y), y1 = ceil_i(v1.y), y2 = ceil_i(v2.y);
     S[F_ITEM][c] = item;
     S[F_SLOT][c] = 2 * t;
     S[F_NU][c] = 0;
@@ -1430,23 +1506,25 @@ __device__ __forceinline__ bool tri_setup(const BatchDev *b, const ViewDev &v, u
         S[F_ND][c] = yend > y ? (uint32_t)(yend - y) : 0u;
     }
     S[F_FLAGS][c] = flags;
-    return true;
+    return v0.y != v0.y || v1.y != v1.y || v2.y != v2.y;
 }
 
-// One row of triangle `slot` of `item` on this lane; every lane of the warp
-// calls it (act = this lane has a row).  Spans wider than the inline limit,
-// and every span of a tall triangle, go to the long-span kernels.  Returns the
-// row's fragments.  `v` caches the item's view (reloaded when it changes).
-// With FRAGS (a view with transparency layers) every fragment is stored
-// instead: the warp reserves its lanes' fragments with one atomic per round
-// of rows, and a binned span carries its first pool entry in the span
-// record's `item` field.
+// Wide spans per round of rows that the walk keeps: the bins' atomic costs a
+// round trip, which more spans share (walk of a terrain's 1080p frame: 32.6,
+// 30.8, 30.0, 27.6 and 28.2 us for 0, 1, 2, 4 and 8).
+constexpr int kWarpSpans = 4;
+// One row of triangle `slot` of `item` (view v) on this lane; every lane of
+// the warp calls it (act = this lane has a row).  A lane walks its span alone
+// up to inline_span pixels; wider ones are walked by eight lanes each, here
+// or (when there are many, they are wider than kReplaySpan, or the triangle is
+// tall) in the long-span kernels.  Returns the row's fragments.  With FRAGS (a view with transparency
+// layers) every fragment is stored instead: the warp reserves its lanes'
+// fragments with one atomic per round of rows, spans beyond inline_span are
+// binned, and a binned span carries its first pool entry in place of its item.
 template <bool FRAGS>
-__device__ __forceinline__ int walk_row(const BatchDev *b, WalkView &v, uint32_t item, uint32_t slot, RowIn &r,
-                                        bool act, bool bin_all)
+__device__ __forceinline__ int walk_row(const BatchDev *b, const WalkView &v, int inline_span, uint32_t item,
+                                        uint32_t slot, RowIn &r, bool act, bool bin_all)
 {
-    if (act && item != v.item)
-        v.load(b, item);
     RowSpan sp;
     sp.x1 = sp.x2 = 0;
     if (act)
@@ -1456,10 +1534,10 @@ __device__ __forceinline__ int walk_row(const BatchDev *b, WalkView &v, uint32_t
     float pl = 0.0f, pr = 0.0f;
     if (has)
         span_interp(sp, q, pl, pr);
-    const bool want = has && (bin_all || sp.x2 - sp.x1 > v.inline_span);
+    const int len = has ? sp.x2 - sp.x1 : 0;
     if constexpr (FRAGS) {
         const int lane = threadIdx.x & 31;
-        const uint32_t n = has ? (uint32_t)(sp.x2 - sp.x1) : 0u;
+        const uint32_t n = (uint32_t)len;
         uint32_t incl = n;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -1473,14 +1551,25 @@ __device__ __forceinline__ int walk_row(const BatchDev *b, WalkView &v, uint32_t
         base = __shfl_sync(0xFFFFFFFFu, base, 31);
         const unsigned long long at = base + incl - n;
         const bool fits = at + n <= (unsigned long long)b->frag_cap; // else counted only: the view is redone
+        const bool want = has && (bin_all || len > inline_span);
         if (!bin_span_warp(b, want && fits, (uint32_t)at, slot, r.y, sp, q, pl, pr, r.bits) && has && fits)
-            span_frags(b, (uint32_t)((r.y - v.y) * v.w - v.x), slot, sp.x1, sp.x2, q, pl, pr, r.bits,
+            span_frags(b, (uint32_t)((long long)r.y * v.w - v.origin), slot, sp.x1, sp.x2, q, pl, pr, r.bits,
                        (uint32_t)at);
     } else {
-        if (!bin_span_warp(b, want, item, slot, r.y, sp, q, pl, pr, r.bits) && has)
-            span_depth(v, r.y, slot, sp.x1, sp.x2, q);
+        // Wide spans: up to kWarpSpans of a round are walked by this warp at
+        // once, more (or longer than the shade replays) go to the bins, whose
+        // atomic's round trip and second kernel they are worth.
+        bool wide = has && (bin_all || len > inline_span);
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, wide);
+        const bool record = bin_all || len > kReplaySpan;
+        const bool want = wide && (record || __popc(m) > kWarpSpans);
+        if (bin_span_warp(b, want, record ? item | kSpanRecorded : item, slot, r.y, sp, q, pl, pr, r.bits))
+            wide = false;
+        else if (has && !wide)
+            span_depth(b, v, item, r.y, slot, sp.x1, sp.x2, q);
+        spans_depth_warp(b, wide, v, item, r.y, slot, sp.x1, sp.x2, q);
     }
-    return has ? sp.x2 - sp.x1 : 0;
+    return len;
 }
 
 // n <= 31 repeated additions x += d of three chains; every lane takes its own
@@ -1499,19 +1588,6 @@ __device__ __forceinline__ void step3(float &x, float &t, float &b, float dx, fl
             }
         }
 }
-__device__ __forceinline__ void step2(float &t, float &b, float dt, float db, int n)
-{
-#pragma unroll
-    for (int bit = 16; bit; bit >>= 1)
-        if (n & bit) {
-#pragma unroll
-            for (int k = 0; k < bit; k++) {
-                t = t + dt;
-                b = b + db;
-            }
-        }
-}
-
 // A tall triangle (set-up in column 0 of S), walked by the whole warp 32 rows
 // at a time: each lane takes its own row's steps from the state of the first
 // of the 32, and lane 31's state after one more step is the next 32 rows'.
@@ -1524,8 +1600,7 @@ __device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, const WalkRow *
     const uint32_t slot = S[F_SLOT][0], item = S[F_ITEM][0];
     uint32_t frags = 0;
     WalkView v;
-    v.load(b, item);
-    v.inline_span = b->inline_span;
+    v.load(b->items[item]);
     float lx = smf(S, F_LX, 0), lt = smf(S, F_LT, 0), lb = smf(S, F_LB, 0);
     int sf = n_u > 0 ? F_UX : F_DX; // the short edge in hand
     float sx = smf(S, sf, 0), st = smf(S, sf + 1, 0), sb = smf(S, sf + 2, 0);
@@ -1561,15 +1636,15 @@ __device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, const WalkRow *
                 sb = smf(S, F_DB, 0);
             }
         }
-        frags += (uint32_t)walk_row<FRAGS>(b, v, item, slot, r, act, true);
+        frags += (uint32_t)walk_row<FRAGS>(b, v, kSpanLanes, item, slot, r, act, true);
     }
     return frags;
 }
 
 // the rare depth walks, defined with the near-clip code below
-__device__ __noinline__ void walk_clip_depth(const BatchDev *b, ItemAcc &acc);
+__device__ __noinline__ void walk_clip_depth(const BatchDev *b);
 template <bool FRAGS>
-__device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc, WalkRow *S);
+__device__ __noinline__ void walk_tall_all(const BatchDev *b, WalkRow *S);
 
 // One warp's shared memory: the set-ups of the group in hand, and what is
 // copied in ahead for the next groups: list entries (three ahead), their
@@ -1583,6 +1658,29 @@ struct WalkShared {
     uint2 entry[4][32];
 };
 
+// Fragments of the lanes' triangles (fewer than 2^26 each, or counted at once)
+// added to the block's sums of the first kWalkItems items, the others' to
+// their counters.  An atomic on the item's counter per group of 32 triangles
+// met all the warps that were walking the same view: 98 us of the 64-view
+// batch's 589.  Every lane of the warp calls it.
+constexpr int kWalkItems = 64;
+__device__ __forceinline__ void block_add(const BatchDev *b, uint32_t *sums, uint32_t item, uint32_t n)
+{
+    const unsigned act = __ballot_sync(0xFFFFFFFFu, n != 0u);
+    if (!n)
+        return;
+    if (__any_sync(act, (n >> 26) || item >= (uint32_t)kWalkItems)) {
+        atomicAdd(b->item_counters + 2 * (size_t)item + 1, (unsigned long long)n);
+        return;
+    }
+    const unsigned grp = __match_any_sync(act, item);
+    const uint32_t sum = __reduce_add_sync(grp, n);
+    if ((threadIdx.x & 31) == __ffs(grp) - 1 && atomicAdd(sums + item, sum) >> 31) {
+        const uint32_t all = atomicExch(sums + item, 0u); // (well before it overflows)
+        atomicAdd(b->item_counters + 2 * (size_t)item + 1, (unsigned long long)all);
+    }
+}
+
 // Set-up and depth walk of the drawable triangles wholly in front of the near
 // plane (fill_triangle's normal case, renderer.cpp:281-285: one sub-triangle,
 // slot 2t).  Each warp takes groups of 32 list entries (warp-strided): a lane
@@ -1594,6 +1692,7 @@ template <bool FRAGS, bool STRIDED>
 __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(const BatchDev *b)
 {
     __shared__ WalkShared shared[kWalkWarps];
+    __shared__ uint32_t item_frags[kWalkItems]; // fragments of the batch's first items, walked by this block
     WalkShared &W = shared[threadIdx.x >> 5];
     WalkRow *S = W.S;
     const int lane = threadIdx.x & 31;
@@ -1631,10 +1730,16 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
             }
         }
     };
-    ItemAcc acc;
-    WalkView view;
-    view.item = 0xFFFFFFFFu;
-    view.inline_span = b->inline_span;
+    if (!STRIDED) {
+        for (int i = (int)threadIdx.x; i < kWalkItems; i += kWalkWarps * 32)
+            item_frags[i] = 0u;
+        __syncthreads();
+    }
+    const int inline_span = b->inline_span;
+    WalkView view{};
+    if (STRIDED)
+        view.load(b->items[0]);
+    unsigned long long fragments = 0; // STRIDED: of this lane's triangles
     // Warps take groups g, g + G, g + 2G, ... (G warps in the grid; work
     // queues were measured slower: 41 -> 48 us on the 1080p frame).
     const uint32_t G = (gridDim.x * blockDim.x) >> 5;
@@ -1655,12 +1760,21 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
     for (int q = 0; g < n_groups; q++, g += G) {
         cp_async_wait<0>();
         const bool valid = index(g) < n;
-        bool drawn = false;
+        bool late = false;
         S[F_FRAGS][lane] = 0;
         if (valid) {
             const uint2 e = W.entry[q & 3][lane];
             const float4 n0 = W.ndc[0][lane], n1 = W.ndc[1][lane], n2 = W.ndc[2][lane];
-            drawn = tri_setup(b, b->items[e.y].v, e.y, e.x - __ldg(b->tri_base + e.y), W.tri[q & 1][lane], n0, n1, n2,
+            if (!STRIDED) {
+                WalkView v;
+                v.load(b->items[e.y]);
+                const unsigned long long kp = reinterpret_cast<unsigned long long>(v.key);
+                S[F_VX][lane] = (uint32_t)v.x;
+                S[F_VW][lane] = (uint32_t)v.w;
+                S[F_KEY][lane] = (uint32_t)kp;
+                S[F_KEY + 1][lane] = (uint32_t)(kp >> 32);
+            }
+            late = tri_setup(b, b->items[e.y].v, e.y, e.x - __ldg(b->tri_base + e.y), W.tri[q & 1][lane], n0, n1, n2,
                               0u, S, lane);
         } else {
             S[F_NU][lane] = 0;
@@ -1697,20 +1811,35 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
                 const int ex = o > 0 ? (int)S[F_INCL][o - 1] : 0;
                 smem_row_in(r, S, o, p - ex);
             }
-            const int fr = walk_row<FRAGS>(b, view, S[F_ITEM][o], S[F_SLOT][o], r, act, false);
+            if (!STRIDED) {
+                view.x = (int)S[F_VX][o];
+                view.w = (int)S[F_VW][o];
+                view.key = reinterpret_cast<unsigned long long *>((unsigned long long)S[F_KEY][o] |
+                                                                  ((unsigned long long)S[F_KEY + 1][o] << 32));
+            }
+            const int fr = walk_row<FRAGS>(b, view, inline_span, S[F_ITEM][o], S[F_SLOT][o], r, act, false);
             if (fr)
                 atomicAdd(&S[F_FRAGS][o], (uint32_t)fr);
         }
         __syncwarp();
-        acc.add(b, valid ? S[F_ITEM][lane] : 0u, drawn ? 1ull : 0ull, (unsigned long long)S[F_FRAGS][lane], valid);
+        const uint32_t fr = S[F_FRAGS][lane];
+        if (STRIDED)
+            fragments += fr;
+        else
+            block_add(b, item_frags, valid ? S[F_ITEM][lane] : 0u, fr);
+        if (__any_sync(0xFFFFFFFFu, late))
+            item_add(b, 0, late ? S[F_ITEM][lane] : 0u, 1u, late);
         // the records with fragments, four per round (a 128-byte line by eight
         // lanes): written by one lane each, as eight 16-byte stores to its own
         // line, the stores' 32 lines per instruction throttled the set-up
         // (20 us at 20 % issue on the 1080p frame)
+        const unsigned kept = __ballot_sync(0xFFFFFFFFu, fr != 0u);
 #pragma unroll
         for (int j0 = 0; j0 < 32; j0 += 4) {
+            if (!((kept >> j0) & 15u))
+                continue;
             const int j = j0 + (lane >> 3), w = 4 * (lane & 7);
-            if (S[F_FRAGS][j]) {
+            if ((kept >> j) & 1u) {
                 const uint32_t r = W.entry[q & 3][j].x;
                 if (in_bounds(r < b->list_cap, CHK_REC, r))
                     reinterpret_cast<uint4 *>(b->recs + r)[lane & 7] =
@@ -1721,10 +1850,22 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
     }
     cp_async_wait<0>();
     // then this warp's share of the near-clip and the tall triangles
+    if (STRIDED) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            fragments += __shfl_xor_sync(0xFFFFFFFFu, fragments, o);
+        if (lane == 0 && fragments)
+            atomicAdd(b->item_counters + 1, fragments);
+    }
     if (!FRAGS)
-        walk_clip_depth(b, acc);
-    walk_tall_all<FRAGS>(b, acc, S);
-    acc.flush(b);
+        walk_clip_depth(b);
+    walk_tall_all<FRAGS>(b, S);
+    if (!STRIDED) {
+        __syncthreads();
+        for (int i = (int)threadIdx.x; i < kWalkItems; i += kWalkWarps * 32)
+            if (item_frags[i])
+                atomicAdd(b->item_counters + 2 * (size_t)i + 1, (unsigned long long)item_frags[i]);
+    }
 }
 
 // ------------------------------------------------------------- near clip --
@@ -1828,7 +1969,7 @@ __device__ __forceinline__ void clip_triangle(const ItemDev &it, uint32_t t, Emi
 // Depth walk of the near-clip triangles (fill_triangle's clip cases), one
 // thread each, over a warp-strided share of the clip list.  Out of line: rare,
 // and its register and stack use stay off the row walk.
-__device__ __noinline__ void walk_clip_depth(const BatchDev *b, ItemAcc &acc)
+__device__ __noinline__ void walk_clip_depth(const BatchDev *b)
 {
     const uint32_t n_raw = *counter32(b, C_CLIP);
     const uint32_t n = n_raw < b->clip_cap ? n_raw : b->clip_cap;
@@ -1837,7 +1978,7 @@ __device__ __noinline__ void walk_clip_depth(const BatchDev *b, ItemAcc &acc)
     for (uint32_t i0 = 32 * gw; i0 < n; i0 += 32 * n_warps) {
         const uint32_t i = i0 + lane;
         const bool valid = i < n;
-        DepthVisitor dvis{b, nullptr, 0u, 0u, b->inline_span, false, 0ull, 0ull};
+        DepthVisitor dvis{b, nullptr, 0u, 0u, b->inline_span, false, 0u, 0ull};
         if (valid) {
             const uint2 e = b->clip[b->clip_cap - 1 - i];
             const ItemDev &it = b->items[e.y];
@@ -1849,14 +1990,15 @@ __device__ __noinline__ void walk_clip_depth(const BatchDev *b, ItemAcc &acc)
             };
             clip_triangle(it, e.x, emit);
         }
-        acc.add(b, dvis.item, dvis.drawn_n, dvis.fragments, valid);
+        item_add(b, 0, dvis.item, dvis.drawn_n, valid);
+        item_add(b, 1, dvis.item, dvis.fragments, valid);
     }
 }
 
 // Set-up and depth walk (or fragment capture) of the tall triangles, one warp
 // each (warp-strided).
 template <bool FRAGS>
-__device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc, WalkRow *S)
+__device__ __noinline__ void walk_tall_all(const BatchDev *b, WalkRow *S)
 {
     const uint32_t nt_raw = *counter32(b, C_TALL);
     const uint32_t nt = nt_raw < b->list_cap ? nt_raw : b->list_cap;
@@ -1869,12 +2011,11 @@ __device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc, Walk
         const uint4 tri = it.s.tris[t];
         __syncwarp();
         // (every lane writes the same values)
-        const bool drawn = tri_setup(b, it.v, item, t, tri, it.ndc[tri.x], it.ndc[tri.y], it.ndc[tri.z], kRecTall, S, 0);
+        tri_setup(b, it.v, item, t, tri, it.ndc[tri.x], it.ndc[tri.y], it.ndc[tri.z], kRecTall, S, 0);
         __syncwarp();
         if (in_bounds(r < b->list_cap, CHK_REC, r))
             reinterpret_cast<uint32_t *>(b->recs + r)[lane] = S[lane][0];
-        const uint32_t fr = walk_tall<FRAGS>(b, S);
-        acc.add(b, item, drawn && lane == 0 ? 1ull : 0ull, fr, true);
+        item_add(b, 1, item, walk_tall<FRAGS>(b, S), true);
     }
 }
 
@@ -1882,7 +2023,7 @@ __device__ __noinline__ void walk_tall_all(const BatchDev *b, ItemAcc &acc, Walk
 // keys are final: binned spans (one warp each, the qpixel chain as in
 // k_spans), near-clip triangles (one thread each) and, after a bin overflow,
 // every span of the walk list.
-__device__ __forceinline__ void spans_pass(const BatchDev *b, bool winner);
+template <bool WINNER> __device__ __forceinline__ void spans_pass(const BatchDev *b);
 
 __device__ __noinline__ void winner_clip(const BatchDev *b, bool overflow)
 {
@@ -1918,64 +2059,72 @@ __device__ __noinline__ void winner_overflow(const BatchDev *b)
     }
 }
 
-__global__ void __launch_bounds__(256) k_winners(const BatchDev *b)
+__global__ void __launch_bounds__(256, 4) k_winners(const BatchDev *b)
 {
     const bool overflow = *counter32(b, C_OVERFLOW) != 0u;
     if (overflow) {
         winner_overflow(b); // records every span, the binned ones included
     } else {
-        spans_pass(b, true);
+        spans_pass<true>(b);
     }
     winner_clip(b, overflow);
 }
 
 // ------------------------------------------------------------- long spans --
 
-// Binned spans, one warp each.  The qpixel chain (top += tstep, bottom +=
-// bstep per pixel, interpolator.hpp:96-100) is serial in floating point, so
-// every lane runs the same 32 steps and keeps the state of its own pixel; the
-// divisions, depth and key work then run on all lanes.
-__device__ __forceinline__ void spans_pass(const BatchDev *b, bool winner)
+// Binned spans, eight lanes each (span_by_eight).  WINNER: the fragments of
+// the recorded ones whose key won record their progress values; else the keys
+// are folded.
+template <bool WINNER> __device__ __forceinline__ void spans_pass(const BatchDev *b)
 {
     const uint32_t n_raw = *counter32(b, C_SPANS);
     const uint32_t n = n_raw < b->span_cap ? n_raw : b->span_cap;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = warp; i < n; i += n_warps) {
-        const SpanRec r = b->spans[i];
-        const ItemDev &it = b->items[r.item];
-        const int y = (int)(r.y_bits & kYMask);
+    const uint32_t step = gridDim.x * blockDim.x / kSpanLanes;
+    const int sub = (int)threadIdx.x & (kSpanLanes - 1);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kSpanLanes; i < n; i += step) {
+        const uint32_t flagged = load_span_item(b, i);
+        if (WINNER && !(flagged & kSpanRecorded))
+            continue;
+        const SpanRec r = load_span(b, i);
+        const uint32_t item = flagged & ~kSpanRecorded, slot = r.at.x;
+        const ItemDev &it = b->items[item];
+        const int y = (int)(r.at.y & kYMask), x2 = (int)r.at.w;
         const long long base = (long long)(y - it.v.y) * it.v.w - it.v.x;
-        float top = r.top, bottom = r.bottom;
-        for (int x0 = r.x1; x0 < r.x2; x0 += 32) {
-            float mt = top, mb = bottom;
-            step2(mt, mb, r.tstep, r.bstep, lane);
-            if (x0 + 32 < r.x2) {
-                top = __shfl_sync(0xFFFFFFFFu, mt + r.tstep, 31);
-                bottom = __shfl_sync(0xFFFFFFFFu, mb + r.bstep, 31);
+        unsigned long long *row = it.key + base;
+        float4 *prec = it.prec + base;
+        // WINNER: the keys of a lane's next four pixels are in flight at once
+        unsigned long long keys[4] = {};
+        int j = 0;
+        span_by_eight((int)r.at.z, x2, sub, r.q.x, r.q.y, r.q.z, r.q.w, [&](int x, float top, float bottom) {
+            if (WINNER) {
+                if ((j & 3) == 0) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        keys[k] = x + kSpanLanes * k < x2 ? row[x + kSpanLanes * k] : 0ull;
+                } else {
+                    keys[0] = keys[1];
+                    keys[1] = keys[2];
+                    keys[2] = keys[3];
+                }
+                j++;
             }
-            const int x = x0 + lane;
-            if (x >= r.x2)
-                continue;
-            const float alpha = mt / mb;
-            const float z = r.v0 + r.dv * alpha;
+            const float alpha = top / bottom;
+            const float z = r.e.x + r.e.y * alpha;
             if (below_near(z) || __float_as_uint(z) >= kMaxZBits)
-                continue;
-            const unsigned long long key = make_key(z, r.slot);
-            unsigned long long *kp = it.key + base + x;
+                return;
             if (!in_bounds(x >= it.v.x && x < it.v.x + it.v.w && y >= it.v.y && y < it.v.y + it.v.h,
-                           winner ? CHK_PREC : CHK_KEY, (unsigned long long)(uint32_t)y << 32 | (uint32_t)x))
-                continue;
-            if (!winner)
-                key_min(kp, key);
-            else if (*kp == key)
-                it.prec[base + x] = make_float4(alpha, r.progL, r.progR, __uint_as_float(r.y_bits & ~kYMask));
-        }
+                           WINNER ? CHK_PREC : CHK_KEY, (unsigned long long)(uint32_t)y << 32 | (uint32_t)x))
+                return;
+            const unsigned long long key = make_key(z, slot);
+            if (!WINNER)
+                key_min(row + x, key);
+            else if (keys[0] == key)
+                prec[x] = make_float4(alpha, r.e.z, r.e.w, __uint_as_float(r.at.y & ~kYMask));
+        });
     }
 }
 
-__global__ void __launch_bounds__(256) k_spans(const BatchDev *b) { spans_pass(b, false); }
+__global__ void __launch_bounds__(256) k_spans(const BatchDev *b) { spans_pass<false>(b); }
 
 // ------------------------------------------------------------------ shade --
 
@@ -2052,8 +2201,7 @@ __device__ __forceinline__ Quarter load_quarter(const TriRec *rp, int k)
 // triangle's set-up (`d`: the record's last quarter): the row's edges after their steps, the span and the
 // qpixel chain up to X (renderer.cpp:474-493).  False when the span was wide
 // enough to be binned (its winners were recorded by the span kernels).
-__device__ __forceinline__ bool rec_replay(const TriRec *rp, const Quarter &d, const ViewDev &v, int inline_span,
-                                           int X, int Y, float4 &out)
+__device__ __forceinline__ bool rec_replay(const TriRec *rp, const Quarter &d, const ViewDev &v, int X, int Y, float4 &out)
 {
     const Quarter a = load_quarter(rp, 0);
     const int y_s = (int)d.w[1], n_u = (int)d.w[2];
@@ -2072,7 +2220,7 @@ __device__ __forceinline__ bool rec_replay(const TriRec *rp, const Quarter &d, c
     row_in(r, k, lg, sh, __uint_as_float(a.w[6]), __uint_as_float(d.w[0]), __uint_as_float(a.w[7]), y_s, y_l, n_u, flags);
     RowSpan sp;
     row_span(r, v.x, v.w, sp);
-    if (sp.x2 - sp.x1 > inline_span)
+    if (sp.x2 - sp.x1 > kReplaySpan)
         return false;
     Interp it;
     float pl, pr;
@@ -2101,7 +2249,7 @@ __device__ __forceinline__ uint32_t shade_winner_impl(const BatchDev *b, uint32_
         return shade_clip_px(it, i, slot);
     const int y = (int)(i / (uint32_t)v.w), x = (int)(i - (uint32_t)y * (uint32_t)v.w);
     float4 rec;
-    if (overflow || (flags & kRecTall) || !rec_replay(rp, d, v, b->inline_span, x + v.x, y + v.y, rec))
+    if (overflow || (flags & kRecTall) || !rec_replay(rp, d, v, x + v.x, y + v.y, rec))
         rec = it.prec[i]; // recorded by the span kernels (or the overflow winner walk)
     return shade_rec<ALL_MODES>(it, make_uint4(d.w[4], d.w[5], d.w[6], d.w[7]), flags, rec);
 }
@@ -2667,7 +2815,8 @@ struct FragVisitor {
     const BatchDev *b;
     const ItemDev *it;
     uint32_t slot;
-    unsigned long long drawn_n, fragments;
+    uint32_t drawn_n;
+    unsigned long long fragments;
     unsigned long long at;
 
     __device__ __forceinline__ bool active() const { return true; }
@@ -2687,21 +2836,8 @@ struct FragVisitor {
                 Interp q;
                 q.init_self(Rs.x - Ls.x, Ls.it.value(), Rs.it.value());
                 q.displace((float)x1 - Ls.x);
-                SpanRec r;
-                r.slot = slot;
-                r.y_bits = (uint32_t)y | bits;
-                r.x1 = x1;
-                r.x2 = x2;
-                r.top = q.top;
-                r.tstep = q.tstep;
-                r.bottom = q.bottom;
-                r.bstep = q.bstep;
-                r.v0 = q.v0;
-                r.dv = q.dv;
-                r.progL = Ls.it.alpha;
-                r.progR = Rs.it.alpha;
-                r.item = (uint32_t)k; // the span's first fragment (a layered batch has one item)
-                b->spans[si] = r;
+                // (item: the span's first fragment; a layered batch has one item)
+                store_span(b, si, (uint32_t)k, slot, (uint32_t)y | bits, x1, x2, q, Ls.it.alpha, Rs.it.alpha);
                 return;
             }
         }
@@ -2724,7 +2860,6 @@ __global__ void __launch_bounds__(256) k_frags(const BatchDev *b)
     const uint32_t c_raw = *counter32(b, C_CLIP);
     const uint32_t nc = c_raw < b->clip_cap ? c_raw : b->clip_cap;
     const int lane = threadIdx.x & 31;
-    ItemAcc acc;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; i0 < nc; i0 += stride) {
         const uint32_t i = i0 + (uint32_t)lane;
@@ -2755,15 +2890,15 @@ __global__ void __launch_bounds__(256) k_frags(const BatchDev *b)
         if (lane == 31 && incl)
             base = atomicAdd(frag_counter(b), incl);
         base = __shfl_sync(0xFFFFFFFFu, base, 31);
-        FragVisitor vis{b, &it, 0u, 0ull, 0ull, base + incl - cnt.n};
+        FragVisitor vis{b, &it, 0u, 0u, 0ull, base + incl - cnt.n};
         walk(vis);
-        acc.add(b, e.y, vis.drawn_n, vis.fragments, valid);
+        item_add(b, 0, e.y, vis.drawn_n, valid);
+        item_add(b, 1, e.y, vis.fragments, valid);
     }
-    acc.flush(b);
 }
 
-// The binned long spans of the capture, one warp each: the qpixel chain as in
-// k_spans, then every lane stores its pixel's fragment.
+// The binned long spans of the capture, eight lanes each as in k_spans: every
+// lane stores its pixels' fragments.
 __global__ void __launch_bounds__(256) k_frag_spans(const BatchDev *b)
 {
     if (frags_overflowed(b))
@@ -2773,33 +2908,23 @@ __global__ void __launch_bounds__(256) k_frag_spans(const BatchDev *b)
     const ItemDev &it = b->items[0];
     const ViewDev &v = it.v;
     Frag *pool = b->frags;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = warp; i < n; i += n_warps) {
-        const SpanRec r = b->spans[i];
-        const int y = (int)(r.y_bits & kYMask);
+    const uint32_t step = gridDim.x * blockDim.x / kSpanLanes;
+    const int sub = (int)threadIdx.x & (kSpanLanes - 1);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kSpanLanes; i < n; i += step) {
+        const SpanRec r = load_span(b, i);
+        const uint32_t first = load_span_item(b, i);
+        const int y = (int)(r.at.y & kYMask), x1 = (int)r.at.z;
         const uint32_t row_px = (uint32_t)((y - v.y) * v.w - v.x);
-        const float fb = __uint_as_float(r.y_bits & ~kYMask);
-        float top = r.top, bottom = r.bottom;
-        for (int x0 = r.x1; x0 < r.x2; x0 += 32) {
-            float mt = top, mb = bottom;
-            step2(mt, mb, r.tstep, r.bstep, lane);
-            if (x0 + 32 < r.x2) {
-                top = __shfl_sync(0xFFFFFFFFu, mt + r.tstep, 31);
-                bottom = __shfl_sync(0xFFFFFFFFu, mb + r.bstep, 31);
-            }
-            const int x = x0 + lane;
-            if (x >= r.x2)
-                continue;
-            const float alpha = mt / mb;
-            const float z = r.v0 + r.dv * alpha;
+        const float fb = __uint_as_float(r.at.y & ~kYMask);
+        span_by_eight(x1, (int)r.at.w, sub, r.q.x, r.q.y, r.q.z, r.q.w, [&](int x, float top, float bottom) {
+            const float alpha = top / bottom;
+            const float z = r.e.x + r.e.y * alpha;
             const bool keep = !below_near(z) && __float_as_uint(z) < kMaxZBits;
-            const uint32_t at = r.item + (uint32_t)(x - r.x1);
-            reinterpret_cast<float4 *>(pool + at)[0] = make_float4(alpha, r.progL, r.progR, fb);
+            const uint32_t at = first + (uint32_t)(x - x1);
+            reinterpret_cast<float4 *>(pool + at)[0] = make_float4(alpha, r.e.z, r.e.w, fb);
             reinterpret_cast<uint4 *>(pool + at)[1] =
-                make_uint4(__float_as_uint(z), r.slot, keep ? row_px + (uint32_t)x : kFragEnd, 0u);
-        }
+                make_uint4(__float_as_uint(z), r.at.x, keep ? row_px + (uint32_t)x : kFragEnd, 0u);
+        });
     }
 }
 
@@ -3150,7 +3275,7 @@ cudaError_t launch_batch(const BatchDev *b, int tile, int flags, cudaStream_t st
     int n = 0;
     mark(PK_GEOM);
     if (flags & kSeqFused) {
-        k_geom<<<sms * kGeomBlocks * 2, kGeomWarps * 32, kGeomSmem, st>>>(b);
+        k_geom<<<sms * kGeomBlocks * 8, kGeomWarps * 32, kGeomSmem, st>>>(b);
         ran(PK_GEOM);
         n++;
     }

@@ -53,6 +53,13 @@ constexpr uint32_t kFuseVerts = 256, kFuseTris = 512;
 // The fused geometry pass: a block takes kGeomWarps primitives of a group (one
 // warp each) and runs them for every item of the group.
 constexpr int kGeomWarps = 8;
+// ... at most kGeomItems at a time: a unit of its work is kGeomWarps primitives
+// and kGeomItems items of a group.
+constexpr int kGeomItems = 8;
+inline uint32_t geom_units(uint32_t n_prims, uint32_t n_items)
+{
+    return (n_prims + kGeomWarps - 1) / kGeomWarps * ((n_items + kGeomItems - 1) / kGeomItems);
+}
 
 struct LightsDev {
     float ambient;
@@ -178,17 +185,11 @@ inline int dof_halo_of(float max_radius)
     return h;
 }
 
-// A span handed from the triangle walk to the long-span kernels: the qpixel
-// interpolator of fill_half_triangle after its displacement to x1.
-struct SpanRec {
-    uint32_t slot;
-    uint32_t y_bits; // y | kBitLower | kBitLLR
-    int x1, x2;
-    float top, tstep, bottom, bstep, v0, dv;
-    float progL, progR; // edge progress of the row (prepare_for_scanline)
-    uint32_t item;
-};
-static_assert(sizeof(SpanRec) == 52, "SpanRec layout");
+// Bytes of a span handed from the triangle walk to the long-span kernels.
+constexpr size_t kSpanBytes = 52;
+// Spans of the walk list wider than this many pixels are binned; the shade
+// replays the others' pixel steps, up to this many.
+constexpr int kReplaySpan = 64;
 
 constexpr uint32_t kBitLower = 1u << 30; // span of the lower half-triangle
 constexpr uint32_t kBitLLR = 1u << 31;   // long_line_on_right
@@ -248,15 +249,15 @@ struct BatchDev {
     // the geometry passes: items of fused scenes in groups that read the same
     // vertex data (one scene, or one posed request's own world positions) —
     // group g holds the items grp_items[grp_item_base[g] .. grp_item_base[g+1])
-    // and the chunks grp_chunk_base[g] .. grp_chunk_base[g+1] of kGeomWarps
-    // primitives each; the other items by vertex and triangle (g_vtx_base,
+    // and the units grp_chunk_base[g] .. grp_chunk_base[g+1] (geom_units: primitives
+    // outermost); the other items by vertex and triangle (g_vtx_base,
     // g_tri_base).  Each item counts in one of the two.
     const uint32_t *g_vtx_base, *g_tri_base;
     const uint32_t *grp_chunk_base, *grp_item_base, *grp_items;
     uint32_t total_gvtx, total_gtri, total_chunks;
     int n_groups;
     int n_items;
-    int inline_span;           // spans wider than this go to the long-span bins
+    int inline_span;           // spans wider than this are walked by several lanes
     uint32_t total_px, total_tiles, total_dof_tiles;
     uint2 *list;               // drawable triangles {batch triangle (tri_base[item] + t), item}
     uint32_t list_cap;
@@ -268,7 +269,7 @@ struct BatchDev {
     int keep_keys;             // leave the depth keys for the caller (debug); else the shade resets them
     unsigned long long *key_pool; // the items' depth keys: batch pixel px_base[item] + i at key_pool[...]
     uint2 *wins;               // kSeqWinList: pixels with a winner {batch pixel, draw slot}, in pixel order
-    SpanRec *spans;            // long-span bins
+    void *spans;               // long-span bins (span_cap spans of kSpanBytes)
     uint32_t span_cap;
     unsigned long long *counters;      // kCounterWords words
     unsigned long long *item_counters; // per item: drawn, fragments

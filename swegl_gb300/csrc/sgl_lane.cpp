@@ -43,7 +43,7 @@ size_t view_scratch_bytes(uint32_t n_vertices, uint32_t n_triangles, int w, int 
     const size_t px = (size_t)w * h;
     return align_up(16 * (size_t)n_vertices, 256) + align_up(n_vertices, 256) + 8 * px + 16 * px  // ndc yes key prec
            + (px >= kWinListMinPixels ? 8 * px : 0)                                               // winner list
-           + (8 + sizeof(TriRec) + 8) * (size_t)n_triangles + sizeof(SpanRec) * (px / 8 + 64)      // lists, set-ups, bins
+           + (8 + sizeof(TriRec) + 8) * (size_t)n_triangles + kSpanBytes * (px / 8 + 64)      // lists, set-ups, bins
            + 8 * px;                                                                               // dof colour, depth
 }
 
@@ -162,7 +162,7 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
                 dofz_px += align_up((size_t)v.w * v.h, 64);
         }
     }
-    // the fused pass's groups: chunks of kGeomWarps primitives, items
+    // the fused pass's groups: units of work, items
     uint64_t tc = 0;
     uint32_t n_grouped = 0;
     const int n_groups = (int)grp_key.size();
@@ -170,7 +170,7 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         gcb[k] = (uint32_t)tc;
         gib[k] = n_grouped;
         const Scene &s = *e[grp_members[k][0]].scene;
-        tc += (s.dev.n_prims + kGeomWarps - 1) / kGeomWarps;
+        tc += geom_units(s.dev.n_prims, (uint32_t)grp_members[k].size());
         for (uint32_t it : grp_members[k])
             gi[n_grouped++] = it;
     }
@@ -207,7 +207,7 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     CUDA_TRY(list.ensure(sizeof(uint2) * std::max<uint64_t>(tt, 1)));
     CUDA_TRY(recs.ensure(sizeof(TriRec) * std::max<uint64_t>(tt, 1)));
     CUDA_TRY(tall.ensure(sizeof(uint32_t) * std::max<uint64_t>(tt, 1)));
-    CUDA_TRY(spans.ensure(sizeof(SpanRec) * span_cap));
+    CUDA_TRY(spans.ensure(kSpanBytes * span_cap));
     if (dof_px) {
         CUDA_TRY(doftmp.ensure(4 * dof_px));
         if (dofz_px)
@@ -324,8 +324,8 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     bd.key_pool = (unsigned long long *)key.ptr;
     bd.wins = win_list ? (uint2 *)wins.ptr : nullptr;
     sl.keep_keys = bd.keep_keys != 0;
-    bd.spans = (SpanRec *)spans.ptr;
-    bd.span_cap = (uint32_t)std::min<size_t>(spans.bytes / sizeof(SpanRec), 0xFFFFFFFFu);
+    bd.spans = spans.ptr;
+    bd.span_cap = (uint32_t)std::min<size_t>(spans.bytes / kSpanBytes, 0xFFFFFFFFu);
     bd.counters = (unsigned long long *)sl.d_counters.ptr;
     bd.item_counters = (unsigned long long *)sl.d_item_counters.ptr;
     bd.slot_flags = slot_flags;
