@@ -2059,7 +2059,7 @@ __device__ __noinline__ void winner_overflow(const BatchDev *b)
     }
 }
 
-__global__ void __launch_bounds__(256, 4) k_winners(const BatchDev *b)
+__device__ __noinline__ void winner_records(const BatchDev *b)
 {
     const bool overflow = *counter32(b, C_OVERFLOW) != 0u;
     if (overflow) {
@@ -2069,6 +2069,8 @@ __global__ void __launch_bounds__(256, 4) k_winners(const BatchDev *b)
     }
     winner_clip(b, overflow);
 }
+
+__global__ void __launch_bounds__(256, 4) k_winners(const BatchDev *b) { winner_records(b); }
 
 // ------------------------------------------------------------- long spans --
 
@@ -2391,98 +2393,116 @@ __global__ void __launch_bounds__(kShadeThreads, SGL_TILE_MIN_BLOCKS) k_shade(co
 }
 
 // The same per-pixel work for a batch of one large view (kSeqWinList), in
-// two passes.  k_classify streams the batch's depth keys (one contiguous pool
-// in batch pixel order, kClassifyPx keys per thread in flight): empty pixels
-// get the background colour and depth at once; a winner gets its depth, its
-// key is reset to empty (unless kept for debug), and it is appended to the
-// winner list in pixel order, with one atomic per block pass.  k_shade_wins
-// then shades one winner per thread, without tiles or barriers.
-constexpr int kClassifyPx = 8; // pixels per thread and block pass
+// two passes.  k_classify streams the view's depth keys, four consecutive
+// pixels a thread: background colour and every pixel's depth are written at
+// once, and the winners appended to the winner list in pixel order, with one
+// atomic per block pass; it also makes k_winners' records (nothing it does
+// depends on them, and a pass of its own cost a launch).  k_shade_wins then
+// shades one winner per thread, without tiles or barriers, and resets its key
+// to empty (unless kept for debug).
+//
+// Bound by the latency of its stream (40 % issue) as single keys, with an
+// integer division a pixel; where the target's rows are contiguous and
+// aligned (a whole frame, a staged or depth-of-field view) a thread reads its
+// keys as 32 bytes and writes colour and depth as 16, without rows.
+// Classify and records: 1080p 14.8 -> 10.0 us, 4K 45.8 -> 37.1 us (132 MB of keys,
+// colour and depth).  Taking the records last in every other block, beside the
+// stream, measured slower (42.5 us).
+constexpr int kClassifyPx = 4;   // consecutive pixels of a thread
+constexpr int kClassifyRuns = 2; // ... and runs of them in flight per block pass
 
-__global__ void __launch_bounds__(256) k_classify(const BatchDev *b)
+__global__ void __launch_bounds__(256, 4) k_classify(const BatchDev *b)
 {
-    static_assert(kClassifyPx % 4 == 0, "the counts divide among the scan warp's lanes");
-    __shared__ uint32_t at[kClassifyPx * 8]; // per (pass row j, warp): winners, then their first list index
+    winner_records(b);
+    __shared__ uint32_t at[kClassifyRuns * 8]; // per (run, warp): winners, then their first list index
     __shared__ uint32_t base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool keep = b->keep_keys != 0;
-    const uint32_t total = b->total_px;
-    int item = -1;
-    uint32_t lo = 0, hi = 0;
-    for (uint32_t c0 = blockIdx.x * (256u * kClassifyPx); c0 < total; c0 += gridDim.x * (256u * kClassifyPx)) {
-        unsigned long long k[kClassifyPx];
+    const ItemDev &it = b->items[0];
+    const uint32_t total = b->total_px, w = (uint32_t)it.v.w;
+    const unsigned long long *keys = b->key_pool;
+    uint32_t *pixels = it.pixels;
+    float *zbuf = it.zbuf;
+    const bool whole = it.pitch_px == it.v.w && ((reinterpret_cast<uintptr_t>(pixels) & 15) == 0) &&
+                       ((reinterpret_cast<uintptr_t>(zbuf) & 15) == 0);
+    const uint32_t pass = 256u * kClassifyPx * kClassifyRuns;
+    for (uint32_t c0 = blockIdx.x * pass; c0 < total; c0 += gridDim.x * pass) {
+        unsigned long long k[kClassifyRuns][kClassifyPx];
 #pragma unroll
-        for (int j = 0; j < kClassifyPx; j++) {
-            const uint32_t g = c0 + j * 256u + threadIdx.x;
-            k[j] = g < total ? b->key_pool[g] : kEmptyKey;
-        }
-        unsigned m[kClassifyPx];
+        for (int r = 0; r < kClassifyRuns; r++) {
+            const uint32_t g = c0 + (r * 256u + threadIdx.x) * kClassifyPx;
+            if (g + kClassifyPx <= total) { // (the key pool is 256-byte aligned)
+                asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                             : "=l"(k[r][0]), "=l"(k[r][1]), "=l"(k[r][2]), "=l"(k[r][3])
+                             : "l"(keys + g));
+            } else {
 #pragma unroll
-        for (int j = 0; j < kClassifyPx; j++) {
-            const uint32_t g = c0 + j * 256u + threadIdx.x;
-            bool win = false;
-            if (g < total) {
-                if (g < lo || g >= hi) {
-                    item = find_item(b->px_base, b->n_items, g);
-                    lo = __ldg(b->px_base + item);
-                    hi = __ldg(b->px_base + item + 1);
-                }
-                const ItemDev &it = b->items[item];
-                const uint32_t i = g - lo, w = (uint32_t)it.v.w;
-                const uint32_t y = i / w, x = i - y * w;
-                if (k[j] == kEmptyKey) {
-                    it.pixels[(long long)y * it.pitch_px + x] = 0u;
-                    if (it.zbuf)
-                        it.zbuf[i] = __uint_as_float(kMaxZBits);
-                } else {
-                    win = true;
-                    if (it.zbuf)
-                        it.zbuf[i] = __uint_as_float((uint32_t)(k[j] >> 32));
-                    if (!keep)
-                        b->key_pool[g] = kEmptyKey;
-                }
+                for (int j = 0; j < kClassifyPx; j++)
+                    k[r][j] = g + j < total ? keys[g + j] : kEmptyKey;
             }
-            m[j] = __ballot_sync(0xFFFFFFFFu, win);
-            if (lane == 0)
-                at[j * 8 + warp] = __popc(m[j]);
         }
-        __syncthreads();
-        if (warp == 0) {
-            // exclusive prefix of the counts in (j, warp) order, which is pixel
-            // order: each lane takes kPerLane consecutive counts
-            constexpr int kPerLane = kClassifyPx * 8 / 32;
-            uint32_t a[kPerLane], sum = 0;
+        uint32_t first[kClassifyRuns]; // this lane's winners follow so many of its warp's
 #pragma unroll
-            for (int q = 0; q < kPerLane; q++) {
-                a[q] = at[kPerLane * lane + q];
-                sum += a[q];
+        for (int r = 0; r < kClassifyRuns; r++) {
+            const uint32_t g = c0 + (r * 256u + threadIdx.x) * kClassifyPx;
+            float z[kClassifyPx];
+            uint32_t n = 0;
+#pragma unroll
+            for (int j = 0; j < kClassifyPx; j++) {
+                const bool win = k[r][j] != kEmptyKey;
+                z[j] = __uint_as_float(win ? (uint32_t)(k[r][j] >> 32) : kMaxZBits);
+                n += win;
             }
-            uint32_t incl = sum;
+            if (whole && g + kClassifyPx <= total) {
+                // (a winner's colour is written by the shade)
+                *reinterpret_cast<uint4 *>(pixels + g) = make_uint4(0u, 0u, 0u, 0u);
+                if (zbuf)
+                    *reinterpret_cast<float4 *>(zbuf + g) = make_float4(z[0], z[1], z[2], z[3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < kClassifyPx; j++)
+                    if (g + j < total) {
+                        const uint32_t y = (g + j) / w, x = g + j - y * w;
+                        pixels[(long long)y * it.pitch_px + x] = 0u;
+                        if (zbuf)
+                            zbuf[g + j] = z[j];
+                    }
+            }
+            uint32_t incl = n;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
                 if (lane >= d)
                     incl += t;
             }
-            uint32_t run = incl - sum;
+            first[r] = incl - n;
+            if (lane == 31)
+                at[r * 8 + warp] = incl;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // exclusive prefix of the counts in (run, warp) order, which is pixel order
+            const uint32_t a = lane < kClassifyRuns * 8 ? at[lane] : 0u;
+            uint32_t incl = a;
 #pragma unroll
-            for (int q = 0; q < kPerLane; q++) {
-                at[kPerLane * lane + q] = run;
-                run += a[q];
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= d)
+                    incl += t;
             }
+            if (lane < kClassifyRuns * 8)
+                at[lane] = incl - a;
             if (lane == 31)
                 base = incl ? atomicAdd(counter32(b, C_WINS), incl) : 0u;
         }
         __syncthreads();
-        const unsigned below = (1u << lane) - 1u;
 #pragma unroll
-        for (int j = 0; j < kClassifyPx; j++)
-            if (m[j] & (1u << lane)) {
-                const uint32_t g = c0 + j * 256u + threadIdx.x;
-                const uint32_t e = base + at[j * 8 + warp] + __popc(m[j] & below);
-                if (in_bounds(e < total, CHK_PIXEL, e))
-                    b->wins[e] = make_uint2(g, (uint32_t)k[j]);
-            }
+        for (int r = 0; r < kClassifyRuns; r++) {
+            uint32_t e = base + at[r * 8 + warp] + first[r];
+#pragma unroll
+            for (int j = 0; j < kClassifyPx; j++)
+                if (k[r][j] != kEmptyKey && in_bounds(e < total, CHK_PIXEL, e))
+                    b->wins[e++] = make_uint2(c0 + (r * 256u + threadIdx.x) * kClassifyPx + j, (uint32_t)k[r][j]);
+        }
         __syncthreads(); // `at` and `base` are reused by the next pass
     }
 }
@@ -2491,22 +2511,18 @@ template <bool ALL_MODES>
 __global__ void __launch_bounds__(kShadeThreads, SGL_SHADE_MIN_BLOCKS) k_shade_wins(const BatchDev *b)
 {
     const uint32_t n = *counter32(b, C_WINS);
-    const bool overflow = *counter32(b, C_OVERFLOW) != 0u;
-    int item = -1;
-    uint32_t lo = 0, hi = 0;
+    const bool overflow = *counter32(b, C_OVERFLOW) != 0u, keep = b->keep_keys != 0;
+    const ItemDev &it = b->items[0];
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const uint2 wn = b->wins[e];
-        if (wn.x < lo || wn.x >= hi) {
-            item = find_item(b->px_base, b->n_items, wn.x);
-            lo = __ldg(b->px_base + item);
-            hi = __ldg(b->px_base + item + 1);
-        }
-        const ItemDev &it = b->items[item];
-        const uint32_t i = wn.x - lo;
-        const uint32_t c = shade_winner_impl<ALL_MODES>(b, (uint32_t)item, i, wn.y, overflow);
+        const uint32_t i = wn.x;
+        const uint32_t c = shade_winner_impl<ALL_MODES>(b, 0u, i, wn.y, overflow);
         const uint32_t y = i / (uint32_t)it.v.w, x = i - y * (uint32_t)it.v.w;
-        if (in_bounds(y < (uint32_t)it.v.h, CHK_PIXEL, i))
+        if (in_bounds(y < (uint32_t)it.v.h, CHK_PIXEL, i)) {
             it.pixels[(long long)y * it.pitch_px + x] = c;
+            if (!keep)
+                b->key_pool[i] = kEmptyKey;
+        }
     }
 }
 
@@ -2520,10 +2536,9 @@ __device__ __forceinline__ bool frags_overflowed(const BatchDev *b)
 
 __constant__ float2 c_dof_taps[SGL_DOF_TAPS];
 
-// Circle of confusion of pixel i of a depth-of-field item.
-__device__ __forceinline__ float dof_radius(const ItemDev &it, uint32_t i)
+// Circle of confusion at depth zp of a depth-of-field item.
+__device__ __forceinline__ float dof_radius_at(const ItemDev &it, float zp)
 {
-    const float zp = it.zbuf[i];
     const float zv = (zp - it.p23) / it.p22;
     float r = (it.dof_ka * fabsf(zv - it.dof_focus)) / zv;
     if (!(r >= 0.0f && r <= it.dof_rmax))
@@ -2531,9 +2546,40 @@ __device__ __forceinline__ float dof_radius(const ItemDev &it, uint32_t i)
     return r;
 }
 
+// ... with `far` the radius of an empty pixel (the cleared depth), whose huge
+// operands would take both divisions through their slow path.
+__device__ __forceinline__ float dof_radius(const ItemDev &it, float zp, float far)
+{
+    return __float_as_uint(zp) == kMaxZBits ? far : dof_radius_at(it, zp);
+}
+
 __device__ __forceinline__ uint32_t dof_average(uint32_t centre, uint32_t sb, uint32_t sg, uint32_t sr)
 {
     return (centre & 0xFF000000u) | (((sr + 16u) / 32u) << 16) | (((sg + 16u) / 32u) << 8) | ((sb + 16u) / 32u);
+}
+
+// 1.5 * 2^23: a float of magnitude below 2^22 added to it is rounded to the
+// nearest integer (ties to even, as __float2int_rn), which is the sum's bits
+// less kTapBias.  One full-rate addition, where the conversion unit takes a
+// warp per two cycles: with two conversions a tap that unit bound the gather
+// of pixels of unlike radius.
+constexpr float kTapRound = 12582912.0f;
+constexpr uint32_t kTapBias = 0x4B400000u;
+
+// r * tap rounded to the nearest integers, each plus kTapBias (|r| < 2^22).
+// (Paired single-precision instructions would halve these four, but a paired
+// product, even as a fused multiply-add with -0, and a paired addition came
+// out contracted: offsets one off in a pixel of a million.)
+__device__ __forceinline__ uint2 tap_offset(float r, float2 t)
+{
+    return make_uint2(__float_as_uint(__fadd_rn(__fmul_rn(r, t.x), kTapRound)),
+                      __float_as_uint(__fadd_rn(__fmul_rn(r, t.y), kTapRound)));
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
 }
 
 // Depth-of-field gather (replaces post_shader_depth_box,
@@ -2548,193 +2594,307 @@ __device__ __forceinline__ uint32_t dof_average(uint32_t centre, uint32_t sb, ui
 // A block takes kDofTile x kDofTile tiles of the items that ask for the
 // gather and stages the tile with its halo (the taps reach at most
 // ceil(max_radius) pixels: every tap component is below 1), clamped to the
-// view as the taps are, in shared memory (rows kDofPitch apart); the 32 taps
-// of each pixel then read shared memory without further clamping.  Views whose reach exceeds
+// view as the taps are, in shared memory; the 32 taps of each pixel then read
+// shared memory without further clamping.  Halos of up to 16 pixels (the usual
+// radius) take half the shared memory, and the next tile's halo is copied in
+// (and its depths loaded) while this one is gathered; wider ones are staged
+// before each tile.  Inside the view a halo is copied as 16-byte words, where
+// the source's rows are aligned to them.  Views whose reach exceeds
 // kDofMaxHalo gather from the colour buffer.
+//
+// Bound by integer issue (two ALU instructions and a shared-memory read a
+// pixel and tap); before, staging took a quarter of the instructions a word at
+// a time and its latency was the main stall (3840 x 2160, radius 16: 64.2 M
+// instructions and 92 us, now 55.7 M and 71 us; 2560 x 1440 of unlike radii up
+// to 24: 64 -> 55 us).
 constexpr int kDofBlocks = 5; // resident blocks per SM (shared memory: 37 KB each)
+constexpr int kDofNear = 16;  // halo whose tiles are staged ahead
+constexpr int kDofNearPitch = kDofTile + 2 * kDofNear;
+static_assert(2 * kDofNearPitch * kDofNearPitch <= kDofPitch * kDofPitch, "two near tiles share the shared memory");
+static_assert(kDofTile == 32 && kDofNear % 4 == 0 && kDofMaxHalo % 4 == 0, "16-byte words of a halo");
+
+// The tile in hand: its item, place and, per thread, the pixels' depths and
+// the staged pixel that a constant tile repeats.
+struct DofTile {
+    const ItemDev *it;
+    int x0, y0, w, h;
+    float z[4]; // of rows y0 + warp + 8 j, column x0 + lane (clamped into the view)
+    uint32_t ref;
+
+    __device__ __forceinline__ void load_depths()
+    {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int x = x0 + lane < w ? x0 + lane : x0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int y = y0 + warp + 8 * j;
+            z[j] = y < h ? it->zbuf[(uint32_t)y * (uint32_t)w + (uint32_t)x] : 0.0f;
+        }
+        ref = __ldg(it->dof_src + (size_t)y0 * it->dof_src_pitch + x0);
+    }
+};
+
+// Copies the tile and PITCH-wide halo (view-clamped) into `halo` with
+// cp.async (not committed); the tile's pixel (0, 0) lands at row and column
+// (PITCH - kDofTile) / 2.
+template <int PITCH> __device__ __forceinline__ void dof_stage(const DofTile &t, uint32_t *halo)
+{
+    constexpr int R = (PITCH - kDofTile) / 2, V = PITCH / 4; // 16-byte words of a row
+    const uint32_t *src = t.it->dof_src;
+    const int sp = t.it->dof_src_pitch;
+    const int xa = t.x0 - R, ya = t.y0 - R;
+    if (xa >= 0 && xa + PITCH <= t.w && (sp & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        for (int i = (int)threadIdx.x; i < PITCH * V; i += 256) {
+            const int yy = i / V, v = i - yy * V;
+            const int sy = min(max(ya + yy, 0), t.h - 1);
+            cp_async<16>(halo + yy * PITCH + 4 * v, src + (size_t)sy * sp + xa + 4 * v);
+        }
+    } else {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int yy = warp; yy < PITCH; yy += 8) {
+            const uint32_t *row = src + (size_t)min(max(ya + yy, 0), t.h - 1) * sp;
+#pragma unroll
+            for (int c = 0; c < PITCH; c += 32)
+                cp_async<4>(halo + yy * PITCH + c + lane, row + min(max(xa + c + lane, 0), t.w - 1));
+        }
+    }
+}
+
+// Whether every word that this thread staged holds t.ref.
+template <int PITCH> __device__ __forceinline__ bool dof_same(const DofTile &t, const uint32_t *halo)
+{
+    bool same = true;
+    for (int i = (int)threadIdx.x; i < PITCH * PITCH / 4; i += 256) {
+        const uint4 v = reinterpret_cast<const uint4 *>(halo)[i];
+        same &= v.x == t.ref && v.y == t.ref && v.z == t.ref && v.w == t.ref;
+    }
+    return same;
+}
+
+// The gather of a staged tile; `far` as in dof_radius.
+template <int PITCH> __device__ __forceinline__ void dof_gather(const DofTile &t, const uint32_t *halo, float far)
+{
+    constexpr int R = (PITCH - kDofTile) / 2;
+    const ItemDev &it = *t.it;
+    // Warp w takes rows w, w + 8, w + 16 and w + 24 of the tile, a lane
+    // one column.  The sums are exact integers, so the taps may be
+    // taken in any order: rb sums bytes 0 and 2 in two 16-bit lanes
+    // (32 x 255 fits), g sums whole pixels modulo 2^32, so that bits
+    // 8..23 of g - rb are the sum of byte 1 (below 2^24 after the
+    // shift: byte 3's sum lands at bit 24 and up); alpha is the
+    // centre's.
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w = t.w, h = t.h, x0 = t.x0, y0 = t.y0, x = x0 + lane;
+    if (y0 + warp >= h)
+        return;
+    const bool valid = x < w;
+    const int xs = valid ? x : x0; // lanes past the view's right edge work on a pixel inside
+    float r[4];
+    bool uniform = true;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        r[j] = y0 + warp + 8 * j < h ? dof_radius(it, t.z[j], far) : 0.0f;
+    const float r0 = __shfl_sync(0xFFFFFFFFu, r[0], 0);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        uniform &= !valid || y0 + warp + 8 * j >= h || r[j] == r0;
+    // the halo holds the view-clamped pixels, so a tap needs no
+    // clamp: |offset| <= ceil(r) <= R keeps it inside
+    const uint32_t *c = halo + (warp + R) * PITCH + (xs - x0 + R);
+    uint32_t rb[4] = {0u, 0u, 0u, 0u}, g[4] = {0u, 0u, 0u, 0u};
+    if (__all_sync(0xFFFFFFFFu, uniform)) {
+        // one radius for the warp's 128 pixels (the clamped radius,
+        // or the empty background's): lane k makes tap k's offset
+        // once, and each offset serves the four rows
+        static_assert(SGL_DOF_TAPS == 32, "one tap per lane");
+        const float2 tap = c_dof_taps[lane];
+        const int off = __float2int_rn(r0 * tap.y) * PITCH + __float2int_rn(r0 * tap.x);
+#pragma unroll 4
+        for (int k = 0; k < SGL_DOF_TAPS; k += 2) {
+            const uint32_t *q = c + __shfl_sync(0xFFFFFFFFu, off, k);
+            const uint32_t *p = c + __shfl_sync(0xFFFFFFFFu, off, k + 1);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t v = q[8 * j * PITCH], u = p[8 * j * PITCH];
+                rb[j] += (v & 0x00FF00FFu) + (u & 0x00FF00FFu);
+                g[j] += v + u;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (y0 + warp + 8 * j >= h)
+                break; // the whole warp
+            const uint32_t *cj = c + 8 * j * PITCH;
+            const float rj0 = __shfl_sync(0xFFFFFFFFu, r[j], 0);
+            if (__all_sync(0xFFFFFFFFu, !valid || r[j] == rj0)) {
+                const float2 tap = c_dof_taps[lane];
+                const int off = __float2int_rn(rj0 * tap.y) * PITCH + __float2int_rn(rj0 * tap.x);
+#pragma unroll 4
+                for (int k = 0; k < SGL_DOF_TAPS; k += 2) {
+                    const uint32_t v = cj[__shfl_sync(0xFFFFFFFFu, off, k)];
+                    const uint32_t u = cj[__shfl_sync(0xFFFFFFFFu, off, k + 1)];
+                    rb[j] += (v & 0x00FF00FFu) + (u & 0x00FF00FFu);
+                    g[j] += v + u;
+                }
+            } else {
+                // the pixel's shared address less the offsets' bias
+                const uint32_t at = (uint32_t)__cvta_generic_to_shared(cj) - kTapBias * (4u + 4u * (uint32_t)PITCH);
+#pragma unroll 8
+                for (int k = 0; k < SGL_DOF_TAPS; k += 2) {
+                    const uint2 a = tap_offset(r[j], c_dof_taps[k]), e = tap_offset(r[j], c_dof_taps[k + 1]);
+                    const uint32_t v = lds32(at + a.y * (4u * (uint32_t)PITCH) + 4u * a.x);
+                    const uint32_t u = lds32(at + e.y * (4u * (uint32_t)PITCH) + 4u * e.x);
+                    rb[j] += (v & 0x00FF00FFu) + (u & 0x00FF00FFu);
+                    g[j] += v + u;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int y = y0 + warp + 8 * j;
+        if (valid && y < h)
+            it.dof_out[(size_t)y * it.dof_pitch + x] =
+                dof_average(c[8 * j * PITCH], rb[j] & 0xFFFFu, ((g[j] - rb[j]) >> 8) & 0xFFFFu, rb[j] >> 16);
+    }
+}
+
+// A tile whose staged pixels all hold t.ref: every tap of every pixel reads
+// that value: 32 equal channels c sum to 32 c, and (32 c + 16) / 32 = c, alpha
+// is the centre's: the gather leaves it unchanged.
+__device__ __forceinline__ void dof_constant(const DofTile &t)
+{
+    const ItemDev &it = *t.it;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int x = t.x0 + lane, y = t.y0 + warp + 8 * j;
+        if (x < t.w && y < t.h)
+            it.dof_out[(size_t)y * it.dof_pitch + x] = t.ref;
+    }
+}
+
+// A tile gathered from the colour buffer.
+__device__ __noinline__ void dof_from_memory(const ItemDev &it, int x0, int y0, float far)
+{
+    const int w = it.v.w, h = it.v.h;
+    for (int p = threadIdx.x; p < kDofTile * kDofTile; p += blockDim.x) {
+        const int x = x0 + (p & (kDofTile - 1)), y = y0 + p / kDofTile;
+        if (y >= h)
+            continue; // the whole warp
+        const bool valid = x < w;
+        const int xs = valid ? x : x0;
+        const float z = it.zbuf[(uint32_t)y * (uint32_t)w + (uint32_t)xs];
+        const float r = dof_radius(it, z, far);
+        uint32_t rb = 0, g = 0; // (as in dof_gather)
+#pragma unroll 8
+        for (int k = 0; k < SGL_DOF_TAPS; k++) {
+            const uint2 o = tap_offset(r, c_dof_taps[k]);
+            int sx = xs + (int)(o.x - kTapBias), sy = y + (int)(o.y - kTapBias);
+            sx = sx < 0 ? 0 : (sx >= w ? w - 1 : sx);
+            sy = sy < 0 ? 0 : (sy >= h ? h - 1 : sy);
+            const uint32_t v = __ldg(it.dof_src + (size_t)sy * it.dof_src_pitch + sx);
+            rb += v & 0x00FF00FFu;
+            g += v;
+        }
+        if (valid)
+            it.dof_out[(size_t)y * it.dof_pitch + x] = dof_average(it.dof_src[(size_t)y * it.dof_src_pitch + xs],
+                                                                   rb & 0xFFFFu, ((g - rb) >> 8) & 0xFFFFu, rb >> 16);
+    }
+}
 
 __global__ void __launch_bounds__(256, kDofBlocks) k_dof(const BatchDev *b)
 {
     if (frags_overflowed(b))
         return; // a layered view whose fragment pool was too small: rendered again
-    __shared__ uint32_t halo[kDofPitch * kDofPitch];
-    __shared__ uint32_t claim[2]; // this tile and the next (tiles cost from a copy to a full gather)
+    __shared__ __align__(16) uint32_t halo[kDofPitch * kDofPitch];
+    __shared__ uint32_t claim[4]; // tiles of the next rounds (tiles cost from a copy to a full gather)
+    const uint32_t total = b->total_dof_tiles;
     int item = -1;
     uint32_t lo = 0, hi = 0;
-    if (threadIdx.x == 0)
-        claim[0] = atomicAdd(counter32(b, C_DOF_NEXT), 1u);
-    __syncthreads();
-    for (int cb = 0;; cb ^= 1) {
-        const uint32_t tg = claim[cb];
-        if (tg >= b->total_dof_tiles)
-            break;
-        if (threadIdx.x == 0)
-            claim[cb ^ 1] = atomicAdd(counter32(b, C_DOF_NEXT), 1u);
+    float far = 0.0f, far_next = 0.0f; // the items' radii of an empty pixel
+    // the place of tile tg
+    auto locate = [&](uint32_t tg, DofTile &t) {
         if (tg < lo || tg >= hi) {
             item = find_item(b->dof_base, b->n_items, tg);
             lo = __ldg(b->dof_base + item);
             hi = __ldg(b->dof_base + item + 1);
+            far_next = dof_radius_at(b->items[item], __uint_as_float(kMaxZBits));
         }
-        const ItemDev &it = b->items[item];
-        const int w = it.v.w, h = it.v.h;
-        const uint32_t tl = tg - lo;
-        const int x0 = (int)(tl % (uint32_t)it.dof_tiles_x) * kDofTile;
-        const int y0 = (int)(tl / (uint32_t)it.dof_tiles_x) * kDofTile;
-        const int R = it.dof_halo;
-        const int S = kDofTile + 2 * R;
-        if (R >= 0) {
-            // rows of the halo to warps, columns to lanes (S <= 96: 3 per lane)
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            int c0 = x0 - R + lane, c1 = c0 + 32, c2 = c0 + 64;
-            c0 = c0 < 0 ? 0 : (c0 >= w ? w - 1 : c0);
-            c1 = c1 < 0 ? 0 : (c1 >= w ? w - 1 : c1);
-            c2 = c2 < 0 ? 0 : (c2 >= w ? w - 1 : c2);
-            // the staged pixels' common value, if they all have one
-            const uint32_t ref = __ldg(it.dof_src + (size_t)y0 * it.dof_src_pitch + x0);
-            bool same = true;
-#pragma unroll 4
-            for (int yy = warp; yy < S; yy += 8) {
-                int sy = y0 - R + yy;
-                sy = sy < 0 ? 0 : (sy >= h ? h - 1 : sy);
-                const uint32_t *row = it.dof_src + (size_t)sy * it.dof_src_pitch;
-                uint32_t *dst = halo + yy * kDofPitch;
-                if (lane < S) {
-                    const uint32_t v = __ldg(row + c0);
-                    dst[lane] = v;
-                    same &= v == ref;
-                }
-                if (lane + 32 < S) {
-                    const uint32_t v = __ldg(row + c1);
-                    dst[lane + 32] = v;
-                    same &= v == ref;
-                }
-                if (lane + 64 < S) {
-                    const uint32_t v = __ldg(row + c2);
-                    dst[lane + 64] = v;
-                    same &= v == ref;
-                }
-            }
-            if (__syncthreads_and(same)) {
-                // Every tap of every pixel of the tile reads the value ref:
-                // 32 equal channels c sum to 32 c, and (32 c + 16) / 32 = c,
-                // alpha is the centre's: the gather leaves ref unchanged.
-                for (int p = threadIdx.x; p < kDofTile * kDofTile; p += blockDim.x) {
-                    const int x = x0 + (p & (kDofTile - 1)), y = y0 + p / kDofTile;
-                    if (x < w && y < h)
-                        it.dof_out[(size_t)y * it.dof_pitch + x] = ref;
-                }
-                __syncthreads(); // the halo is reused by the next tile, claim[cb ^ 1] is written
-                continue;
-            }
-        }
-        if (R >= 0) {
-            // Warp w takes rows w, w + 8, w + 16 and w + 24 of the tile, a lane
-            // one column.  The sums are exact integers, so the taps may be
-            // taken in any order: rb sums bytes 0 and 2 in two 16-bit lanes
-            // (32 x 255 fits), g sums whole pixels modulo 2^32, so that bits
-            // 8..23 of g - rb are the sum of byte 1 (below 2^24 after the
-            // shift: byte 3's sum lands at bit 24 and up); alpha is the
-            // centre's.
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            const int x = x0 + lane;
-            const bool valid = x < w;
-            const int xs = valid ? x : x0; // lanes past the view's right edge work on a pixel inside
-            if (y0 + warp < h) {
-                float r[4];
-                bool uniform = true;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int y = y0 + warp + 8 * j;
-                    r[j] = y < h ? dof_radius(it, (uint32_t)y * (uint32_t)w + (uint32_t)xs) : 0.0f;
-                }
-                const float r0 = __shfl_sync(0xFFFFFFFFu, r[0], 0);
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    uniform &= !valid || y0 + warp + 8 * j >= h || r[j] == r0;
-                // the halo holds the view-clamped pixels, so a tap needs no
-                // clamp: |offset| <= ceil(r) <= R keeps it inside
-                const uint32_t *c = halo + (warp + R) * kDofPitch + (xs - x0 + R);
-                uint32_t rb[4] = {0u, 0u, 0u, 0u}, g[4] = {0u, 0u, 0u, 0u};
-                if (__all_sync(0xFFFFFFFFu, uniform)) {
-                    // one radius for the warp's 128 pixels (the clamped radius,
-                    // or the empty background's): lane k makes tap k's offset
-                    // once, and each offset serves the four rows
-                    static_assert(SGL_DOF_TAPS == 32, "one tap per lane");
-                    const float2 t = c_dof_taps[lane];
-                    const int off = __float2int_rn(r0 * t.y) * kDofPitch + __float2int_rn(r0 * t.x);
-#pragma unroll 4
-                    for (int k = 0; k < SGL_DOF_TAPS; k++) {
-                        const uint32_t *q = c + __shfl_sync(0xFFFFFFFFu, off, k);
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const uint32_t v = q[8 * j * kDofPitch];
-                            rb[j] += v & 0x00FF00FFu;
-                            g[j] += v;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if (y0 + warp + 8 * j >= h)
-                            break; // the whole warp
-                        const uint32_t *cj = c + 8 * j * kDofPitch;
-                        const float rj0 = __shfl_sync(0xFFFFFFFFu, r[j], 0);
-                        if (__all_sync(0xFFFFFFFFu, !valid || r[j] == rj0)) {
-                            const float2 t = c_dof_taps[lane];
-                            const int off = __float2int_rn(rj0 * t.y) * kDofPitch + __float2int_rn(rj0 * t.x);
-#pragma unroll 8
-                            for (int k = 0; k < SGL_DOF_TAPS; k++) {
-                                const uint32_t v = cj[__shfl_sync(0xFFFFFFFFu, off, k)];
-                                rb[j] += v & 0x00FF00FFu;
-                                g[j] += v;
-                            }
-                        } else {
-#pragma unroll 8
-                            for (int k = 0; k < SGL_DOF_TAPS; k++) {
-                                const float2 t = c_dof_taps[k];
-                                const uint32_t v = cj[__float2int_rn(r[j] * t.y) * kDofPitch + __float2int_rn(r[j] * t.x)];
-                                rb[j] += v & 0x00FF00FFu;
-                                g[j] += v;
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int y = y0 + warp + 8 * j;
-                    if (valid && y < h)
-                        it.dof_out[(size_t)y * it.dof_pitch + x] =
-                            dof_average(c[8 * j * kDofPitch], rb[j] & 0xFFFFu, ((g[j] - rb[j]) >> 8) & 0xFFFFu,
-                                        rb[j] >> 16);
-                }
-            }
-        } else {
-            for (int p = threadIdx.x; p < kDofTile * kDofTile; p += blockDim.x) {
-                const int x = x0 + (p & (kDofTile - 1)), y = y0 + p / kDofTile;
-                if (y >= h)
-                    continue; // the whole warp
-                const bool valid = x < w;
-                const int xs = valid ? x : x0;
-                const float r = dof_radius(it, (uint32_t)y * (uint32_t)w + (uint32_t)xs);
-                uint32_t sb = 0, sg = 0, sr = 0;
-#pragma unroll 8
-                for (int k = 0; k < SGL_DOF_TAPS; k++) {
-                    const float2 t = c_dof_taps[k];
-                    int sx = xs + __float2int_rn(r * t.x), sy = y + __float2int_rn(r * t.y);
-                    sx = sx < 0 ? 0 : (sx >= w ? w - 1 : sx);
-                    sy = sy < 0 ? 0 : (sy >= h ? h - 1 : sy);
-                    const uint32_t v = __ldg(it.dof_src + (size_t)sy * it.dof_src_pitch + sx);
-                    sb += v & 0xFFu;
-                    sg += (v >> 8) & 0xFFu;
-                    sr += (v >> 16) & 0xFFu;
-                }
-                if (valid)
-                    it.dof_out[(size_t)y * it.dof_pitch + x] =
-                        dof_average(it.dof_src[(size_t)y * it.dof_src_pitch + xs], sb, sg, sr);
-            }
-        }
-        __syncthreads(); // the halo is reused by the next tile, claim[cb ^ 1] is written
+        t.it = b->items + item;
+        t.w = t.it->v.w;
+        t.h = t.it->v.h;
+        const uint32_t tl = tg - lo, tx = (uint32_t)t.it->dof_tiles_x;
+        t.y0 = (int)(tl / tx) * kDofTile;
+        t.x0 = (int)(tl % tx) * kDofTile;
+    };
+    auto near = [](const DofTile &t) { return t.it->dof_halo >= 0 && t.it->dof_halo <= kDofNear; };
+    if (threadIdx.x == 0) {
+        claim[0] = atomicAdd(counter32(b, C_DOF_NEXT), 1u);
+        claim[1] = atomicAdd(counter32(b, C_DOF_NEXT), 1u);
     }
+    __syncthreads();
+    DofTile t{}, next{};
+    uint32_t tg = claim[0];
+    if (tg < total) {
+        locate(tg, t);
+        far = far_next;
+        if (near(t)) {
+            dof_stage<kDofNearPitch>(t, halo);
+            t.load_depths();
+        }
+    }
+    cp_async_commit();
+    for (int q = 0; tg < total; q++) {
+        // this round's tile is in hand; claim the one after the next, and
+        // start on the next
+        const uint32_t tn = claim[(q + 1) & 3];
+        if (threadIdx.x == 0)
+            claim[(q + 2) & 3] = atomicAdd(counter32(b, C_DOF_NEXT), 1u);
+        uint32_t *mine = halo + (q & 1) * kDofNearPitch * kDofNearPitch;
+        const bool mine_near = near(t);
+        bool next_near = false;
+        if (tn < total) {
+            locate(tn, next);
+            next_near = near(next);
+            if (next_near && mine_near) {
+                dof_stage<kDofNearPitch>(next, halo + ((q + 1) & 1) * kDofNearPitch * kDofNearPitch);
+                next.load_depths();
+            }
+        }
+        cp_async_commit();
+        if (mine_near) {
+            cp_async_wait<1>();
+            __syncthreads();
+            if (__syncthreads_and(dof_same<kDofNearPitch>(t, mine)))
+                dof_constant(t);
+            else
+                dof_gather<kDofNearPitch>(t, mine, far);
+        } else if (t.it->dof_halo >= 0) {
+            dof_stage<kDofPitch>(t, halo);
+            t.load_depths();
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncthreads();
+            if (__syncthreads_and(dof_same<kDofPitch>(t, halo)))
+                dof_constant(t);
+            else
+                dof_gather<kDofPitch>(t, halo, far);
+        } else {
+            dof_from_memory(*t.it, t.x0, t.y0, far);
+        }
+        __syncthreads(); // the halo is reused, claim[(q + 2) & 3] is written
+        if (next_near && !mine_near) { // (its place was in use)
+            dof_stage<kDofNearPitch>(next, halo + ((q + 1) & 1) * kDofNearPitch * kDofNearPitch);
+            next.load_depths();
+            cp_async_commit();
+        }
+        t = next;
+        tg = tn;
+        far = far_next;
+    }
+    cp_async_wait<0>();
 }
 
 // The gather's input for a view with transparency layers: its rectangle of
@@ -3341,15 +3501,17 @@ cudaError_t launch_batch(const BatchDev *b, int tile, int flags, cudaStream_t st
     ran(PK_SPANS);
     n++;
     mark(PK_WINNER);
-    k_winners<<<sms * 4, 256, 0, st>>>(b);
-    ran(PK_WINNER);
-    n++;
+    if (!(flags & kSeqWinList)) { // (else by k_classify)
+        k_winners<<<sms * 4, 256, 0, st>>>(b);
+        ran(PK_WINNER);
+        n++;
+    }
     mark(PK_SHADE);
     // the kernel with every pixel shader only when a view asks for another
     // than the default, which then keeps all the registers
     const unsigned sg = sms * ((flags & kSeqWinList) ? SGL_SHADE_MIN_BLOCKS : SGL_TILE_MIN_BLOCKS);
     if (flags & kSeqWinList) {
-        k_classify<<<sms * 8, 256, 0, st>>>(b);
+        k_classify<<<sms * 4, 256, 0, st>>>(b);
         if (flags & kSeqShaders)
             k_shade_wins<true><<<sg, kShadeThreads, 0, st>>>(b);
         else
