@@ -20,7 +20,7 @@
 //
 // The array is shared by every call in a CUDA context and keeps the last
 // call's contents; each call clears what must start cleared (the counters in
-// the descriptor kernel, the depth keys to all ones with cudaMemsetAsync; the
+// the descriptor kernel, the depth keys to all ones there too; the
 // visibility flags are cleared by the kernels).  Calls that overlap on the
 // GPU in one context (on different streams, or from different host threads)
 // race on the array: the caller must order them.  Each CUDA context has its
@@ -33,6 +33,7 @@
 // (cuCtxGetId: ids are never reused in a process, so a context created after
 // cudaDeviceReset gets a fresh look-up).  Make that first call before any
 // stream capture.
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -119,20 +120,32 @@ static cudaError_t noalloc_scratch(unsigned char **out)
 struct NoAllocBases {
     uint32_t v[20];
 };
-__global__ void k_noalloc_setup(ItemDev it, BatchDev b, NoAllocBases bases, ItemDev *item_dst, BatchDev *batch_dst,
-                                uint32_t *bases_dst, unsigned long long *counters, unsigned long long *item_counters)
+// (Block 0 writes the descriptors, a word a thread; every block fills its
+// share of the depth keys with kEmptyKey, `key_words` 16-byte words.  One
+// thread copying the descriptors and a fill of its own cost 6.3 us before the
+// first kernel of a 960 x 540 frame.)
+__global__ void __launch_bounds__(256) k_noalloc_setup(ItemDev it, BatchDev b, NoAllocBases bases, ItemDev *item_dst,
+                                                       BatchDev *batch_dst, uint32_t *bases_dst,
+                                                       unsigned long long *counters,
+                                                       unsigned long long *item_counters, uint4 *keys,
+                                                       size_t key_words)
 {
+    static_assert(sizeof(ItemDev) % 8 == 0 && sizeof(BatchDev) % 8 == 0, "copied as words");
     const int t = threadIdx.x;
-    if (t == 0) {
-        *item_dst = it;
-        *batch_dst = b;
+    if (blockIdx.x == 0) {
+        for (int i = t; i < (int)(sizeof(ItemDev) / 8); i += 256)
+            reinterpret_cast<unsigned long long *>(item_dst)[i] = reinterpret_cast<const unsigned long long *>(&it)[i];
+        for (int i = t; i < (int)(sizeof(BatchDev) / 8); i += 256)
+            reinterpret_cast<unsigned long long *>(batch_dst)[i] = reinterpret_cast<const unsigned long long *>(&b)[i];
+        if (t < 20)
+            bases_dst[t] = bases.v[t];
+        for (int i = t; i < kCounterWords; i += 256)
+            counters[i] = 0ull;
+        if (t < 2)
+            item_counters[t] = 0ull;
     }
-    if (t < 20)
-        bases_dst[t] = bases.v[t];
-    for (int i = t; i < kCounterWords; i += blockDim.x)
-        counters[i] = 0ull;
-    if (t < 2)
-        item_counters[t] = 0ull;
+    for (size_t i = (size_t)blockIdx.x * 256 + t; i < key_words; i += (size_t)gridDim.x * 256)
+        keys[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
 }
 
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -298,11 +311,12 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     b.slot_flags = nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     // descriptors by value; the counters start at zero on every call
-    k_noalloc_setup<<<1, 256, 0, st>>>(it, b, bases, (ItemDev *)(base + o_item), (BatchDev *)(base + o_batch),
-                                       (uint32_t *)(base + o_bases), (unsigned long long *)(base + o_counters),
-                                       (unsigned long long *)(base + o_item_counters));
+    const size_t key_words = up256(8 * px) / 16;
+    k_noalloc_setup<<<(unsigned)std::min<size_t>((key_words + 1023) / 1024, 1024), 256, 0, st>>>(
+        it, b, bases, (ItemDev *)(base + o_item), (BatchDev *)(base + o_batch), (uint32_t *)(base + o_bases),
+        (unsigned long long *)(base + o_counters), (unsigned long long *)(base + o_item_counters),
+        (uint4 *)(base + o_key), key_words);
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemsetAsync(base + o_key, 0xFF, 8 * px, st)); // kEmptyKey
 
     const int seq = (dof ? kSeqDof : 0) | (v.shader != SGL_SHADER_PHONG_BILINEAR ? kSeqShaders : 0) |
                     (fused ? kSeqFused : 0) | (split ? kSeqSplit : 0) | (win_list ? kSeqWinList : 0) | kSeqOne;

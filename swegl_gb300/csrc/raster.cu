@@ -111,20 +111,49 @@ __global__ void k_world(SceneDev s)
     s.wnrm[g] = make_float4(nw.x, nw.y, nw.z, q.w);
 }
 
-// k_world for one posed request: the same transforms under the request's
-// node matrices, into its own arrays.
-__global__ void k_pose(SceneDev s, const float *node_world, const float *node_rs, float4 *wpos, float4 *wnrm)
+// k_world for a batch's posed views: the same transforms under each view's own
+// node matrices, into its own arrays, all views in one launch (a launch and a
+// copy per view, half of a 16-view batch's passes before its first triangle,
+// left the GPU idle between them).
+// Index of the pose whose blocks (`first`) hold block x.
+template <uint32_t PoseDev::*FIRST> __device__ __forceinline__ int find_pose(const PoseDev *p, int n, uint32_t x)
 {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= s.n_vertices)
-        return;
-    const uint32_t n = s.vnode[g];
-    const float4 p = s.pos_u[g];
-    const float4 q = s.nrm_v[g];
-    const V3 w = transform3(mk3(p.x, p.y, p.z), node_world + 16 * n);
-    const V3 nw = normalize3(normalize3(rotate_n(mk3(q.x, q.y, q.z), node_rs + 16 * n)));
-    wpos[g] = make_float4(w.x, w.y, w.z, p.w);
-    wnrm[g] = make_float4(nw.x, nw.y, nw.z, q.w);
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (p[mid].*FIRST <= x)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    return lo;
+}
+__global__ void __launch_bounds__(256) k_pose(const PoseDev *poses, int n)
+{
+    const PoseDev p = poses[find_pose<&PoseDev::vertex_block>(poses, n, blockIdx.x)];
+    const uint32_t g0 = (blockIdx.x - p.vertex_block) * kPoseVertices + threadIdx.x;
+    constexpr int kPer = kPoseVertices / 256;
+    float4 a[kPer], q[kPer];
+    uint32_t node[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint32_t g = g0 + 256 * k;
+        if (g < p.n_vertices) {
+            a[k] = p.pos_u[g];
+            q[k] = p.nrm_v[g];
+            node[k] = p.vnode[g];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint32_t g = g0 + 256 * k;
+        if (g >= p.n_vertices)
+            break;
+        const V3 w = transform3(mk3(a[k].x, a[k].y, a[k].z), p.node_world + 16 * node[k]);
+        const V3 nw = normalize3(normalize3(rotate_n(mk3(q[k].x, q[k].y, q[k].z), p.node_rs + 16 * node[k])));
+        p.wpos[g] = make_float4(w.x, w.y, w.z, a[k].w);
+        p.wnrm[g] = make_float4(nw.x, nw.y, nw.z, q[k].w);
+    }
 }
 
 // The box of each primitive's world positions (a warp per primitive), for the
@@ -133,15 +162,12 @@ __global__ void k_pose(SceneDev s, const float *node_world, const float *node_rs
 // each test of inside_camera_frustum that its other vertices fail, the
 // comparisons with NaN being false); a box that is empty or not finite gets a
 // NaN centre and is never culled.
-__global__ void k_box(SceneDev s, const float4 *wpos, float4 *pbox)
+__device__ __forceinline__ void primitive_box(uint4 gq, uint32_t n_vertices, const float4 *wpos, float4 *out)
 {
-    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (q >= s.n_prims)
-        return;
-    const uint4 gq = s.pgeo[q];
+    const uint32_t lane = threadIdx.x & 31;
     V3 lo = mk3(INFINITY, INFINITY, INFINITY), hi = mk3(-INFINITY, -INFINITY, -INFINITY);
     for (uint32_t i = lane; i < gq.y; i += 32) {
-        if (!in_bounds(gq.x + i < s.n_vertices, CHK_NDC, gq.x + i))
+        if (!in_bounds(gq.x + i < n_vertices, CHK_NDC, gq.x + i))
             break;
         const float4 w = wpos[gq.x + i];
         lo = mk3(fminf(lo.x, w.x), fminf(lo.y, w.y), fminf(lo.z, w.z));
@@ -159,9 +185,23 @@ __global__ void k_box(SceneDev s, const float4 *wpos, float4 *pbox)
     if (lane == 0) {
         float4 c, h;
         cull_box(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z), c, h);
-        pbox[2 * q] = c;
-        pbox[2 * q + 1] = h;
+        out[0] = c;
+        out[1] = h;
     }
+}
+__global__ void k_box(SceneDev s, const float4 *wpos, float4 *pbox)
+{
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (q < s.n_prims)
+        primitive_box(s.pgeo[q], s.n_vertices, wpos, pbox + 2 * q);
+}
+// ... of a batch's posed views.
+__global__ void __launch_bounds__(kPosePrims * 32) k_pose_box(const PoseDev *poses, int n)
+{
+    const PoseDev &p = poses[find_pose<&PoseDev::prim_block>(poses, n, blockIdx.x)];
+    const uint32_t q = (blockIdx.x - p.prim_block) * kPosePrims + (threadIdx.x >> 5);
+    if (p.pbox && q < p.n_prims)
+        primitive_box(p.pgeo[q], p.n_vertices, p.wpos, p.pbox + 2 * q);
 }
 
 // world_to_camera_or_frustum (vertex_shaders.hpp:35-52): view, projection
@@ -3320,14 +3360,12 @@ cudaError_t launch_world(const SceneDev &s, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_pose(const SceneDev &s, const float *node_world, const float *node_rs, float4 *wpos, float4 *wnrm,
-                        float4 *pbox, cudaStream_t st)
+cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, uint32_t prim_blocks, cudaStream_t st)
 {
-    if (s.n_vertices == 0)
-        return cudaSuccess;
-    k_pose<<<grid_for(s.n_vertices, 256), 256, 0, st>>>(s, node_world, node_rs, wpos, wnrm);
-    if (pbox && s.n_prims)
-        k_box<<<(s.n_prims + 7) / 8, 256, 0, st>>>(s, wpos, pbox);
+    if (vertex_blocks)
+        k_pose<<<vertex_blocks, 256, 0, st>>>(poses, n);
+    if (prim_blocks)
+        k_pose_box<<<prim_blocks, kPosePrims * 32, 0, st>>>(poses, n);
     return cudaGetLastError();
 }
 

@@ -117,7 +117,7 @@ static sgl_status render_layered(Ctx *ctx, Lane *lane, BatchEntry &e, const sgl_
     for (int attempt = 0; attempt < 3 && !fit; attempt++) {
         sgl_status r = lane->prepare(ctx, &e, 1, ctx->tile, ctx->inline_span, nullptr, &slot);
         if (r == SGL_OK)
-            r = lane->launch(ctx, slot, ctx->tile, false, launches, &ctx->prof);
+            r = lane->launch(ctx, slot, ctx->tile, false, want_stats, launches, &ctx->prof);
         if (r == SGL_OK)
             r = lane->layered_fit(ctx, slot, &fit);
         if (r != SGL_OK)
@@ -388,7 +388,7 @@ SGL_API sgl_status sgl_render(sgl_ctx *c, int scene_id, const sgl_view *views, c
         if (r == SGL_OK) {
             // one CUDA graph launch per view (captured once per lane slot and
             // sequence variant); direct launches while per-kernel timing is on
-            r = lane->launch(ctx, slot, ctx->tile, !ctx->prof.enabled, &launches, &ctx->prof);
+            r = lane->launch(ctx, slot, ctx->tile, !ctx->prof.enabled, stats != nullptr, &launches, &ctx->prof);
         }
         if (r != SGL_OK)
             return r;
@@ -445,7 +445,7 @@ SGL_API sgl_status sgl_render_debug(sgl_ctx *c, int scene_id, const sgl_view *vi
     int slot = 0, launches = 0;
     r = lane->prepare(ctx, &e, 1, ctx->tile, ctx->inline_span, (uint8_t *)ctx->debug_flags.ptr, &slot);
     if (r == SGL_OK)
-        r = lane->launch(ctx, slot, ctx->tile, false, &launches, nullptr);
+        r = lane->launch(ctx, slot, ctx->tile, false, true, &launches, nullptr);
     if (r != SGL_OK)
         return r;
     const sgl_target &t = *target;
@@ -503,14 +503,14 @@ static sgl_status batch_entries(Ctx *ctx, const sgl_batch_item *items, int n, st
 }
 
 // Batch items with their own pose: the node matrices composed on the host (as
-// sgl_scene_set_nodes does), then k_pose writes the item's world positions and
-// normals (and k_box its primitives' boxes) into the lane's pose scratch on
-// the lane's stream, and the item's entry points at them (the scene's own arrays and nodes are untouched).
+// sgl_scene_set_nodes does), then k_pose writes the items' world positions and
+// normals (and k_pose_box their primitives' boxes) into the lane's pose scratch
+// on the lane's stream, and the items' entries point at them (the scene's own
+// arrays and nodes are untouched).
 static sgl_status pose_items(Ctx *ctx, Lane *lane, const sgl_batch_item *items, int n, std::vector<BatchEntry> &e)
 {
     std::vector<std::vector<float>> mats((size_t)n);
-    size_t total = 0;
-    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    std::vector<PosedView> posed;
     for (int i = 0; i < n; i++) {
         if (!items[i].nodes)
             continue;
@@ -528,40 +528,15 @@ static sgl_status pose_items(Ctx *ctx, Lane *lane, const sgl_batch_item *items, 
         }
         mats[i] = std::move(world);
         mats[i].insert(mats[i].end(), rs.begin(), rs.end());
-        total += up(sizeof(float) * mats[i].size()) + up(2 * sizeof(float4) * std::max<size_t>(s->n_vertices, 1)) +
-                 (s->dev.pbox ? up(2 * sizeof(float4) * s->dev.n_prims) : 0);
+        posed.push_back(PosedView{&mats[i], &e[i]});
     }
-    if (!total)
+    if (posed.empty())
         return SGL_OK;
-    CUDA_TRY(lane->poses.ensure(total));
-    uint8_t *base = (uint8_t *)lane->poses.ptr;
-    size_t off = 0;
-    for (int i = 0; i < n; i++) {
-        if (!items[i].nodes)
-            continue;
-        const Scene *s = e[i].scene;
-        float *m = (float *)(base + off);
-        off += up(sizeof(float) * mats[i].size());
-        float4 *wpos = (float4 *)(base + off);
-        float4 *wnrm = wpos + s->n_vertices;
-        off += up(2 * sizeof(float4) * std::max<size_t>(s->n_vertices, 1));
-        float4 *pbox = nullptr;
-        if (s->dev.pbox) {
-            pbox = (float4 *)(base + off);
-            off += up(2 * sizeof(float4) * s->dev.n_prims);
-        }
-        const size_t nm = mats[i].size() / 2;
-        // (from pageable memory: staged before the call returns)
-        CUDA_TRY(cudaMemcpyAsync(m, mats[i].data(), sizeof(float) * mats[i].size(), cudaMemcpyHostToDevice,
-                                 lane->stream));
-        CUDA_TRY(launch_pose(s->dev, m, m + nm, wpos, wnrm, pbox, lane->stream));
-        e[i].wpos = wpos;
-        e[i].wnrm = wnrm;
-        e[i].pbox = pbox;
-        e[i].node_world = m;
-        e[i].node_rs = m + nm;
-    }
-    return SGL_OK;
+    Lane::Slot &sl = lane->slots[lane->next]; // (the batch takes this slot next)
+    CUDA_TRY(cudaEventSynchronize(sl.posed)); // its staging is free again
+    const sgl_status r = pose_views(ctx, lane->poses, sl.h_pose, posed, lane->stream);
+    CUDA_TRY(cudaEventRecord(sl.posed, lane->stream));
+    return r;
 }
 
 SGL_API sgl_status sgl_render_batch(sgl_ctx *c, const sgl_batch_item *items, int n_items,
@@ -600,7 +575,7 @@ SGL_API sgl_status sgl_render_batch(sgl_ctx *c, const sgl_batch_item *items, int
     if (!e.empty()) {
         r = lane->prepare(ctx, e.data(), (int)e.size(), tile, bin, nullptr, &slot);
         if (r == SGL_OK)
-            r = lane->launch(ctx, slot, tile, graph, &launches, graph ? nullptr : &ctx->prof);
+            r = lane->launch(ctx, slot, tile, graph, stats != nullptr, &launches, graph ? nullptr : &ctx->prof);
         if (r != SGL_OK)
             return r;
         if (stats) {
@@ -663,7 +638,7 @@ SGL_API sgl_status sgl_autotune(sgl_ctx *c, const sgl_batch_item *items, int n_i
                 if (r != SGL_OK)
                     break;
                 cudaEventRecord(a, lane->stream);
-                r = lane->launch(ctx, slot, tiles[ti], true, nullptr, nullptr);
+                r = lane->launch(ctx, slot, tiles[ti], true, false, nullptr, nullptr);
                 cudaEventRecord(b, lane->stream);
                 if (cudaEventSynchronize(b) != cudaSuccess) {
                     r = SGL_ERR_CUDA;
@@ -745,14 +720,19 @@ SGL_API sgl_status sgl_dof(sgl_ctx *c, const sgl_view *view, const sgl_target *i
     it.dof_halo = dof_halo_of(v.dof.max_radius);
     it.dof_tiles_x = (v.w + kDofTile - 1) / kDofTile;
     const uint32_t dof_tiles = (uint32_t)it.dof_tiles_x * (uint32_t)((v.h + kDofTile - 1) / kDofTile);
-    const size_t counters_at = (sizeof(ItemDev) + sizeof(BatchDev) + 4 * sizeof(uint32_t) + 15) & ~(size_t)15;
-    CUDA_TRY(ctx->dof_desc.ensure(counters_at + sizeof(unsigned long long) * kCounterWords));
-    uint8_t *dd = (uint8_t *)ctx->dof_desc.ptr;
-    ItemDev *d_it = (ItemDev *)dd;
-    BatchDev *d_b = (BatchDev *)(dd + sizeof(ItemDev));
-    uint32_t *d_base = (uint32_t *)(dd + sizeof(ItemDev) + sizeof(BatchDev));
+    // the item, the batch, the prefixes and the (zero) counters in one
+    // page-locked block and one copy (the call waits before it returns, so the
+    // block is free again)
+    const size_t b_at = sizeof(ItemDev), base_at = b_at + sizeof(BatchDev),
+                 counters_at = (base_at + 4 * sizeof(uint32_t) + 15) & ~(size_t)15,
+                 desc_bytes = counters_at + sizeof(unsigned long long) * kCounterWords;
+    CUDA_TRY(ctx->dof_desc.ensure(desc_bytes));
+    CUDA_TRY(ctx->dof_host.ensure(desc_bytes));
+    uint8_t *dd = (uint8_t *)ctx->dof_desc.ptr, *hd = (uint8_t *)ctx->dof_host.ptr;
+    const BatchDev *d_b = (const BatchDev *)(dd + b_at);
+    const uint32_t *d_base = (const uint32_t *)(dd + base_at);
     BatchDev b{};
-    b.items = d_it;
+    b.items = (const ItemDev *)dd;
     b.counters = (unsigned long long *)(dd + counters_at); // the gather's tile counter
     b.px_base = d_base;
     b.dof_base = d_base + 2;
@@ -760,16 +740,17 @@ SGL_API sgl_status sgl_dof(sgl_ctx *c, const sgl_view *view, const sgl_target *i
     b.total_px = (uint32_t)px;
     b.total_dof_tiles = dof_tiles;
     const uint32_t base[4] = {0u, (uint32_t)px, 0u, dof_tiles};
-    CUDA_TRY(cudaMemcpyAsync(d_it, &it, sizeof it, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(d_b, &b, sizeof b, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(d_base, base, sizeof base, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemsetAsync(b.counters, 0, sizeof(unsigned long long) * kCounterWords, st));
+    memset(hd, 0, desc_bytes);
+    memcpy(hd, &it, sizeof it);
+    memcpy(hd + b_at, &b, sizeof b);
+    memcpy(hd + base_at, base, sizeof base);
+    CUDA_TRY(cudaMemcpyAsync(dd, hd, desc_bytes, cudaMemcpyHostToDevice, st));
     CUDA_TRY(launch_dof(d_b, st));
     if (!device_buffers) {
         CUDA_TRY(cudaMemcpy2DAsync((uint8_t *)out->pixels + (size_t)v.y * out->pitch + 4 * (size_t)v.x, out->pitch,
                                    dst, 4 * (size_t)v.w, 4 * (size_t)v.w, v.h, cudaMemcpyDeviceToHost, st));
     }
-    CUDA_TRY(cudaStreamSynchronize(st)); // the descriptors above live on this call's stack
+    CUDA_TRY(cudaStreamSynchronize(st)); // (and the descriptors' block is free again)
     return SGL_OK;
 }
 

@@ -298,12 +298,21 @@ void prof_flush(Profiler *p);
 
 // kernel launchers (raster.cu)
 cudaError_t launch_world(const SceneDev &s, cudaStream_t st);
-// The world positions and normals of a scene under other node matrices
-// (`node_world`, `node_rs`, device) into `wpos` / `wnrm` (a posed request),
-// and the boxes of its primitives into `pbox` (2 float4 per primitive, may
-// be null); the scene's own arrays are not touched.
-cudaError_t launch_pose(const SceneDev &s, const float *node_world, const float *node_rs, float4 *wpos, float4 *wnrm,
-                        float4 *pbox, cudaStream_t st);
+// One posed view: the scene's arrays, the pose's node matrices (device) and
+// where its own world positions, normals and primitive boxes go (`pbox` may be
+// null); the scene's own arrays are not touched.
+struct PoseDev {
+    const float4 *pos_u, *nrm_v;
+    const uint32_t *vnode;
+    const uint4 *pgeo;
+    const float *node_world, *node_rs;
+    float4 *wpos, *wnrm, *pbox;
+    uint32_t n_vertices, n_prims;
+    uint32_t vertex_block, prim_block; // blocks of the two kernels before this pose's
+};
+constexpr uint32_t kPoseVertices = 1024, kPosePrims = 8; // per block
+// `poses` (device) of `n` views, covering vertex_blocks and prim_blocks blocks.
+cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, uint32_t prim_blocks, cudaStream_t st);
 // The launch sequence of a batch whose BatchDev lives at `b` (device memory).
 // `flags`: kSeqDof adds the depth-of-field gather, kSeqShaders shades with
 // every pixel shader (a view asks for another than the default).  The depth

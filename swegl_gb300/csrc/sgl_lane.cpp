@@ -47,6 +47,21 @@ size_t view_scratch_bytes(uint32_t n_vertices, uint32_t n_triangles, int w, int 
            + 8 * px;                                                                               // dof colour, depth
 }
 
+// Offsets of a slot's staging block for a batch of n items (Lane::Slot).
+struct StageLayout {
+    size_t counters, item_counters, items, bases, bytes;
+};
+static StageLayout stage_layout(int n)
+{
+    StageLayout l;
+    l.counters = align_up(sizeof(BatchDev), 256);
+    l.item_counters = l.counters + align_up(sizeof(unsigned long long) * kCounterWords, 256);
+    l.items = l.item_counters + align_up(2 * sizeof(unsigned long long) * (size_t)n, 256);
+    l.bases = l.items + align_up(sizeof(ItemDev) * (size_t)n, 256);
+    l.bytes = l.bases + sizeof(uint32_t) * Lane::kBaseArrays * ((size_t)n + 1);
+    return l;
+}
+
 Lane::~Lane()
 {
     for (auto &sl : slots) {
@@ -54,10 +69,10 @@ Lane::~Lane()
             for (auto &g : gt)
                 if (g)
                     cudaGraphExecDestroy(g);
-        if (sl.staged)
-            cudaEventDestroy(sl.staged);
         if (sl.done)
             cudaEventDestroy(sl.done);
+        if (sl.posed)
+            cudaEventDestroy(sl.posed);
     }
     if (own_stream && stream)
         cudaStreamDestroy(stream);
@@ -77,17 +92,11 @@ sgl_status Lane::init(Ctx *ctx, int max_items_, cudaStream_t external, bool bloc
         own_stream = true;
     }
     for (auto &sl : slots) {
-        CUDA_TRY(sl.d_items.ensure(sizeof(ItemDev) * (size_t)max_items));
-        CUDA_TRY(sl.d_bases.ensure(sizeof(uint32_t) * kBaseArrays * ((size_t)max_items + 1)));
-        CUDA_TRY(sl.d_batch.ensure(sizeof(BatchDev)));
-        CUDA_TRY(sl.d_counters.ensure(sizeof(unsigned long long) * kCounterWords));
-        CUDA_TRY(sl.d_item_counters.ensure(2 * sizeof(unsigned long long) * (size_t)max_items));
-        CUDA_TRY(sl.h_items.ensure(sizeof(ItemDev) * (size_t)max_items));
-        CUDA_TRY(sl.h_bases.ensure(sizeof(uint32_t) * kBaseArrays * ((size_t)max_items + 1)));
-        CUDA_TRY(sl.h_batch.ensure(sizeof(BatchDev)));
+        CUDA_TRY(sl.d_stage.ensure(stage_layout(max_items).bytes));
+        CUDA_TRY(sl.h_stage.ensure(stage_layout(max_items).bytes));
         CUDA_TRY(sl.h_counters.ensure(sizeof(unsigned long long) * (kCounterWords + 2 * (size_t)max_items)));
-        CUDA_TRY(cudaEventCreateWithFlags(&sl.staged, cudaEventDisableTiming));
         CUDA_TRY(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
+        CUDA_TRY(cudaEventCreateWithFlags(&sl.posed, cudaEventDisableTiming));
     }
     return SGL_OK;
 }
@@ -105,7 +114,9 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     if (sl.used)
         CUDA_TRY(cudaEventSynchronize(sl.done)); // its staging buffers are free again
     // prefixes and pool offsets
-    uint32_t *hb = (uint32_t *)sl.h_bases.ptr;
+    const StageLayout at = stage_layout(n);
+    uint8_t *hs = (uint8_t *)sl.h_stage.ptr, *ds = (uint8_t *)sl.d_stage.ptr;
+    uint32_t *hb = (uint32_t *)(hs + at.bases);
     uint32_t *vb = hb, *tb = hb + (n + 1), *pb = hb + 2 * (n + 1), *gb = hb + 3 * (n + 1), *fb = hb + 4 * (n + 1);
     uint32_t *gvb = hb + 5 * (n + 1), *gtb = hb + 6 * (n + 1);
     uint32_t *gcb = hb + 7 * (n + 1), *gib = hb + 8 * (n + 1), *gi = hb + 9 * (n + 1);
@@ -233,7 +244,7 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         frag_cap = std::min<size_t>(frags.bytes / sizeof(Frag), 0xFFFFFFFFu);
         seq_flags |= kSeqLayers;
     }
-    ItemDev *hi = (ItemDev *)sl.h_items.ptr;
+    ItemDev *hi = (ItemDev *)(hs + at.items);
     for (int i = 0; i < n; i++) {
         const BatchEntry &en = e[i];
         ItemDev it{};
@@ -292,10 +303,9 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         }
         hi[i] = it;
     }
-    BatchDev *hbd = (BatchDev *)sl.h_batch.ptr;
     BatchDev bd{};
-    bd.items = (const ItemDev *)sl.d_items.ptr;
-    const uint32_t *db = (const uint32_t *)sl.d_bases.ptr;
+    bd.items = (const ItemDev *)(ds + at.items);
+    const uint32_t *db = (const uint32_t *)(ds + at.bases);
     bd.tri_base = db + (n + 1); // (db[0 .. n]: the vertex prefix, read by nothing on the device)
     bd.px_base = db + 2 * (n + 1);
     bd.tile_base = db + 3 * (n + 1);
@@ -326,18 +336,16 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     sl.keep_keys = bd.keep_keys != 0;
     bd.spans = spans.ptr;
     bd.span_cap = (uint32_t)std::min<size_t>(spans.bytes / kSpanBytes, 0xFFFFFFFFu);
-    bd.counters = (unsigned long long *)sl.d_counters.ptr;
-    bd.item_counters = (unsigned long long *)sl.d_item_counters.ptr;
+    bd.counters = (unsigned long long *)(ds + at.counters);
+    bd.item_counters = (unsigned long long *)(ds + at.item_counters);
     bd.slot_flags = slot_flags;
     bd.frags = (Frag *)frags.ptr;
     bd.frag_cap = (uint32_t)frag_cap;
-    *hbd = bd;
-    CUDA_TRY(cudaMemcpyAsync(sl.d_items.ptr, hi, sizeof(ItemDev) * n, cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(sl.d_bases.ptr, hb, sizeof(uint32_t) * kBaseArrays * (n + 1), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(sl.d_batch.ptr, hbd, sizeof(BatchDev), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemsetAsync(sl.d_counters.ptr, 0, sizeof(unsigned long long) * kCounterWords, stream));
-    CUDA_TRY(cudaMemsetAsync(sl.d_item_counters.ptr, 0, 2 * sizeof(unsigned long long) * n, stream));
-    CUDA_TRY(cudaEventRecord(sl.staged, stream));
+    memcpy(hs, &bd, sizeof bd);
+    memset(hs + at.counters, 0, at.items - at.counters);
+    // one copy: as three copies and two fills, the descriptors cost a 1080p
+    // frame 7 us on the stream and the gaps between them
+    CUDA_TRY(cudaMemcpyAsync(ds, hs, at.bytes, cudaMemcpyHostToDevice, stream));
     sl.used = true;
     sl.n_items = n;
     sl.seq_flags = seq_flags;
@@ -345,12 +353,63 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     return SGL_OK;
 }
 
+sgl_status pose_views(Ctx *ctx, DevBuf &dev, HostBuf &host, const std::vector<PosedView> &views, cudaStream_t st)
+{
+    if (views.empty())
+        return SGL_OK;
+    // the copied part: descriptors, then each view's matrices; then the arrays
+    const size_t n = views.size();
+    size_t copied = align_up(sizeof(PoseDev) * n, 256), total = 0;
+    for (const PosedView &v : views)
+        copied += align_up(sizeof(float) * v.mats->size(), 256);
+    total = copied;
+    for (const PosedView &v : views) {
+        const Scene &s = *v.entry->scene;
+        total += align_up(2 * sizeof(float4) * std::max<size_t>(s.n_vertices, 1), 256) +
+                 (s.dev.pbox ? align_up(2 * sizeof(float4) * s.dev.n_prims, 256) : 0);
+    }
+    CUDA_TRY(dev.ensure(total));
+    CUDA_TRY(host.ensure(copied));
+    uint8_t *d = (uint8_t *)dev.ptr, *h = (uint8_t *)host.ptr;
+    size_t at = align_up(sizeof(PoseDev) * n, 256), arrays = copied;
+    uint64_t vb = 0, pb = 0;
+    for (size_t i = 0; i < n; i++) {
+        BatchEntry &e = *views[i].entry;
+        const Scene &s = *e.scene;
+        const std::vector<float> &m = *views[i].mats;
+        memcpy(h + at, m.data(), sizeof(float) * m.size());
+        e.node_world = (const float *)(d + at);
+        e.node_rs = e.node_world + m.size() / 2;
+        at += align_up(sizeof(float) * m.size(), 256);
+        e.wpos = (float4 *)(d + arrays);
+        e.wnrm = e.wpos + s.n_vertices;
+        arrays += align_up(2 * sizeof(float4) * std::max<size_t>(s.n_vertices, 1), 256);
+        e.pbox = nullptr;
+        if (s.dev.pbox) {
+            e.pbox = (float4 *)(d + arrays);
+            arrays += align_up(2 * sizeof(float4) * s.dev.n_prims, 256);
+        }
+        const PoseDev p{s.dev.pos_u, s.dev.nrm_v, s.dev.vnode, s.dev.pgeo, e.node_world, e.node_rs, e.wpos, e.wnrm,
+                        e.pbox, s.n_vertices, s.dev.n_prims, (uint32_t)vb, (uint32_t)pb};
+        memcpy(h + sizeof(PoseDev) * i, &p, sizeof p);
+        vb += (s.n_vertices + kPoseVertices - 1) / kPoseVertices;
+        pb += e.pbox ? (s.dev.n_prims + kPosePrims - 1) / kPosePrims : 0;
+    }
+    if (vb >= (1ull << 31) || pb >= (1ull << 31)) {
+        ctx->fail("posed batch too large");
+        return SGL_ERR_UNSUPPORTED;
+    }
+    CUDA_TRY(cudaMemcpyAsync(d, h, copied, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(launch_poses((const PoseDev *)d, (int)n, (uint32_t)vb, (uint32_t)pb, st));
+    return SGL_OK;
+}
+
 static int tile_index(int tile) { return tile == 8 ? 0 : (tile == 32 ? 2 : 1); }
 
-sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, int *launches, Profiler *prof)
+sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, bool counted, int *launches, Profiler *prof)
 {
     Slot &sl = slots[si];
-    const BatchDev *db = (const BatchDev *)sl.d_batch.ptr;
+    const BatchDev *db = (const BatchDev *)sl.d_stage.ptr;
     keys_dirty = true; // until the sequence is enqueued: its shade kernel empties the keys
     if (use_graph) {
         cudaGraphExec_t &g = sl.graph[tile_index(tile)][sl.seq_flags];
@@ -378,11 +437,14 @@ sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, int *launche
         CUDA_TRY(launch_batch(db, tile, sl.seq_flags, stream, launches, prof));
     }
     keys_dirty = sl.keep_keys;
-    unsigned long long *hc = (unsigned long long *)sl.h_counters.ptr; // per-item counters only
-    CUDA_TRY(cudaMemcpyAsync(hc + kCounterWords, sl.d_item_counters.ptr,
-                             2 * sizeof(unsigned long long) * sl.n_items, cudaMemcpyDeviceToHost, stream));
-    if (sl.seq_flags & kSeqLayers) // and the fragment count of a layered view
-        CUDA_TRY(cudaMemcpyAsync(hc + C_FRAGS / 2, (unsigned long long *)sl.d_counters.ptr + C_FRAGS / 2,
+    unsigned long long *hc = (unsigned long long *)sl.h_counters.ptr;
+    const StageLayout at = stage_layout(sl.n_items);
+    const uint8_t *ds = (const uint8_t *)sl.d_stage.ptr;
+    if (counted) // the items' counters
+        CUDA_TRY(cudaMemcpyAsync(hc + kCounterWords, ds + at.item_counters,
+                                 2 * sizeof(unsigned long long) * sl.n_items, cudaMemcpyDeviceToHost, stream));
+    if (sl.seq_flags & kSeqLayers) // the fragment count of a layered view
+        CUDA_TRY(cudaMemcpyAsync(hc + C_FRAGS / 2, ds + at.counters + sizeof(unsigned long long) * (C_FRAGS / 2),
                                  sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaEventRecord(sl.done, stream));
     return SGL_OK;

@@ -87,6 +87,17 @@ struct BatchEntry {
 // for a cycle or a bad parent.
 bool node_matrices(const std::vector<sgl_node_desc> &nodes, std::vector<float> &world, std::vector<float> &rs);
 
+// A posed view: its node matrices on the host (world, then the normal matrices;
+// kept until pose_views returns) and the entry that gets its device arrays.
+struct PosedView {
+    const std::vector<float> *mats;
+    BatchEntry *entry;
+};
+// Poses views on `st`: their matrices and descriptors in one copy from `host`
+// (which must not be reused before that copy is done), then all of them in one
+// launch sequence, into `dev`.
+sgl_status pose_views(Ctx *ctx, DevBuf &dev, HostBuf &host, const std::vector<PosedView> &views, cudaStream_t st);
+
 // Scratch bytes a view needs beyond its output buffers: vertex NDC and flags,
 // per-pixel keys and winner records, and its share of the batch lists.
 size_t view_scratch_bytes(uint32_t n_vertices, uint32_t n_triangles, int w, int h);
@@ -103,10 +114,14 @@ struct Lane {
     cudaStream_t capture_stream = nullptr;
     bool own_stream = false;
     struct Slot {
-        DevBuf d_items, d_bases, d_batch, d_counters, d_item_counters;
-        HostBuf h_items, h_bases, h_batch, h_counters;
-        cudaEvent_t staged = nullptr; // staging copies of this slot done
-        cudaEvent_t done = nullptr;   // launch sequence of this slot done
+        // The batch's descriptors in one block, copied to the device at once:
+        // the BatchDev (whose address the graphs hold), the counters (copied
+        // as zeros), the items' counters (zeros), the items and the prefixes.
+        DevBuf d_stage;
+        HostBuf h_stage, h_counters;
+        HostBuf h_pose;              // the batch's posed items: descriptors and matrices
+        cudaEvent_t posed = nullptr; // ... copied
+        cudaEvent_t done = nullptr; // launch sequence of this slot done
         bool used = false;
         cudaGraphExec_t graph[3][kSeqVariants] = {}; // per tile 8/16/32 and sequence flags (kSeq*)
         int graph_kernels[3][kSeqVariants] = {};     // kernels in each graph
@@ -131,7 +146,8 @@ struct Lane {
     sgl_status prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inline_span, uint8_t *slot_flags,
                        int *slot_out);
     // Run the launch sequence of a prepared slot (directly, or as a CUDA graph).
-    sgl_status launch(Ctx *ctx, int slot, int tile, bool use_graph, int *launches, Profiler *prof);
+    // `counted`: read_counters will be called.
+    sgl_status launch(Ctx *ctx, int slot, int tile, bool use_graph, bool counted, int *launches, Profiler *prof);
     // Per-batch and per-item counters of a finished slot (synchronises the slot).
     sgl_status read_counters(Ctx *ctx, int slot, unsigned long long *drawn, unsigned long long *fragments,
                              std::vector<unsigned long long> *per_item);
@@ -149,6 +165,7 @@ struct Ctx {
     std::unique_ptr<Lane> lane;        // the plain renderer's lane (internal stream)
     std::unique_ptr<Lane> ext_lane;    // lane bound to caller streams
     DevBuf stage_pixels, stage_z, debug_flags, dof_stage, dof_desc;
+    HostBuf dof_host; // sgl_dof's descriptors, page-locked
     Profiler prof;
     int tile = 16;                     // shade tile of the plain renderer
     int inline_span = 16;              // long-span bin threshold of the plain renderer

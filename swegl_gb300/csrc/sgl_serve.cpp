@@ -50,6 +50,7 @@ struct Server {
         std::unique_ptr<Lane> lane;
         DevBuf frames; // framebuffers of the batch in flight: colour then depth per job
         DevBuf poses;  // posed requests: node matrices, world positions and normals per job
+        HostBuf h_pose; // ... their descriptors and matrices
         std::vector<Job> jobs;
         size_t bytes = 0;
         int slot = 0;
@@ -104,22 +105,10 @@ void Server::launch_batch_on(LaneState &ls, std::vector<Job> &&jobs)
         c->fail("serving: framebuffer allocation of %zu bytes failed", fb);
         st = SGL_ERR_OOM;
     }
-    // posed requests: their node matrices and world arrays, then k_pose
-    auto pose_span = [](const Job &j) {
-        return (sizeof(float) * j.pose.size() + 16 + 32 * (size_t)j.scene->n_vertices +
-                (j.scene->dev.pbox ? 32 * (size_t)j.scene->dev.n_prims : 0) + 255) & ~(size_t)255;
-    };
-    size_t pose_bytes = 0;
-    for (auto &j : jobs)
-        if (!j.pose.empty())
-            pose_bytes += pose_span(j);
-    if (st == SGL_OK && pose_bytes && ls.poses.ensure(pose_bytes) != cudaSuccess) {
-        c->fail("serving: pose scratch of %zu bytes failed", pose_bytes);
-        st = SGL_ERR_OOM;
-    }
     std::vector<BatchEntry> entries;
     entries.reserve(jobs.size());
-    size_t off = 0, pose_off = 0;
+    size_t off = 0;
+    std::vector<PosedView> posed;
     std::vector<std::pair<uint32_t *, float *>> bufs;
     for (auto &j : jobs) {
         const size_t px = (size_t)j.req.view.w * j.req.view.h;
@@ -132,34 +121,20 @@ void Server::launch_batch_on(LaneState &ls, std::vector<Job> &&jobs)
         entries.push_back(BatchEntry{j.scene, v, pix, v.w, z});
         entries.back().surface = pix; // a layered request's surface is its own framebuffer
         bufs.emplace_back(pix, z);
-        if (!j.pose.empty() && st == SGL_OK) {
-            uint8_t *base = (uint8_t *)ls.poses.ptr + pose_off;
-            float *mats = (float *)base;
-            const size_t nm = j.pose.size() / 2;
-            float4 *wpos = (float4 *)(base + ((sizeof(float) * j.pose.size() + 15) & ~(size_t)15));
-            float4 *wnrm = wpos + j.scene->n_vertices;
-            float4 *pbox = j.scene->dev.pbox ? wnrm + j.scene->n_vertices : nullptr; // (2 per primitive)
-            pose_off += pose_span(j);
-            if (cudaMemcpyAsync(mats, j.pose.data(), sizeof(float) * j.pose.size(), cudaMemcpyHostToDevice,
-                                ls.lane->stream) != cudaSuccess ||
-                launch_pose(j.scene->dev, mats, mats + nm, wpos, wnrm, pbox, ls.lane->stream) != cudaSuccess) {
-                c->fail("serving: pose of request %llu failed", (unsigned long long)j.ticket);
-                st = SGL_ERR_CUDA;
-            }
-            entries.back().wpos = wpos;
-            entries.back().wnrm = wnrm;
-            entries.back().pbox = pbox;
-            entries.back().node_world = mats;
-            entries.back().node_rs = mats + nm;
-        }
+        if (!j.pose.empty())
+            posed.push_back(PosedView{&j.pose, &entries.back()}); // (entries does not grow beyond its reserve)
     }
+    // posed requests: their node matrices and world arrays (the lane is idle,
+    // so its staging is free)
+    if (st == SGL_OK)
+        st = pose_views(c, ls.poses, ls.h_pose, posed, ls.lane->stream);
     ls.layered = jobs.size() == 1 && jobs[0].req.view.layers > 0;
     const double t0 = now_s();
     if (st == SGL_OK)
         st = ls.lane->prepare(c, entries.data(), (int)entries.size(), tile, span_bin, nullptr, &ls.slot);
     int kernels_launched = 0;
     if (st == SGL_OK)
-        st = ls.lane->launch(c, ls.slot, tile, !ls.layered, &kernels_launched, nullptr);
+        st = ls.lane->launch(c, ls.slot, tile, !ls.layered, true, &kernels_launched, nullptr);
     {
         std::lock_guard<std::mutex> g(mu);
         batches++;
