@@ -97,6 +97,8 @@ struct SceneDev {
     int n_mats;
     int n_texs;
     MatDesc default_mat;
+    uint32_t *alpha;         // per texture the AND of its texels, then the triangles whose material has an alpha
+                             // below 255 (k_texture_alpha, k_translucent: at upload)
 };
 
 struct ViewDev {
@@ -157,7 +159,7 @@ struct __align__(16) Frag {
     uint32_t z;   // depth bits
     uint32_t slot;
     uint32_t next; // the next fragment of the pixel; before linking, the view pixel (kFragEnd: a hole)
-    uint32_t pad;
+    uint32_t color; // shaded when it is linked (unless frags_on_demand)
 };
 static_assert(sizeof(Frag) == 32 && offsetof(Frag, next) == 24, "Frag layout");
 constexpr uint32_t kFragEnd = 0xFFFFFFFFu;
@@ -298,6 +300,8 @@ void prof_flush(Profiler *p);
 
 // kernel launchers (raster.cu)
 cudaError_t launch_world(const SceneDev &s, cudaStream_t st);
+// Fills SceneDev::alpha (n_texs + 1 words).
+cudaError_t launch_alpha(const SceneDev &s, cudaStream_t st);
 // One posed view: the scene's arrays, the pose's node matrices (device) and
 // where its own world positions, normals and primitive boxes go (`pbox` may be
 // null); the scene's own arrays are not touched.
@@ -328,8 +332,10 @@ cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, ui
 // then k_shade_wins, for a batch of one large view) instead of the tiled
 // k_shade; BatchDev::wins must then hold total_px entries.  kSeqOne: the
 // batch has one view (the walk deals its list entries strided over groups).
+// kSeqOrigin: a layered view at the surface's top left, whose flatten and copy
+// passes read and write the pixel that the resolve has in hand.
 constexpr int kSeqDof = 1, kSeqShaders = 2, kSeqLayers = 4, kSeqFused = 8, kSeqSplit = 16, kSeqWinList = 32,
-              kSeqOne = 64, kSeqVariants = 128;
+              kSeqOne = 64, kSeqOrigin = 128, kSeqVariants = 256;
 // A batch of one view of at least this many pixels shades through the winner
 // list: the tiled shade's per-tile key reads and barriers then cost more than
 // the list's second kernel and its round trip through L2.

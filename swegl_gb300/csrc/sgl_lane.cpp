@@ -242,7 +242,7 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         CUDA_TRY(layer0.ensure(4 * tp));
         CUDA_TRY(cudaMemsetAsync(frag_head.ptr, 0xFF, 4 * tp, stream)); // kFragEnd
         frag_cap = std::min<size_t>(frags.bytes / sizeof(Frag), 0xFFFFFFFFu);
-        seq_flags |= kSeqLayers;
+        seq_flags |= kSeqLayers | (e[0].view.x == 0 && e[0].view.y == 0 ? kSeqOrigin : 0);
     }
     ItemDev *hi = (ItemDev *)(hs + at.items);
     for (int i = 0; i < n; i++) {
