@@ -202,9 +202,8 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     off += up256(8 * px);
     const size_t o_prec = off;
     off += up256(16 * px);
-    const bool win_list = px >= kWinListMinPixels; // the shade goes through a winner list
     const size_t o_wins = off;
-    off += win_list ? up256(8 * px) : 0;
+    off += px >= kWinListCounted ? up256(8 * px) : 0;
     const size_t o_list = off;
     off += up256(8 * (nt ? nt : 1));
     const size_t o_recs = off;
@@ -222,13 +221,19 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
                   scene_id, need, kNoAllocScratchBytes);
         return SGL_ERR_BUDGET;
     }
+    // the shade goes through a winner list: of a smaller view where it leaves
+    // the span bins their usual size
+    const size_t spare = kNoAllocScratchBytes - o_spans, list_bytes = up256(8 * px);
+    const bool win_list = px >= kWinListCounted || spare >= list_bytes + std::max<size_t>(min_spans, px / 8) * kSpanBytes;
+    const size_t span_bytes = spare - (win_list && px < kWinListCounted ? list_bytes : 0);
+    const size_t o_small_wins = o_spans + (span_bytes & ~(size_t)255); // after the spans
     unsigned char *base = nullptr;
     cudaError_t e = noalloc_scratch(&base);
     if (e != cudaSuccess) {
         ctx->fail("sgl_render_noalloc: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
         return SGL_ERR_CUDA;
     }
-    const uint32_t span_cap = (uint32_t)((kNoAllocScratchBytes - o_spans) / kSpanBytes);
+    const uint32_t span_cap = (uint32_t)((span_bytes & ~(size_t)255) / kSpanBytes);
     ItemDev it{};
     it.s = s->dev;
     it.v = make_view(v);
@@ -303,7 +308,7 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     b.tall = (uint32_t *)(base + o_tall);
     b.keep_keys = 0;
     b.key_pool = (unsigned long long *)(base + o_key);
-    b.wins = win_list ? (uint2 *)(base + o_wins) : nullptr;
+    b.wins = win_list ? (uint2 *)(base + (px >= kWinListCounted ? o_wins : o_small_wins)) : nullptr;
     b.spans = base + o_spans;
     b.span_cap = span_cap;
     b.counters = (unsigned long long *)(base + o_counters);

@@ -1397,18 +1397,18 @@ __device__ __forceinline__ void span_depth(const BatchDev *b, const WalkView &v,
     }
 }
 
-// A span's pixels by eight lanes, the `sub`-th of them pixels x1 + sub, + 8, ...:
+// A span's pixels by L lanes, the `sub`-th of them pixels x1 + sub, + L, ...:
 // each lane repeats the chain's additions up to its own pixels.  (Eight lanes
-// rather than 32: the additions a lane repeats are 8 per 8 pixels instead of
-// 32 per 32, so that four spans side by side take a third of the instructions
-// of one after another.)
+// where there are spans enough: the additions a lane repeats are 8 per 8 pixels
+// instead of 32 per 32, so that four spans side by side take a third of the
+// instructions of one after another.)
 constexpr int kSpanLanes = 8;
-template <class Op>
-__device__ __forceinline__ void span_by_eight(int x1, int x2, int sub, float top, float tstep, float bottom, float bstep,
-                                              Op &&op)
+template <int L, class Op>
+__device__ __forceinline__ void span_by(int x1, int x2, int sub, float top, float tstep, float bottom, float bstep,
+                                        Op &&op)
 {
 #pragma unroll
-    for (int bit = kSpanLanes / 2; bit; bit >>= 1)
+    for (int bit = L / 2; bit; bit >>= 1)
         if (sub & bit) {
 #pragma unroll
             for (int k = 0; k < bit; k++) {
@@ -1416,10 +1416,10 @@ __device__ __forceinline__ void span_by_eight(int x1, int x2, int sub, float top
                 bottom = bottom + bstep;
             }
         }
-    for (int x = x1 + sub; x < x2; x += kSpanLanes) {
+    for (int x = x1 + sub; x < x2; x += L) {
         op(x, top, bottom);
 #pragma unroll
-        for (int k = 0; k < kSpanLanes; k++) {
+        for (int k = 0; k < L; k++) {
             top = top + tstep;
             bottom = bottom + bstep;
         }
@@ -1452,7 +1452,7 @@ __device__ __forceinline__ void spans_depth_warp(const BatchDev *b, bool want, c
         unsigned long long *rs = reinterpret_cast<unsigned long long *>(
             __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(row), src));
         if (mine)
-            span_by_eight(xa, xb, sub, top, tstep, bottom, bstep, [&](int x, float t, float bt) {
+            span_by<kSpanLanes>(xa, xb, sub, top, tstep, bottom, bstep, [&](int x, float t, float bt) {
                 pixel_depth(b, si, rs, x, ys, sl, t, bt, v0, dv);
             });
 #pragma unroll
@@ -1660,23 +1660,45 @@ __device__ __forceinline__ void step3(float &x, float &t, float &b, float dx, fl
             }
         }
 }
-// A tall triangle (set-up in column 0 of S), walked by the whole warp 32 rows
-// at a time: each lane takes its own row's steps from the state of the first
-// of the 32, and lane 31's state after one more step is the next 32 rows'.
-// Every span is binned.  Returns this lane's fragments.
+// The same additions n times by every lane alike.
+__device__ __forceinline__ void advance3(float &x, float &t, float &b, float dx, float dt, float db, int n)
+{
+#pragma unroll 8
+    for (int k = 0; k < n; k++) {
+        x = x + dx;
+        t = t + dt;
+        b = b + db;
+    }
+}
+
+// A tall triangle (set-up in column 0 of S), walked by `share` warps, this one
+// the `sub`-th: each takes 32 rows in share * 32, its lanes a row each, from
+// the state of the first of the 32, to which the warp repeats the additions
+// from its last.  Every span is binned.  Returns this lane's fragments.
 template <bool FRAGS>
-__device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, const WalkRow *S)
+__device__ __forceinline__ unsigned long long walk_tall(const BatchDev *b, const WalkRow *S, int sub, int share)
 {
     const int lane = threadIdx.x & 31;
     const int n_u = (int)S[F_NU][0], n = n_u + (int)S[F_ND][0];
     const uint32_t slot = S[F_SLOT][0], item = S[F_ITEM][0];
-    uint32_t frags = 0;
+    unsigned long long frags = 0;
     WalkView v;
     v.load(b->items[item]);
     float lx = smf(S, F_LX, 0), lt = smf(S, F_LT, 0), lb = smf(S, F_LB, 0);
-    int sf = n_u > 0 ? F_UX : F_DX; // the short edge in hand
+    // the short edge in hand (the upper one until row n_u) and the row of its state
+    bool upper = n_u > 0;
+    int sf = upper ? F_UX : F_DX, at = 0;
     float sx = smf(S, sf, 0), st = smf(S, sf + 1, 0), sb = smf(S, sf + 2, 0);
-    for (int r0 = 0; r0 < n; r0 += 32) {
+    for (int r0 = 32 * sub; r0 < n; r0 += 32 * share) {
+        advance3(lx, lt, lb, smf(S, F_LR, 0), smf(S, F_LTS, 0), smf(S, F_LBS, 0), r0 - at);
+        if (upper && r0 >= n_u) { // on to the lower edge, from its first row
+            upper = false;
+            sf = F_DX;
+            sx = smf(S, sf, 0), st = smf(S, sf + 1, 0), sb = smf(S, sf + 2, 0);
+            at = n_u;
+        }
+        advance3(sx, st, sb, smf(S, sf + 3, 0), smf(S, sf + 4, 0), smf(S, sf + 5, 0), r0 - at);
+        at = r0;
         const int k = r0 + lane;
         const bool act = k < n;
         RowIn r;
@@ -1685,30 +1707,14 @@ __device__ __forceinline__ uint32_t walk_tall(const BatchDev *b, const WalkRow *
         step3(r.lx, r.lt, r.lb, r.lr, r.lts, r.lbs, lane);
         // rows of the half in hand continue its chain; a row beyond it starts
         // on the lower short edge (smem_row_in's state)
-        const bool cont = (k < n_u) == (sf == F_UX);
+        const bool cont = (k < n_u) == upper;
         if (cont) {
             r.sx = sx; r.st = st; r.sb = sb;
         }
         step3(r.sx, r.st, r.sb, r.sr, r.sts, r.sbs, cont ? lane : k - n_u);
         r.ls = 0;
         r.ss = 0;
-        // the state of row r0 + 32, if lane 31 has a row
-        if (r0 + 32 < n) {
-            lx = __shfl_sync(0xFFFFFFFFu, r.lx + r.lr, 31);
-            lt = __shfl_sync(0xFFFFFFFFu, r.lt + r.lts, 31);
-            lb = __shfl_sync(0xFFFFFFFFu, r.lb + r.lbs, 31);
-            const int half = r0 + 31 < n_u ? F_UX : F_DX; // lane 31's half
-            sx = __shfl_sync(0xFFFFFFFFu, r.sx + r.sr, 31);
-            st = __shfl_sync(0xFFFFFFFFu, r.st + r.sts, 31);
-            sb = __shfl_sync(0xFFFFFFFFu, r.sb + r.sbs, 31);
-            sf = r0 + 32 < n_u ? F_UX : F_DX;
-            if (sf != half) { // row r0 + 32 is the first of the lower half
-                sx = smf(S, F_DX, 0);
-                st = smf(S, F_DT, 0);
-                sb = smf(S, F_DB, 0);
-            }
-        }
-        frags += (uint32_t)walk_row<FRAGS>(b, v, kSpanLanes, item, slot, r, act, true);
+        frags += (unsigned long long)walk_row<FRAGS>(b, v, kSpanLanes, item, slot, r, act, true);
     }
     return frags;
 }
@@ -2067,8 +2073,10 @@ __device__ __noinline__ void walk_clip_depth(const BatchDev *b)
     }
 }
 
-// Set-up and depth walk (or fragment capture) of the tall triangles, one warp
-// each (warp-strided).
+// Set-up and depth walk (or fragment capture) of the tall triangles, a warp
+// each, or several where there are warps to spare: one triangle of 300 rows
+// was ten turns of one warp, most of a small frame's walk (640 x 480 cube: 14.5 ->
+// 7.4 us).
 template <bool FRAGS>
 __device__ __noinline__ void walk_tall_all(const BatchDev *b, WalkRow *S)
 {
@@ -2076,8 +2084,9 @@ __device__ __noinline__ void walk_tall_all(const BatchDev *b, WalkRow *S)
     const uint32_t nt = nt_raw < b->list_cap ? nt_raw : b->list_cap;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = gw; k < nt; k += n_warps) {
-        const uint32_t r = b->tall[k];
+    const uint32_t share = nt && nt < n_warps ? n_warps / nt : 1u;
+    for (uint32_t k = gw; k < nt * share; k += n_warps) {
+        const uint32_t r = b->tall[k % nt], sub = k / nt;
         const uint32_t item = (uint32_t)find_item(b->tri_base, b->n_items, r), t = r - __ldg(b->tri_base + item);
         const ItemDev &it = b->items[item];
         const uint4 tri = it.s.tris[t];
@@ -2085,9 +2094,9 @@ __device__ __noinline__ void walk_tall_all(const BatchDev *b, WalkRow *S)
         // (every lane writes the same values)
         tri_setup(b, it.v, item, t, tri, it.ndc[tri.x], it.ndc[tri.y], it.ndc[tri.z], kRecTall, S, 0);
         __syncwarp();
-        if (in_bounds(r < b->list_cap, CHK_REC, r))
+        if (sub == 0 && in_bounds(r < b->list_cap, CHK_REC, r))
             reinterpret_cast<uint32_t *>(b->recs + r)[lane] = S[lane][0];
-        item_add(b, 1, item, walk_tall<FRAGS>(b, S), true);
+        item_add(b, 1, item, walk_tall<FRAGS>(b, S, (int)sub, (int)share), true);
     }
 }
 
@@ -2146,16 +2155,13 @@ __global__ void __launch_bounds__(256, 4) k_winners(const BatchDev *b) { winner_
 
 // ------------------------------------------------------------- long spans --
 
-// Binned spans, eight lanes each (span_by_eight).  WINNER: the fragments of
-// the recorded ones whose key won record their progress values; else the keys
-// are folded.
-template <bool WINNER> __device__ __forceinline__ void spans_pass(const BatchDev *b)
+// Binned spans, L lanes each (span_by).  WINNER: the fragments of the recorded
+// ones whose key won record their progress values; else the keys are folded.
+template <bool WINNER, int L> __device__ __forceinline__ void spans_pass_by(const BatchDev *b, uint32_t n)
 {
-    const uint32_t n_raw = *counter32(b, C_SPANS);
-    const uint32_t n = n_raw < b->span_cap ? n_raw : b->span_cap;
-    const uint32_t step = gridDim.x * blockDim.x / kSpanLanes;
-    const int sub = (int)threadIdx.x & (kSpanLanes - 1);
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kSpanLanes; i < n; i += step) {
+    const uint32_t step = gridDim.x * blockDim.x / L;
+    const int sub = (int)threadIdx.x & (L - 1);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / L; i < n; i += step) {
         const uint32_t flagged = load_span_item(b, i);
         if (WINNER && !(flagged & kSpanRecorded))
             continue;
@@ -2169,12 +2175,12 @@ template <bool WINNER> __device__ __forceinline__ void spans_pass(const BatchDev
         // WINNER: the keys of a lane's next four pixels are in flight at once
         unsigned long long keys[4] = {};
         int j = 0;
-        span_by_eight((int)r.at.z, x2, sub, r.q.x, r.q.y, r.q.z, r.q.w, [&](int x, float top, float bottom) {
+        span_by<L>((int)r.at.z, x2, sub, r.q.x, r.q.y, r.q.z, r.q.w, [&](int x, float top, float bottom) {
             if (WINNER) {
                 if ((j & 3) == 0) {
 #pragma unroll
                     for (int k = 0; k < 4; k++)
-                        keys[k] = x + kSpanLanes * k < x2 ? row[x + kSpanLanes * k] : 0ull;
+                        keys[k] = x + L * k < x2 ? row[x + L * k] : 0ull;
                 } else {
                     keys[0] = keys[1];
                     keys[1] = keys[2];
@@ -2196,6 +2202,19 @@ template <bool WINNER> __device__ __forceinline__ void spans_pass(const BatchDev
                 prec[x] = make_float4(alpha, r.e.z, r.e.w, __uint_as_float(r.at.y & ~kYMask));
         });
     }
+}
+
+// A span takes a warp while there are warps for all of them: its pixels are
+// then the longest chain left (640 x 480 cube: spans 4.4 -> 3.2 us, their records
+// 2 us less).
+template <bool WINNER> __device__ __forceinline__ void spans_pass(const BatchDev *b)
+{
+    const uint32_t n_raw = *counter32(b, C_SPANS);
+    const uint32_t n = n_raw < b->span_cap ? n_raw : b->span_cap;
+    if (32ull * n <= (unsigned long long)gridDim.x * blockDim.x)
+        spans_pass_by<WINNER, 32>(b, n);
+    else
+        spans_pass_by<WINNER, kSpanLanes>(b, n);
 }
 
 __global__ void __launch_bounds__(256) k_spans(const BatchDev *b) { spans_pass<false>(b); }
@@ -2464,7 +2483,7 @@ __global__ void __launch_bounds__(kShadeThreads, SGL_TILE_MIN_BLOCKS) k_shade(co
     }
 }
 
-// The same per-pixel work for a batch of one large view (kSeqWinList), in
+// The same per-pixel work for a batch of one view (kSeqWinList), in
 // two passes.  k_classify streams the view's depth keys, four consecutive
 // pixels a thread: background colour and every pixel's depth are written at
 // once, and the winners appended to the winner list in pixel order, with one
@@ -3148,7 +3167,7 @@ __global__ void __launch_bounds__(256) k_frag_spans(const BatchDev *b)
         const int y = (int)(r.at.y & kYMask), x1 = (int)r.at.z;
         const uint32_t row_px = (uint32_t)((y - v.y) * v.w - v.x);
         const float fb = __uint_as_float(r.at.y & ~kYMask);
-        span_by_eight(x1, (int)r.at.w, sub, r.q.x, r.q.y, r.q.z, r.q.w, [&](int x, float top, float bottom) {
+        span_by<kSpanLanes>(x1, (int)r.at.w, sub, r.q.x, r.q.y, r.q.z, r.q.w, [&](int x, float top, float bottom) {
             const float alpha = top / bottom;
             const float z = r.e.x + r.e.y * alpha;
             const bool keep = !below_near(z) && __float_as_uint(z) < kMaxZBits;

@@ -336,10 +336,13 @@ cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, ui
 // passes read and write the pixel that the resolve has in hand.
 constexpr int kSeqDof = 1, kSeqShaders = 2, kSeqLayers = 4, kSeqFused = 8, kSeqSplit = 16, kSeqWinList = 32,
               kSeqOne = 64, kSeqOrigin = 128, kSeqVariants = 256;
-// A batch of one view of at least this many pixels shades through the winner
-// list: the tiled shade's per-tile key reads and barriers then cost more than
-// the list's second kernel and its round trip through L2.
-constexpr uint64_t kWinListMinPixels = 1u << 20;
+// A batch of one view shades through the winner list (8 B a pixel): the tiled
+// shade's per-tile key reads and barriers cost more than the list's second
+// kernel and its round trip through L2, at any size (winner records and shade,
+// tiled / list: 640 x 480 cube 16.8 / 13.9 us, 960 x 540 18.9 / 13.8, 1283 x
+// 719 flat 24.6 / 15.3).  Views below this many pixels do not count the list
+// in their scratch bytes: the allocation-free call uses it where it fits.
+constexpr uint64_t kWinListCounted = 1u << 20;
 cudaError_t launch_batch(const BatchDev *b, int tile, int flags, cudaStream_t st, int *launches, Profiler *prof);
 // The device-side bounds checks of the checked build (-DSGL_BOUNDS_CHECK):
 // the first failure's check code and index and the failure count, cleared

@@ -42,7 +42,7 @@ size_t view_scratch_bytes(uint32_t n_vertices, uint32_t n_triangles, int w, int 
 {
     const size_t px = (size_t)w * h;
     return align_up(16 * (size_t)n_vertices, 256) + align_up(n_vertices, 256) + 8 * px + 16 * px  // ndc yes key prec
-           + (px >= kWinListMinPixels ? 8 * px : 0)                                               // winner list
+           + (px >= kWinListCounted ? 8 * px : 0)                                               // winner list
            + (8 + sizeof(TriRec) + 8) * (size_t)n_triangles + kSpanBytes * (px / 8 + 64)      // lists, set-ups, bins
            + 8 * px;                                                                               // dof colour, depth
 }
@@ -211,8 +211,8 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         keys_dirty = false;
     }
     CUDA_TRY(prec.ensure(sizeof(float4) * std::max<uint64_t>(tp, 1)));
-    // one large view: the shade goes through a winner list
-    const bool win_list = n == 1 && tp >= kWinListMinPixels && e[0].view.layers == 0;
+    // one view: the shade goes through a winner list
+    const bool win_list = n == 1 && e[0].view.layers == 0;
     if (win_list)
         CUDA_TRY(wins.ensure(sizeof(uint2) * tp));
     CUDA_TRY(list.ensure(sizeof(uint2) * std::max<uint64_t>(tt, 1)));
