@@ -107,7 +107,7 @@ __global__ void k_world(SceneDev s)
     const float4 p = s.pos_u[g];
     const float4 q = s.nrm_v[g];
     const V3 w = transform3(mk3(p.x, p.y, p.z), M);
-    const V3 nw = normalize3(normalize3(rotate_n(mk3(q.x, q.y, q.z), RS)));
+    const V3 nw = normalize_fast<true>(normalize_fast<true>(rotate_n(mk3(q.x, q.y, q.z), RS)));
     s.wpos[g] = make_float4(w.x, w.y, w.z, p.w);
     s.wnrm[g] = make_float4(nw.x, nw.y, nw.z, q.w);
 }
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) k_pose(const PoseDev *poses, int n)
         if (g >= p.n_vertices)
             break;
         const V3 w = transform3(mk3(a[k].x, a[k].y, a[k].z), p.node_world + 16 * node[k]);
-        const V3 nw = normalize3(normalize3(rotate_n(mk3(q[k].x, q[k].y, q[k].z), p.node_rs + 16 * node[k])));
+        const V3 nw = normalize_fast<true>(normalize_fast<true>(rotate_n(mk3(q[k].x, q[k].y, q[k].z), p.node_rs + 16 * node[k])));
         p.wpos[g] = make_float4(w.x, w.y, w.z, a[k].w);
         p.wnrm[g] = make_float4(nw.x, nw.y, nw.z, q[k].w);
     }
@@ -1974,7 +1974,7 @@ __device__ __forceinline__ void load_tv(const ItemDev &it, uint32_t g, TV &o)
 __device__ __forceinline__ void world_to_viewport(const ViewDev &v, TV &o, const float *rs)
 {
     V3 p = transform3(o.world, v.view);
-    o.nworld = normalize3(normalize3(rotate_n(o.normal, rs)));
+    o.nworld = normalize_fast<true>(normalize_fast<true>(rotate_n(o.normal, rs)));
     p = transform3(p, v.proj);
     if (p.z != 0.0f) {
         p.x = p.x / fabsf(p.z);

@@ -121,7 +121,7 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
         float diffuse = pl.w / d2;
         if (diffuse < 0.05f) // (double)diffuse < 0.05, see sgl_device.cuh
             continue;
-        ld = normalize3(ld);
+        ld = normalize_fast(ld);
         const float alignment = -dot3(normal, ld);
         if (alignment < 0.0f)
             continue;
@@ -142,8 +142,8 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
 // pixel_shader_lights_phong::shade (src/render/pixel_shaders.cpp:159-205)
 __device__ __forceinline__ int sh_phong(const Shader &sh, const LightsDev &L, const ViewDev &v)
 {
-    const V3 normal = normalize3(sh.n);
-    const V3 camvec = normalize3(sub3(mk3(v.campos[0], v.campos[1], v.campos[2]), sh.center));
+    const V3 normal = normalize_fast(sh.n);
+    const V3 camvec = normalize_fast(sub3(mk3(v.campos[0], v.campos[1], v.campos[2]), sh.center));
     return f2i(65536.0f * light_sum(L, sh.center, normal, camvec, sh.shininess));
 }
 
