@@ -458,6 +458,41 @@ __device__ __forceinline__ bool tall_rows(float lo_y, float hi_y, int y, int y_e
     return z > a && z - a > kTallRows;
 }
 
+// A triangle of one row (its screen y range lo_y .. hi_y holds one whole
+// number) whose row's span holds no pixel: no whole number between the
+// crossings of the row with its two edges that span it, widened by `eps` to
+// both sides.  Each crossing here is within 2^-20 mx (mx the largest |x|, below
+// 2^20) of the exact one (differences, the hardware reciprocal, products and
+// the sum: 7 roundings of 2^-24 of at most 2 mx), the reference's x within
+// 18 * 2^-24 mx of it (its start has 6 roundings), and eps is at least 33 *
+// 2^-23 mx, nearly twice both.  Such triangles are two fifths of the walk list
+// of a batch of small views (2.8 M of 7.1 M of the 64 views of 200 spheres; a
+// fifth of the 1080p frame's) and cost the walk a set-up each: 64 views, walk 470
+// -> 347 us for 46 us more of geometry.  (k_compact does not ask: on terrains of
+// 512 x 512 cells at 256 x 256 to 1920 x 1080 it took 0.7 us and saved none.)
+__device__ __forceinline__ bool row_empty(float x0, float y0, float x1, float y1, float x2, float y2, float lo_y,
+                                          float hi_y, float mx, float eps)
+{
+    const float y = ceilf(lo_y);
+    if (!(y + 1.0f >= hi_y && mx < 0x1p20f && fabsf(y) < 0x1p20f))
+        return false;
+    float lo = INFINITY, hi = -INFINITY, sum = 0.0f;
+    auto edge = [&](float xa, float ya, float xb, float yb) {
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(yb - ya));
+        const float x = xa + (y - ya) * (xb - xa) * r;
+        if ((ya <= y) != (yb <= y)) {
+            lo = fminf(lo, x);
+            hi = fmaxf(hi, x);
+            sum = sum + x;
+        }
+    };
+    edge(x0, y0, x1, y1);
+    edge(x1, y1, x2, y2);
+    edge(x2, y2, x0, y0);
+    return fabsf(sum) < 0x1p22f && ceilf(lo - eps) >= hi + eps; // (the sum is NaN or infinite where a crossing is)
+}
+
 // Batch triangles r of the lanes that ask for it into the tall list, one
 // atomic per warp.  Every lane of the warp calls it.
 __device__ __forceinline__ void list_tall(const BatchDev *b, bool want, uint32_t r)
@@ -638,7 +673,7 @@ struct GeomShared {
     uint32_t clip[kGeomItems][kGeomWarps][kGeomTG]; // ... of the clip list
     uint32_t cnt[kGeomItems * kGeomWarps];          // entries: walk list | clip list << 16
     uint32_t off[kGeomItems * kGeomWarps];          // ... of the items and warps before
-    uint32_t nx[kGeomItems];                        // triangles that reach fill_triangle_2's set-up
+    uint32_t nx[kGeomItems * kGeomWarps];           // triangles that reach fill_triangle_2's set-up
     uint32_t base[2];                               // the block's first position in each list
 };
 static_assert(kFuseVerts <= 256, "local vertex indices are bytes");
@@ -723,8 +758,6 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                     S.ndc[warp] = it.ndc;
             }
         }
-        if (threadIdx.x < kGeomItems)
-            S.nx[threadIdx.x] = 0;
         const SceneDev &sc = b->items[__ldg(b->grp_items + i_lo)].s; // vertex data shared by the group
         const uint32_t q = chunk * kGeomWarps + warp;                  // this warp's primitive
         const bool has = q < sc.n_prims && (!sc.psmall || sc.psmall[q]); // (a mixed scene's larger ones: general passes)
@@ -749,7 +782,7 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
         wpos += gq.x;
         __syncthreads(); // the cameras are staged
         for (int vi = 0; vi < nv; vi++) {
-            uint32_t entries = 0;
+            uint32_t entries = 0, nx = 0;
             if (has && !((unseen >> vi) & 1u)) {
                 const float *vw = S.view[vi];
                 __syncwarp(); // the previous item's reads of pos are done
@@ -804,7 +837,6 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                     __syncwarp();
                     // the compaction's decisions, as k_compact
                     const float vm00 = vw[GV_VM00], vm03 = vw[GV_VM03], vm11 = vw[GV_VM11], vm13 = vw[GV_VM13];
-                    uint32_t nx = 0;
                     bool listed = false;
                     for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
                         const uint32_t t = t0 + lane;
@@ -835,8 +867,9 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                                             const float eps = (rows + 32.0f) * 0x1p-23f * (mx + 1.0f);
                                             const float lo_x = fminf(x0, fminf(x1, x2)) - eps;
                                             const float hi_x = fmaxf(x0, fmaxf(x1, x2)) + eps;
-                                            if (ceilf(lo_x) == ceilf(hi_x)) {
-                                                d = 3; // no pixel column
+                                            if (ceilf(lo_x) == ceilf(hi_x) ||
+                                                row_empty(x0, y0, x1, y1, x2, y2, lo_y, hi_y, mx, eps)) {
+                                                d = 3; // no pixel column, or no pixel in its row
                                                 if (b->slot_flags)
                                                     b->slot_flags[2 * (gq.z + t)] = 1;
                                             } else if (tall_rows(lo_y, hi_y, __float_as_int(vw[GV_Y]),
@@ -870,12 +903,12 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                             if (in_bounds(gq.x + i < sc.n_vertices, CHK_NDC, gq.x + i))
                                 ndc[i] = pos[i];
                     }
-                    if (lane == 0 && nx)
-                        atomicAdd(&S.nx[vi], nx);
                 }
             }
-            if (lane == 0)
+            if (lane == 0) {
                 S.cnt[vi * kGeomWarps + warp] = entries;
+                S.nx[vi * kGeomWarps + warp] = nx;
+            }
         }
         __syncthreads();
         if (warp == 0) {
@@ -896,32 +929,43 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                 S.base[0] = (uint32_t)old;
                 S.base[1] = (uint32_t)(old >> 32);
             }
-            if ((int)lane < nv && S.nx[lane])
-                atomicAdd(b->item_counters + 2 * (size_t)__float_as_uint(S.view[lane][GV_ITEM]),
-                          (unsigned long long)S.nx[lane]);
+            // the items' drawn triangles (a lane's two counts are one item's, four lanes' make it whole)
+            uint32_t x = k < nv * kGeomWarps ? S.nx[k] + S.nx[k + 1] : 0u;
+            x += __shfl_xor_sync(0xFFFFFFFFu, x, 1);
+            x += __shfl_xor_sync(0xFFFFFFFFu, x, 2);
+            if ((lane & 3) == 0 && x)
+                atomicAdd(b->item_counters + 2 * (size_t)__float_as_uint(S.view[lane >> 2][GV_ITEM]),
+                          (unsigned long long)x);
         }
         __syncthreads();
         if (has) {
+            const uint32_t list_cap = b->list_cap, base0 = S.base[0], base1 = S.base[1];
+            uint2 *list = b->list;
             for (int vi = 0; vi < nv; vi++) {
-                if (!S.cnt[vi * kGeomWarps + warp])
+                const uint32_t n = S.cnt[vi * kGeomWarps + warp];
+                if (!n)
                     continue;
                 const uint32_t off = S.off[vi * kGeomWarps + warp];
-                uint32_t o0 = S.base[0] + (off & 0xFFFFu), o1 = S.base[1] + (off >> 16);
                 const uint32_t item = __float_as_uint(S.view[vi][GV_ITEM]), tlo = __float_as_uint(S.view[vi][GV_TRI]);
+                uint32_t o0 = base0 + (off & 0xFFFFu);
                 for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
-                    const unsigned m1 = S.walk[vi][warp][t0 >> 5], m2 = S.clip[vi][warp][t0 >> 5];
-                    const uint32_t t = t0 + lane;
-                    if ((m1 >> lane) & 1u) {
-                        const uint32_t j = o0 + __popc(m1 & below);
-                        if (j < b->list_cap)
-                            b->list[j] = make_uint2(tlo + gq.z + t, item);
-                    } else if ((m2 >> lane) & 1u) {
+                    const unsigned m1 = S.walk[vi][warp][t0 >> 5];
+                    const uint32_t j = o0 + __popc(m1 & below);
+                    if (((m1 >> lane) & 1u) && j < list_cap)
+                        list[j] = make_uint2(tlo + gq.z + t0 + lane, item);
+                    o0 += __popc(m1);
+                }
+                if (!(n >> 16))
+                    continue;
+                uint32_t o1 = base1 + (off >> 16);
+                for (uint32_t t0 = 0; t0 < gq.w; t0 += 32) {
+                    const unsigned m2 = S.clip[vi][warp][t0 >> 5];
+                    if ((m2 >> lane) & 1u) {
                         const uint32_t j = o1 + __popc(m2 & below);
                         if (j < b->clip_cap)
-                            b->clip[b->clip_cap - 1 - j] = make_uint2(gq.z + t, item); // from the end
-                        mark_clip(b, tlo + gq.z + t);
+                            b->clip[b->clip_cap - 1 - j] = make_uint2(gq.z + t0 + lane, item); // from the end
+                        mark_clip(b, tlo + gq.z + t0 + lane);
                     }
-                    o0 += __popc(m1);
                     o1 += __popc(m2);
                 }
             }
