@@ -2321,17 +2321,21 @@ __device__ __forceinline__ uint32_t shade_clip_px(const ItemDev &it, uint32_t i,
     return shade_clip_rec(it, slot, it.prec[i]);
 }
 
-// A 32-byte quarter of a record, one load.
+// 32 bytes in one load: a quarter of a record, or a fragment.
 struct Quarter {
     uint32_t w[8];
 };
-__device__ __forceinline__ Quarter load_quarter(const TriRec *rp, int k)
+__device__ __forceinline__ Quarter load_quarter(const void *p)
 {
     Quarter q;
     asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=r"(q.w[0]), "=r"(q.w[1]), "=r"(q.w[2]), "=r"(q.w[3]), "=r"(q.w[4]), "=r"(q.w[5]), "=r"(q.w[6]), "=r"(q.w[7])
-        : "l"(reinterpret_cast<const char *>(rp) + 32 * k));
+        : "l"(p));
     return q;
+}
+__device__ __forceinline__ Quarter load_quarter(const TriRec *rp, int k)
+{
+    return load_quarter(reinterpret_cast<const char *>(rp) + 32 * k);
 }
 
 // The progress values of pixel (X, Y) (surface coordinates) from its winning
@@ -3263,13 +3267,16 @@ __global__ void __launch_bounds__(256, SGL_SHADE_MIN_BLOCKS) k_link(const BatchD
     uint32_t *head = it.frag_head;
     Frag *pool = b->frags;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint4 m = reinterpret_cast<const uint4 *>(pool + i)[1]; // z, slot, pixel
-        if (m.z == kFragEnd)
+        const Quarter f = load_quarter(pool + i);
+        const uint32_t px = f.w[6];
+        if (px == kFragEnd)
             continue;
-        const uint32_t next = atomicExch(head + m.z, i);
+        const uint32_t next = atomicExch(head + px, i);
         uint32_t c = 0u;
         if (!on_demand)
-            c = shade_frag<ALL_MODES>(b, it, 0u, m.y, reinterpret_cast<const float4 *>(pool + i)[0]);
+            c = shade_frag<ALL_MODES>(b, it, 0u, f.w[5],
+                                      make_float4(__uint_as_float(f.w[0]), __uint_as_float(f.w[1]),
+                                                  __uint_as_float(f.w[2]), __uint_as_float(f.w[3])));
         reinterpret_cast<uint2 *>(pool + i)[3] = make_uint2(next, c);
     }
 }
@@ -3294,28 +3301,34 @@ __device__ __forceinline__ void write_pixel(const ItemDev &it, uint32_t i, uint3
 
 // One pixel whose fragments are shaded: one run over its chain for the nearest
 // opaque (the first drawn of equal depth), one for the transparent ones in
-// front of it, kept nearest first (of equal depth the last drawn).
-template <bool ORIGIN> __device__ __forceinline__ void resolve_shaded(const BatchDev *b, const ItemDev &it, uint32_t i)
+// front of it, kept nearest first (of equal depth the last drawn).  `first`:
+// the second half of its head fragment (depth, slot, next, colour).
+template <bool ORIGIN>
+__device__ __forceinline__ void resolve_shaded(const BatchDev *b, const ItemDev &it, uint32_t i, uint4 first)
 {
     const Frag *pool = b->frags;
-    const uint32_t head = it.frag_head[i];
     unsigned long long opaque = ((unsigned long long)kMaxZBits << 32) | 0xFFFFFFFFull;
-    uint32_t wc = 0u;
-    int clear = 0; // transparent fragments
-    for (uint32_t f = head; f != kFragEnd;) {
-        const uint4 m = reinterpret_cast<const uint4 *>(pool + f)[1];
+    uint32_t wc = 0u, l0 = 0u, lone = 0u;
+    int clear = 0; // transparent fragments, the last one's depth and colour
+    for (uint4 m = first;;) {
         const unsigned long long key = ((unsigned long long)m.x << 32) | m.y;
         if ((m.w >> 24) != 255u) {
             clear++;
+            lone = m.x;
+            l0 = m.w;
         } else if (key < opaque) {
             opaque = key;
             wc = m.w;
         }
-        f = m.z;
+        if (m.z == kFragEnd)
+            break;
+        m = reinterpret_cast<const uint4 *>(pool + m.z)[1];
     }
     const uint32_t wz = (uint32_t)(opaque >> 32);
-    uint32_t l0 = 0u;
-    if (clear) {
+    if (clear == 1) { // most pixels: no order to find (30.7 -> 26.6 us)
+        l0 = lone < wz ? l0 : 0u;
+    } else if (clear) {
+        l0 = 0u;
         unsigned long long lk[SGL_MAX_LAYERS]; // kept, nearest first: depth, then the complement of the slot
         uint32_t lc[SGL_MAX_LAYERS];
 #pragma unroll
@@ -3324,8 +3337,7 @@ template <bool ORIGIN> __device__ __forceinline__ void resolve_shaded(const Batc
             lc[k] = 0u;
         }
         const int n_layers = it.layers;
-        for (uint32_t f = head; f != kFragEnd;) {
-            const uint4 m = reinterpret_cast<const uint4 *>(pool + f)[1];
+        for (uint4 m = first;;) {
             if ((m.w >> 24) != 255u && m.x < wz) {
                 unsigned long long key = ((unsigned long long)m.x << 32) | (uint32_t)~m.y;
                 uint32_t c = m.w;
@@ -3340,7 +3352,9 @@ template <bool ORIGIN> __device__ __forceinline__ void resolve_shaded(const Batc
                         c = tc;
                     }
             }
-            f = m.z;
+            if (m.z == kFragEnd)
+                break;
+            m = reinterpret_cast<const uint4 *>(pool + m.z)[1];
         }
         // the farthest kept is the first layer, the nearer ones blend onto it
         // (an unused place holds 0, which blends nothing)
@@ -3437,10 +3451,11 @@ __device__ __forceinline__ void resolve_on_demand(const BatchDev *b, const ItemD
             l0 = blend_px(l0, f);
     }
     write_pixel<ORIGIN>(it, i, wz, wc, l0);
+    it.frag_head[i] = kFragEnd;
 }
 
-// Per pixel of the layered view: pixels without fragments get the background
-// at once, the others are resolved, those with fragments to shade queued in
+// Per pixel of the layered view (list heads are left empty for the next):
+// pixels without fragments get the background at once, the others are resolved, those with fragments to shade queued in
 // shared memory for full warps.
 template <bool ALL_MODES, bool ORIGIN>
 __global__ void __launch_bounds__(256, 4) k_layers(const BatchDev *b)
@@ -3450,11 +3465,29 @@ __global__ void __launch_bounds__(256, 4) k_layers(const BatchDev *b)
     const ItemDev &it = b->items[0];
     const uint32_t total = (uint32_t)it.v.w * (uint32_t)it.v.h;
     if (!frags_on_demand(it.s)) {
-        for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
-            if (it.frag_head[i] == kFragEnd)
+        // (a pixel's list head is loaded two turns ahead and its first fragment
+        // one, so that a turn waits for neither: 26.6 -> 23.5 us; four consecutive
+        // pixels a thread, with 16-byte accesses, 41.6 us)
+        uint32_t *head = it.frag_head;
+        const uint32_t step = gridDim.x * 256u;
+        uint32_t i = blockIdx.x * 256u + threadIdx.x;
+        auto fragment = [&](uint32_t f) {
+            return f != kFragEnd ? reinterpret_cast<const uint4 *>(b->frags + f)[1] : make_uint4(0u, 0u, kFragEnd, 0u);
+        };
+        uint32_t h = i < total ? head[i] : kFragEnd, h1 = i + step < total ? head[i + step] : kFragEnd;
+        uint4 m = fragment(h);
+        for (; i < total; i += step) {
+            const uint4 m1 = fragment(h1);
+            const uint32_t h2 = i + 2 * step < total ? head[i + 2 * step] : kFragEnd;
+            if (h == kFragEnd) {
                 write_pixel<ORIGIN>(it, i, kMaxZBits, 0u, 0u);
-            else
-                resolve_shaded<ORIGIN>(b, it, i);
+            } else {
+                resolve_shaded<ORIGIN>(b, it, i, m);
+                head[i] = kFragEnd;
+            }
+            h = h1;
+            m = m1;
+            h1 = h2;
         }
         return;
     }

@@ -154,7 +154,7 @@ struct ItemDev {
 
 // One fragment of a view with transparency layers: its depth, draw slot and
 // the progress values that shade it, chained per pixel.
-struct __align__(16) Frag {
+struct __align__(32) Frag {
     float4 rec;   // progress, progL, progR, span bits (as in ItemDev::prec)
     uint32_t z;   // depth bits
     uint32_t slot;

@@ -204,8 +204,9 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     CUDA_TRY(ndc.ensure(sizeof(float4) * std::max<size_t>(ndc_off, 1)));
     CUDA_TRY(yes.ensure(std::max<size_t>(yes_off, 1)));
     const void *key_was = key.ptr;
+    const size_t key_bytes = key.bytes;
     CUDA_TRY(key.ensure(sizeof(unsigned long long) * std::max<uint64_t>(tp, 1)));
-    if (key.ptr != key_was || keys_dirty) {
+    if (key.ptr != key_was || key.bytes != key_bytes || keys_dirty) {
         // a new pool, or one a debug render or a failed launch left dirty
         CUDA_TRY(cudaMemsetAsync(key.ptr, 0xFF, key.bytes, stream)); // kEmptyKey is all ones
         keys_dirty = false;
@@ -238,9 +239,14 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         }
         frag_want = std::max<size_t>(frag_want, std::max<size_t>(4 * tp, 65536));
         CUDA_TRY(frags.ensure(sizeof(Frag) * frag_want));
+        const void *head_was = frag_head.ptr;
+        const size_t head_bytes = frag_head.bytes;
         CUDA_TRY(frag_head.ensure(4 * tp));
         CUDA_TRY(layer0.ensure(4 * tp));
-        CUDA_TRY(cudaMemsetAsync(frag_head.ptr, 0xFF, 4 * tp, stream)); // kFragEnd
+        if (frag_head.ptr != head_was || frag_head.bytes != head_bytes || heads_dirty) { // (the resolve leaves them empty)
+            CUDA_TRY(cudaMemsetAsync(frag_head.ptr, 0xFF, frag_head.bytes, stream)); // kFragEnd
+            heads_dirty = false;
+        }
         frag_cap = std::min<size_t>(frags.bytes / sizeof(Frag), 0xFFFFFFFFu);
         seq_flags |= kSeqLayers | (e[0].view.x == 0 && e[0].view.y == 0 ? kSeqOrigin : 0);
     }
@@ -411,6 +417,8 @@ sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, bool counted
     Slot &sl = slots[si];
     const BatchDev *db = (const BatchDev *)sl.d_stage.ptr;
     keys_dirty = true; // until the sequence is enqueued: its shade kernel empties the keys
+    if (sl.seq_flags & kSeqLayers)
+        heads_dirty = true; // (its resolve the list heads)
     if (use_graph) {
         cudaGraphExec_t &g = sl.graph[tile_index(tile)][sl.seq_flags];
         if (!g) {
@@ -437,6 +445,8 @@ sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, bool counted
         CUDA_TRY(launch_batch(db, tile, sl.seq_flags, stream, launches, prof));
     }
     keys_dirty = sl.keep_keys;
+    if (sl.seq_flags & kSeqLayers)
+        heads_dirty = false;
     unsigned long long *hc = (unsigned long long *)sl.h_counters.ptr;
     const StageLayout at = stage_layout(sl.n_items);
     const uint8_t *ds = (const uint8_t *)sl.d_stage.ptr;
