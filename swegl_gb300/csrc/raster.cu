@@ -658,10 +658,14 @@ __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
 // visible triangle (about half of a closed mesh's) stops after the visibility
 // test, and projected vertices are stored only for primitives with an entry
 // in a list, which are all that the later passes read: 64 views 691 -> 573 us,
-// of 200 spheres.
+// of 200 spheres.  Blocks are of four warps, as all of a block wait for its
+// slowest primitive and for the reservation, and the first item's world
+// positions are copied beside the triangles: 1080p 27.5 -> 25.5 us, 64 views
+// 595 -> 579 us (with row_empty); eight warps 27.2 and 583, two 27.0 and 602.
+// The grid is eight waves of blocks: 64 views take 643 us in two, 679 in one.
 constexpr int kGeomVerts = 2;           // vertices of a lane with loads in flight (four spill registers: 683 us for 573)
 constexpr int kGeomTG = kFuseTris / 32; // groups of 32 triangles
-constexpr int kGeomBlocks = 4;          // resident blocks per SM the pass is compiled for
+constexpr int kGeomBlocks = 32 / kGeomWarps; // resident blocks per SM the pass is compiled for
 // words of an item's camera in shared memory: view and projection rows 0-2, then
 enum { GV_VM00 = 24, GV_VM03, GV_VM11, GV_VM13, GV_Y, GV_YEND, GV_ITEM, GV_TRI, kGeomViewWords };
 static_assert(kGeomViewWords == 32, "a warp stages an item's camera, a word per lane");
@@ -677,7 +681,8 @@ struct GeomShared {
     uint32_t base[2];                               // the block's first position in each list
 };
 static_assert(kFuseVerts <= 256, "local vertex indices are bytes");
-static_assert(kGeomItems * kGeomWarps == 64 && 64 * kFuseTris < 65536, "a warp scans the counts, two a lane, in 16 bits");
+static_assert(kGeomItems * kGeomWarps <= 64 && kGeomWarps % 2 == 0 && 64 * kFuseTris < 65536,
+              "a warp scans the counts, two of one item a lane, in 16 bits");
 constexpr size_t kGeomSmem = sizeof(GeomShared);
 
 // The local vertex indices of triangle t of a fused primitive (a | b << 8 | c << 16).
@@ -737,9 +742,9 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
         if (g_lo + first != i_lo) {
             i_lo = g_lo + first;
             nv = (int)min((uint32_t)kGeomItems, g_n - first);
-            // warp vi stages item vi's camera (kGeomItems <= kGeomWarps)
-            if (warp < nv) {
-                const uint32_t item = __ldg(b->grp_items + i_lo + warp);
+            // a warp stages an item's camera at a time
+            for (int sv = warp; sv < nv; sv += kGeomWarps) {
+                const uint32_t item = __ldg(b->grp_items + i_lo + sv);
                 const ItemDev &it = b->items[item];
                 float x;
                 if (lane < 12)
@@ -753,9 +758,9 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                                         : lane == GV_YEND ? (uint32_t)(it.v.y + it.v.h)
                                         : lane == GV_ITEM ? item
                                                           : __ldg(b->tri_base + item));
-                S.view[warp][lane] = x;
+                S.view[sv][lane] = x;
                 if (lane == 0)
-                    S.ndc[warp] = it.ndc;
+                    S.ndc[sv] = it.ndc;
             }
         }
         const SceneDev &sc = b->items[__ldg(b->grp_items + i_lo)].s; // vertex data shared by the group
@@ -771,15 +776,22 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
             gq = sc.pgeo[q];
             gq.y = min(gq.y, kFuseVerts); // (a fused scene's primitives are within both limits)
             gq.w = min(gq.w, kFuseTris);
+            if (sc.pbox)
+                unseen = geom_unseen(b, sc.pbox, q, i_lo, (uint32_t)nv, lane);
+            // the first item's world positions go where its vertices will be
+            // (each lane transforms those it copied)
+            if (!(unseen & 1u))
+                for (uint32_t i = lane; i < gq.y; i += 32)
+                    cp_async<16>(pos + i, wpos + gq.x + i);
             if (lane < gq.w)
                 tr0 = geom_tri(tris, gq, lane);
             if (lane + 32 < gq.w)
                 tr1 = geom_tri(tris, gq, lane + 32);
             ds = sc.pshade[q].double_sided != 0;
-            if (sc.pbox)
-                unseen = geom_unseen(b, sc.pbox, q, i_lo, (uint32_t)nv, lane);
         }
         wpos += gq.x;
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncthreads(); // the cameras are staged
         for (int vi = 0; vi < nv; vi++) {
             uint32_t entries = 0, nx = 0;
@@ -799,7 +811,7 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
 #pragma unroll
                         for (int k = 0; k < kGeomVerts; k++)
                             if (i0 + lane + 32 * k < gq.y)
-                                w[k] = wpos[i0 + lane + 32 * k];
+                                w[k] = vi ? wpos[i0 + lane + 32 * k] : pos[i0 + lane + 32 * k];
 #pragma unroll
                         for (int k = 0; k < kGeomVerts; k++) {
                             const uint32_t i = i0 + lane + 32 * k;
@@ -922,19 +934,22 @@ __global__ void __launch_bounds__(kGeomWarps * 32, kGeomBlocks) k_geom(const Bat
                 if ((int)lane >= d)
                     incl += u;
             }
-            S.off[k] = incl - a - z;
-            S.off[k + 1] = incl - z;
+            if (k < kGeomItems * kGeomWarps) {
+                S.off[k] = incl - a - z;
+                S.off[k + 1] = incl - z;
+            }
             if (lane == 31) {
                 const unsigned long long old = reserve_lists(b, incl & 0xFFFFu, incl >> 16);
                 S.base[0] = (uint32_t)old;
                 S.base[1] = (uint32_t)(old >> 32);
             }
-            // the items' drawn triangles (a lane's two counts are one item's, four lanes' make it whole)
+            // the items' drawn triangles (kGeomWarps / 2 lanes hold one item's)
             uint32_t x = k < nv * kGeomWarps ? S.nx[k] + S.nx[k + 1] : 0u;
-            x += __shfl_xor_sync(0xFFFFFFFFu, x, 1);
-            x += __shfl_xor_sync(0xFFFFFFFFu, x, 2);
-            if ((lane & 3) == 0 && x)
-                atomicAdd(b->item_counters + 2 * (size_t)__float_as_uint(S.view[lane >> 2][GV_ITEM]),
+#pragma unroll
+            for (int d = 1; d < kGeomWarps / 2; d <<= 1)
+                x += __shfl_xor_sync(0xFFFFFFFFu, x, d);
+            if (lane % (kGeomWarps / 2) == 0 && x)
+                atomicAdd(b->item_counters + 2 * (size_t)__float_as_uint(S.view[lane / (kGeomWarps / 2)][GV_ITEM]),
                           (unsigned long long)x);
         }
         __syncthreads();

@@ -52,7 +52,7 @@ static_assert(sizeof(PrimShade) == 32, "PrimShade layout");
 constexpr uint32_t kFuseVerts = 256, kFuseTris = 512;
 // The fused geometry pass: a block takes kGeomWarps primitives of a group (one
 // warp each) and runs them for every item of the group.
-constexpr int kGeomWarps = 8;
+constexpr int kGeomWarps = 4;
 // ... at most kGeomItems at a time: a unit of its work is kGeomWarps primitives
 // and kGeomItems items of a group.
 constexpr int kGeomItems = 8;
