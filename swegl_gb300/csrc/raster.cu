@@ -115,7 +115,13 @@ __global__ void k_world(SceneDev s)
 // k_world for a batch's posed views: the same transforms under each view's own
 // node matrices, into its own arrays, all views in one launch (a launch and a
 // copy per view, half of a 16-view batch's passes before its first triangle,
-// left the GPU idle between them).
+// left the GPU idle between them).  Blocks beyond the vertices' make the boxes
+// of the small primitives, each from its box before the transform (pose_box;
+// a primitive is under one node): read back from the posed positions, a warp
+// a primitive, they took a second pass (16 views of 50 spheres: 18 us beside
+// the transforms' 32; now 32 together, the looser boxes cost k_geom nothing).
+// One pass with a warp a primitive took 48: a strip's 66 vertices fill 69 % of
+// its lanes, and the transforms are bound by instruction issue.
 // Index of the pose whose blocks (`first`) hold block x.
 template <uint32_t PoseDev::*FIRST> __device__ __forceinline__ int find_pose(const PoseDev *p, int n, uint32_t x)
 {
@@ -129,8 +135,22 @@ template <uint32_t PoseDev::*FIRST> __device__ __forceinline__ int find_pose(con
     }
     return lo;
 }
-__global__ void __launch_bounds__(256) k_pose(const PoseDev *poses, int n)
+__global__ void __launch_bounds__(256) k_pose(const PoseDev *poses, int n, uint32_t vertex_blocks)
 {
+    if (blockIdx.x >= vertex_blocks) {
+        const uint32_t x = blockIdx.x - vertex_blocks;
+        const PoseDev &p = poses[find_pose<&PoseDev::prim_block>(poses, n, x)];
+        const uint32_t q = (x - p.prim_block) * kPosePrims + threadIdx.x;
+        if (p.pbox && q < p.n_prims) {
+            const uint4 gq = p.pgeo[q];
+            float4 c = make_float4(NAN, 0.0f, 0.0f, 0.0f), h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (gq.y && in_bounds(gq.x < p.n_vertices, CHK_NDC, gq.x))
+                pose_box(p.node_world + 16 * p.vnode[gq.x], p.lbox[2 * q], p.lbox[2 * q + 1], c, h);
+            p.pbox[2 * q] = c;
+            p.pbox[2 * q + 1] = h;
+        }
+        return;
+    }
     const PoseDev p = poses[find_pose<&PoseDev::vertex_block>(poses, n, blockIdx.x)];
     const uint32_t g0 = (blockIdx.x - p.vertex_block) * kPoseVertices + threadIdx.x;
     constexpr int kPer = kPoseVertices / 256;
@@ -227,15 +247,6 @@ __global__ void k_box(SceneDev s, const float4 *wpos, float4 *pbox)
     if (q < s.n_prims)
         primitive_box(s.pgeo[q], s.n_vertices, wpos, pbox + 2 * q);
 }
-// ... of a batch's posed views.
-__global__ void __launch_bounds__(kPosePrims * 32) k_pose_box(const PoseDev *poses, int n)
-{
-    const PoseDev &p = poses[find_pose<&PoseDev::prim_block>(poses, n, blockIdx.x)];
-    const uint32_t q = (blockIdx.x - p.prim_block) * kPosePrims + (threadIdx.x >> 5);
-    if (p.pbox && q < p.n_prims)
-        primitive_box(p.pgeo[q], p.n_vertices, p.wpos, p.pbox + 2 * q);
-}
-
 // world_to_camera_or_frustum (vertex_shaders.hpp:35-52): view, projection
 // (rows 0-2), x and y divided by |z'|; also clears the visibility flag.  The
 // item's matrices stay in registers while the index is inside it.  Each
@@ -3604,12 +3615,17 @@ cudaError_t launch_world(const SceneDev &s, cudaStream_t st)
     return cudaGetLastError();
 }
 
+cudaError_t launch_local_boxes(const SceneDev &s, float4 *lbox, cudaStream_t st)
+{
+    if (s.n_prims)
+        k_box<<<(s.n_prims + 7) / 8, 256, 0, st>>>(s, s.pos_u, lbox);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, uint32_t prim_blocks, cudaStream_t st)
 {
-    if (vertex_blocks)
-        k_pose<<<vertex_blocks, 256, 0, st>>>(poses, n);
-    if (prim_blocks)
-        k_pose_box<<<prim_blocks, kPosePrims * 32, 0, st>>>(poses, n);
+    if (vertex_blocks + prim_blocks)
+        k_pose<<<vertex_blocks + prim_blocks, 256, 0, st>>>(poses, n, vertex_blocks);
     return cudaGetLastError();
 }
 

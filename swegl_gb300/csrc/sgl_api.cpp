@@ -504,7 +504,7 @@ static sgl_status batch_entries(Ctx *ctx, const sgl_batch_item *items, int n, st
 
 // Batch items with their own pose: the node matrices composed on the host (as
 // sgl_scene_set_nodes does), then k_pose writes the items' world positions and
-// normals (and k_pose_box their primitives' boxes) into the lane's pose scratch
+// normals (and the primitives' boxes) into the lane's pose scratch
 // on the lane's stream, and the items' entries point at them (the scene's own
 // arrays and nodes are untouched).
 static sgl_status pose_items(Ctx *ctx, Lane *lane, const sgl_batch_item *items, int n, std::vector<BatchEntry> &e)

@@ -63,6 +63,27 @@ __host__ __device__ __forceinline__ void cull_box(float3 lo, float3 hi, float4 &
         bc.x = NAN;
 }
 
+// A box that holds the positions of a box (bc, bh) transformed in float by rows
+// 0-2 of M (transform3, whose error is below 8 ulp of the sum of the absolute
+// terms; 64 are added, which also hold the rounding here): NaN centre when it
+// is not finite.
+__host__ __device__ __forceinline__ void pose_box(const float *M, float4 bc, float4 bh, float4 &pc, float4 &ph)
+{
+    float c[3], h[3];
+    for (int i = 0; i < 3; i++) {
+        const float *m = M + 4 * i;
+        const float mx = fabsf(m[0]), my = fabsf(m[1]), mz = fabsf(m[2]);
+        const float reach = mx * bh.x + my * bh.y + mz * bh.z;
+        c[i] = m[0] * bc.x + m[1] * bc.y + m[2] * bc.z + m[3];
+        h[i] = reach + 0x1p-18f * (mx * fabsf(bc.x) + my * fabsf(bc.y) + mz * fabsf(bc.z) + fabsf(m[3]) + reach) +
+               0x1p-120f;
+    }
+    pc = make_float4(c[0], c[1], c[2], 0.0f);
+    ph = make_float4(h[0], h[1], h[2], 0.0f);
+    if (!(fabsf(c[0]) + h[0] + fabsf(c[1]) + h[1] + fabsf(c[2]) + h[2] < 0x1p100f))
+        pc.x = NAN;
+}
+
 // True when the box lies in front of the camera (region z' > 0) and beyond
 // one of the side planes: no triangle inside it passes inside_camera_frustum.
 __host__ __device__ __forceinline__ bool cull_unseen(const float4 cull[5][2], float4 bc, float4 bh)

@@ -300,6 +300,8 @@ void prof_flush(Profiler *p);
 
 // kernel launchers (raster.cu)
 cudaError_t launch_world(const SceneDev &s, cudaStream_t st);
+// The boxes of the primitives' positions before any transform.
+cudaError_t launch_local_boxes(const SceneDev &s, float4 *lbox, cudaStream_t st);
 // Fills SceneDev::alpha (n_texs + 1 words).
 cudaError_t launch_alpha(const SceneDev &s, cudaStream_t st);
 // One posed view: the scene's arrays, the pose's node matrices (device) and
@@ -309,12 +311,13 @@ struct PoseDev {
     const float4 *pos_u, *nrm_v;
     const uint32_t *vnode;
     const uint4 *pgeo;
+    const float4 *lbox; // the primitives' boxes before any transform
     const float *node_world, *node_rs;
     float4 *wpos, *wnrm, *pbox;
     uint32_t n_vertices, n_prims;
-    uint32_t vertex_block, prim_block; // blocks of the two kernels before this pose's
+    uint32_t vertex_block, prim_block; // blocks of vertices and of primitives before this pose's
 };
-constexpr uint32_t kPoseVertices = 1024, kPosePrims = 8; // per block
+constexpr uint32_t kPoseVertices = 1024, kPosePrims = 256; // per block
 // `poses` (device) of `n` views, covering vertex_blocks and prim_blocks blocks.
 cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, uint32_t prim_blocks, cudaStream_t st);
 // The launch sequence of a batch whose BatchDev lives at `b` (device memory).

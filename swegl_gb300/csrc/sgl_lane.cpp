@@ -395,13 +395,14 @@ sgl_status pose_views(Ctx *ctx, DevBuf &dev, HostBuf &host, const std::vector<Po
             e.pbox = (float4 *)(d + arrays);
             arrays += align_up(2 * sizeof(float4) * s.dev.n_prims, 256);
         }
-        const PoseDev p{s.dev.pos_u, s.dev.nrm_v, s.dev.vnode, s.dev.pgeo, e.node_world, e.node_rs, e.wpos, e.wnrm,
+        const PoseDev p{s.dev.pos_u, s.dev.nrm_v, s.dev.vnode, s.dev.pgeo, (const float4 *)s.d_lbox.ptr,
+                        e.node_world, e.node_rs, e.wpos, e.wnrm,
                         e.pbox, s.n_vertices, s.dev.n_prims, (uint32_t)vb, (uint32_t)pb};
         memcpy(h + sizeof(PoseDev) * i, &p, sizeof p);
         vb += (s.n_vertices + kPoseVertices - 1) / kPoseVertices;
         pb += e.pbox ? (s.dev.n_prims + kPosePrims - 1) / kPosePrims : 0;
     }
-    if (vb >= (1ull << 31) || pb >= (1ull << 31)) {
+    if (vb + pb >= (1ull << 31)) {
         ctx->fail("posed batch too large");
         return SGL_ERR_UNSUPPORTED;
     }

@@ -443,6 +443,7 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     if (dev.fused) { // the primitives' boxes, written with the world positions
         CUDA_TRY(d_pbox.ensure(2 * sizeof(float4) * pgeo.size()));
         dev.pbox = (float4 *)d_pbox.ptr;
+        CUDA_TRY(d_lbox.ensure(2 * sizeof(float4) * pgeo.size())); // ... and before any transform, for poses
     }
     dev.n_vertices = n_vertices;
     dev.n_triangles = n_triangles;
@@ -455,6 +456,8 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     CUDA_TRY(d_alpha.ensure(sizeof(uint32_t) * ((size_t)d->n_textures + 1)));
     dev.alpha = (uint32_t *)d_alpha.ptr;
     CUDA_TRY(launch_alpha(dev, 0));
+    if (dev.fused)
+        CUDA_TRY(launch_local_boxes(dev, (float4 *)d_lbox.ptr, 0));
     st = set_lights(ctx, d->ambient, d->sun_direction, d->sun_intensity, d->point_lights, d->n_point_lights);
     if (st != SGL_OK)
         return st;
@@ -462,7 +465,7 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     if (st != SGL_OK)
         return st;
     device_bytes = d_pos_u.bytes + d_nrm_v.bytes + d_vnode.bytes + d_tris.bytes + d_prims.bytes + d_mats.bytes +
-                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes + d_alpha.bytes;
+                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes + d_lbox.bytes + d_alpha.bytes;
     return SGL_OK;
 }
 
