@@ -263,9 +263,11 @@ SGL_API sgl_status sgl_render_debug(sgl_ctx *ctx, int scene_id, const sgl_view *
  * Replaces a loop of swegl::_render calls (src/render/renderer.cpp:77-235)
  * over independent viewports. */
 typedef struct sgl_batch_opts {
-    int tile;      /* shade tile edge: 8, 16 or 32 pixels (0 = context default) */
-    int span_bin;  /* spans wider than this many pixels are binned to the
-                      warp-cooperative span kernels (1..64, 0 = default 16) */
+    int tile;      /* shade tile edge: 8, 16 or 32 pixels (0 = context default;
+                      a batch of one view is not shaded by tiles) */
+    int span_bin;  /* spans wider than this many pixels are walked by several
+                      lanes together (1..64, 0 = default 16; beyond 64 pixels,
+                      and those of tall triangles, by the span kernel) */
     int use_graph; /* run the launch sequence as a captured CUDA graph */
 } sgl_batch_opts;
 

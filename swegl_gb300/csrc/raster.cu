@@ -5,6 +5,7 @@
 // totals from device memory, so one launch sequence (and one CUDA graph)
 // serves any batch.  The plain one-frame-per-launch renderer is a batch of one.
 //
+//   k_geom        the next three for primitives of few vertices, a warp each
 //   k_vertex      world -> view -> projection, |z'| divide      (vertex_shaders.hpp:35-52)
 //   k_flags       visibility flags of triangles                  (renderer.cpp:86-185)
 //   k_compact     drawable triangles -> the walk, tall or near-clip list
@@ -12,11 +13,15 @@
 //                 rows dealt across a warp's lanes, fragment keys folded with
 //                 an atomic min; then the warp's share of the near-clip
 //                 triangles and of the tall triangles
-//   k_spans       long spans binned by the walk, one warp each
+//   k_spans       long spans binned by the walk, several lanes each
 //   k_winners     winner records of binned spans and near-clip triangles
 //                 (every span after a bin overflow)
-//   k_shade       per pixel: background or the winner's colour, and depth;
-//                 winners are queued so that shading runs on full warps
+//   k_shade       batches of several views, per pixel: background or the
+//                 winner's colour, and depth; winners are queued so that
+//                 shading runs on full warps
+//   k_classify    single views: background, depth, the list of winners (and
+//                 k_winners' records)
+//   k_shade_wins  ... and the winners' colours
 //   k_dof         depth-of-field gather of the items that ask for it
 //
 // Depth test.  The reference draws triangles in order and keeps a fragment
@@ -522,7 +527,7 @@ __device__ __forceinline__ void list_tall(const BatchDev *b, bool want, uint32_t
 
 // Drawable triangles (all three vertices flagged, renderer.cpp:248-253) into
 // the walk list, or the tall list when they have many rows; triangles crossing
-// the near plane go to their own list and are marked in the record map.  One
+// the near plane go to their own list and are marked in their records.  One
 // global atomic per list per block.
 constexpr int kCompactBlock = 512;
 __global__ void __launch_bounds__(kCompactBlock) k_compact(const BatchDev *b)
