@@ -100,6 +100,17 @@ __device__ __forceinline__ void sh_fragment(Shader &sh, const SVert &s, const SV
 // intensity / distance^2 ratio only skips more).  Sums below 2^-100 (where
 // products could be subnormal), squared distances from 2^100 up (where the
 // length could overflow) and NaNs take the full path.
+//
+// The specular power is left out where the term cannot change the diffuse one
+// that it is added to: with b the base, the term is b^p p / 2 / d2, and where
+// p log2(b) < log2(diffuse d2) - 36 it is below p / 2 * 2^-36 of the diffuse
+// term, for p up to 1024 below 2^-27 of it, while half a unit in its last
+// place is at least 2^-25 of it.  The factor of 4 between them holds what the
+// approximate logarithms (2^-22 each, the first times p), the roundings of the
+// test and a subnormal diffuse d2 can add, together less than a factor of 2.
+// Only materials are held to 1024 at upload: a default material's exponent
+// beyond it, or below 0, takes the power (without that bound 59,328 of the
+// 2,000,000 sums of tests/shade_math/light_skip.cu differ).
 __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 center, V3 normal, V3 camvec,
                                                     int shininess)
 {
@@ -128,7 +139,9 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
         diffuse = diffuse * alignment;
         const V3 reflection = add3(ld, mul3(normal, alignment * 2.0f));
         float specular = dot3(reflection, camvec);
-        if (specular > 0.0f && !(fp * log2_approx(specular) < log2_approx(diffuse * d2) - 36.0f)) {
+        const bool unseen =
+            (uint32_t)shininess <= 1024u && fp * log2_approx(specular) < log2_approx(diffuse * d2) - 36.0f;
+        if (specular > 0.0f && !unseen) {
             specular = spec_pow(specular, shininess);
             specular = specular * fp / 2.0f;
             dyn = dyn + (diffuse + specular / d2);
