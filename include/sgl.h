@@ -228,7 +228,9 @@ SGL_API sgl_status sgl_scene_info(sgl_ctx *ctx, int scene_id, uint64_t *n_triang
  * `targets[i]` receives view i.  When `device_buffers` is 0 the target
  * pointers are host memory and the call copies in and out (synchronous);
  * when 1 they are device memory and the call is asynchronous on `stream`
- * (a cudaStream_t, NULL = legacy default stream). */
+ * (a cudaStream_t, NULL = legacy default stream); a context's device calls
+ * share their scratch, so a call on another stream waits there for the one
+ * before. */
 SGL_API sgl_status sgl_render(sgl_ctx *ctx, int scene_id, const sgl_view *views, const sgl_target *targets,
                               int n_views, int device_buffers, void *stream, sgl_frame_stats *stats);
 

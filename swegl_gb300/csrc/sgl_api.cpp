@@ -77,9 +77,8 @@ static sgl_status ext_lane(Ctx *ctx, cudaStream_t st, Lane **out)
             return r;
         ctx->ext_lane = std::move(l);
     }
-    ctx->ext_lane->stream = st;
     *out = ctx->ext_lane.get();
-    return SGL_OK;
+    return ctx->ext_lane->move_to(ctx, st);
 }
 
 // Entry points other than sgl_render take opaque views only.
@@ -536,6 +535,7 @@ static sgl_status pose_items(Ctx *ctx, Lane *lane, const sgl_batch_item *items, 
     CUDA_TRY(cudaEventSynchronize(sl.posed)); // its staging is free again
     const sgl_status r = pose_views(ctx, lane->poses, sl.h_pose, posed, lane->stream);
     CUDA_TRY(cudaEventRecord(sl.posed, lane->stream));
+    lane->last = sl.posed;
     return r;
 }
 

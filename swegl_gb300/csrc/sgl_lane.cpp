@@ -101,6 +101,23 @@ sgl_status Lane::init(Ctx *ctx, int max_items_, cudaStream_t external, bool bloc
     return SGL_OK;
 }
 
+sgl_status Lane::move_to(Ctx *ctx, cudaStream_t st)
+{
+    if (st == stream)
+        return SGL_OK;
+    // (the event was recorded with the work: the old stream may be gone.  A
+    // stream under capture cannot wait for work outside its graph; ordering
+    // the graph's launches is then the caller's.)
+    if (last && cudaEventQuery(last) == cudaErrorNotReady) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
+            CUDA_TRY(cudaStreamWaitEvent(st, last, 0));
+    }
+    cudaGetLastError();
+    stream = st;
+    return SGL_OK;
+}
+
 sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inline_span, uint8_t *slot_flags,
                          int *slot_out)
 {
@@ -458,6 +475,7 @@ sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, bool counted
         CUDA_TRY(cudaMemcpyAsync(hc + C_FRAGS / 2, ds + at.counters + sizeof(unsigned long long) * (C_FRAGS / 2),
                                  sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaEventRecord(sl.done, stream));
+    last = sl.done;
     return SGL_OK;
 }
 

@@ -139,10 +139,15 @@ struct Lane {
     size_t frag_want = 0;            // fragments the pool must hold (grown after an overflow)
     bool heads_dirty = false; // the list heads may hold other than kFragEnd (failed launch)
     bool keys_dirty = false; // the key pool may hold other than kEmptyKey (debug, failed launch)
+    cudaEvent_t last = nullptr; // recorded after the lane's newest work (a slot's `done` or `posed`)
     ~Lane();
 
     // external == nullptr: own stream, blocking (ordered with the legacy default stream) or not
     sgl_status init(Ctx *ctx, int max_items, cudaStream_t external, bool blocking = false);
+    // Further work goes to `st`, after what the lane has enqueued elsewhere:
+    // all of it uses the lane's pools, and some of it leaves state in them
+    // (empty depth keys and list heads) that the next sequence starts from.
+    sgl_status move_to(Ctx *ctx, cudaStream_t st);
     // Stage and copy the descriptors of a batch into a free slot; returns its index.
     sgl_status prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inline_span, uint8_t *slot_flags,
                        int *slot_out);
