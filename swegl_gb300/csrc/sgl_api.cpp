@@ -72,7 +72,7 @@ static sgl_status ext_lane(Ctx *ctx, cudaStream_t st, Lane **out)
 {
     if (!ctx->ext_lane) {
         auto l = std::make_unique<Lane>();
-        sgl_status r = l->init(ctx, kMaxBatch, st);
+        sgl_status r = l->init(ctx, kMaxBatch, &st);
         if (r != SGL_OK)
             return r;
         ctx->ext_lane = std::move(l);

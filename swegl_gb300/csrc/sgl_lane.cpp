@@ -74,22 +74,21 @@ Lane::~Lane()
         if (sl.posed)
             cudaEventDestroy(sl.posed);
     }
-    if (own_stream && stream)
-        cudaStreamDestroy(stream);
+    if (own_stream)
+        cudaStreamDestroy(own_stream);
     if (capture_stream)
         cudaStreamDestroy(capture_stream);
 }
 
-sgl_status Lane::init(Ctx *ctx, int max_items_, cudaStream_t external, bool blocking)
+sgl_status Lane::init(Ctx *ctx, int max_items_, const cudaStream_t *external, bool blocking)
 {
     max_items = max_items_;
     CUDA_TRY(init_device_constants());
     if (external) {
-        stream = external;
-        own_stream = false;
+        stream = *external;
     } else {
-        CUDA_TRY(cudaStreamCreateWithFlags(&stream, blocking ? cudaStreamDefault : cudaStreamNonBlocking));
-        own_stream = true;
+        CUDA_TRY(cudaStreamCreateWithFlags(&own_stream, blocking ? cudaStreamDefault : cudaStreamNonBlocking));
+        stream = own_stream;
     }
     for (auto &sl : slots) {
         CUDA_TRY(sl.d_stage.ensure(stage_layout(max_items).bytes));

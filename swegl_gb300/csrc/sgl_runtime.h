@@ -112,7 +112,7 @@ struct Lane {
     int max_items = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t capture_stream = nullptr;
-    bool own_stream = false;
+    cudaStream_t own_stream = nullptr; // made by init when it was given none
     struct Slot {
         // The batch's descriptors in one block, copied to the device at once:
         // the BatchDev (whose address the graphs hold), the counters (copied
@@ -142,8 +142,8 @@ struct Lane {
     cudaEvent_t last = nullptr; // recorded after the lane's newest work (a slot's `done` or `posed`)
     ~Lane();
 
-    // external == nullptr: own stream, blocking (ordered with the legacy default stream) or not
-    sgl_status init(Ctx *ctx, int max_items, cudaStream_t external, bool blocking = false);
+    // external: the caller's stream; nullptr: own stream, blocking (ordered with the legacy default stream) or not
+    sgl_status init(Ctx *ctx, int max_items, const cudaStream_t *external, bool blocking = false);
     // Further work goes to `st`, after what the lane has enqueued elsewhere:
     // all of it uses the lane's pools, and some of it leaves state in them
     // (empty depth keys and list heads) that the next sequence starts from.

@@ -97,6 +97,30 @@ static int streams()
     return 0;
 }
 
+// A context first used on the legacy default stream, then on its caller's and
+// on its own (the tuner): only streams that it made are destroyed, once.
+static int ownership()
+{
+    const int id = upload();
+    cudaStream_t a = test_stream();
+    sgl_batch_item it{};
+    it.scene_id = id, it.view = view_of(64, 48), it.target = target_of(64, 48);
+    sgl_batch_opts o{};
+    if (frame(id, nullptr) != SGL_OK || frame(id, a) != SGL_OK)
+        return 2;
+    sgl_ctx *first = ctx;
+    if (sgl_create(&ctx, 0) != SGL_OK)
+        return 2;
+    it.scene_id = upload();
+    if (frame(it.scene_id, nullptr) != SGL_OK || sgl_autotune(ctx, &it, 1, &o) != SGL_OK)
+        return 2;
+    sgl_destroy(ctx);
+    sgl_destroy(first);
+    ctx = nullptr;
+    printf("%ld %ld\n", fake::foreign_streams_destroyed, fake::streams_destroyed_twice);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     if (sgl_create(&ctx, 0) != SGL_OK)
@@ -104,6 +128,8 @@ int main(int argc, char **argv)
     int r = 2;
     if (argc > 1 && !strcmp(argv[1], "streams"))
         r = streams();
+    else if (argc > 1 && !strcmp(argv[1], "ownership"))
+        r = ownership();
     fake::auto_progress = true;
     sgl_destroy(ctx);
     return r;

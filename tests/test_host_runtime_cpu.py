@@ -37,3 +37,8 @@ def test_calls_on_alternating_streams_are_ordered(exe):
     stream starts after the one before."""
     (unordered,) = run(exe, "streams")
     assert unordered == 0
+
+
+def test_only_own_streams_are_destroyed(exe):
+    foreign, twice = run(exe, "ownership")
+    assert foreign == 0 and twice == 0
