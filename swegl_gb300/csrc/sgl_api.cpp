@@ -721,8 +721,8 @@ SGL_API sgl_status sgl_dof(sgl_ctx *c, const sgl_view *view, const sgl_target *i
     it.dof_tiles_x = (v.w + kDofTile - 1) / kDofTile;
     const uint32_t dof_tiles = (uint32_t)it.dof_tiles_x * (uint32_t)((v.h + kDofTile - 1) / kDofTile);
     // the item, the batch, the prefixes and the (zero) counters in one
-    // page-locked block and one copy (the call waits before it returns, so the
-    // block is free again)
+    // page-locked block and one copy (the call waits before it returns, also
+    // when it fails, so the block is free again)
     const size_t b_at = sizeof(ItemDev), base_at = b_at + sizeof(BatchDev),
                  counters_at = (base_at + 4 * sizeof(uint32_t) + 15) & ~(size_t)15,
                  desc_bytes = counters_at + sizeof(unsigned long long) * kCounterWords;
@@ -745,12 +745,14 @@ SGL_API sgl_status sgl_dof(sgl_ctx *c, const sgl_view *view, const sgl_target *i
     memcpy(hd + b_at, &b, sizeof b);
     memcpy(hd + base_at, base, sizeof base);
     CUDA_TRY(cudaMemcpyAsync(dd, hd, desc_bytes, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(launch_dof(d_b, st));
-    if (!device_buffers) {
-        CUDA_TRY(cudaMemcpy2DAsync((uint8_t *)out->pixels + (size_t)v.y * out->pitch + 4 * (size_t)v.x, out->pitch,
-                                   dst, 4 * (size_t)v.w, 4 * (size_t)v.w, v.h, cudaMemcpyDeviceToHost, st));
-    }
-    CUDA_TRY(cudaStreamSynchronize(st)); // (and the descriptors' block is free again)
+    cudaError_t gathered = launch_dof(d_b, st);
+    if (gathered == cudaSuccess && !device_buffers)
+        gathered = cudaMemcpy2DAsync((uint8_t *)out->pixels + (size_t)v.y * out->pitch + 4 * (size_t)v.x,
+                                     out->pitch, dst, 4 * (size_t)v.w, 4 * (size_t)v.w, v.h, cudaMemcpyDeviceToHost,
+                                     st);
+    const cudaError_t waited = cudaStreamSynchronize(st);
+    CUDA_TRY(gathered);
+    CUDA_TRY(waited);
     return SGL_OK;
 }
 

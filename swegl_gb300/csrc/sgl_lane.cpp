@@ -431,6 +431,18 @@ static int tile_index(int tile) { return tile == 8 ? 0 : (tile == 32 ? 2 : 1); }
 
 sgl_status Lane::launch(Ctx *ctx, int si, int tile, bool use_graph, bool counted, int *launches, Profiler *prof)
 {
+    const sgl_status r = enqueue(ctx, si, tile, use_graph, counted, launches, prof);
+    if (r != SGL_OK) {
+        // no event follows the slot's staged copy then: wait for it here, so
+        // that the slot's next batch does not rewrite what it reads
+        cudaStreamSynchronize(stream);
+        cudaGetLastError();
+    }
+    return r;
+}
+
+sgl_status Lane::enqueue(Ctx *ctx, int si, int tile, bool use_graph, bool counted, int *launches, Profiler *prof)
+{
     Slot &sl = slots[si];
     const BatchDev *db = (const BatchDev *)sl.d_stage.ptr;
     keys_dirty = true; // until the sequence is enqueued: its shade kernel empties the keys

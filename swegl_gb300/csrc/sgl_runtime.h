@@ -153,7 +153,9 @@ struct Lane {
                        int *slot_out);
     // Run the launch sequence of a prepared slot (directly, or as a CUDA graph).
     // `counted`: read_counters will be called.
+    // A failed launch has waited for what it enqueued.
     sgl_status launch(Ctx *ctx, int slot, int tile, bool use_graph, bool counted, int *launches, Profiler *prof);
+    sgl_status enqueue(Ctx *ctx, int slot, int tile, bool use_graph, bool counted, int *launches, Profiler *prof);
     // Per-batch and per-item counters of a finished slot (synchronises the slot).
     sgl_status read_counters(Ctx *ctx, int slot, unsigned long long *drawn, unsigned long long *fragments,
                              std::vector<unsigned long long> *per_item);

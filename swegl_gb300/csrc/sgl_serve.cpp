@@ -157,6 +157,10 @@ void Server::launch_batch_on(LaneState &ls, std::vector<Job> &&jobs)
     int kernels_launched = 0;
     if (st == SGL_OK)
         st = ls.lane->launch(c, ls.slot, tile, !ls.layered, true, &kernels_launched, nullptr);
+    if (st != SGL_OK) { // the poses' staging may still be copied from, and no event will say when it is free
+        cudaStreamSynchronize(ls.lane->stream);
+        cudaGetLastError();
+    }
     {
         std::lock_guard<std::mutex> g(mu);
         batches++;

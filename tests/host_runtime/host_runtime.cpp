@@ -121,6 +121,57 @@ static int ownership()
     return 0;
 }
 
+// Calls that fail after their staging was handed to an asynchronous copy, and
+// the same calls again.
+static int failures()
+{
+    const int id = upload();
+    cudaStream_t a = test_stream();
+    fake::overwritten = 0;
+    for (int k = 0; k < 4; k++) {
+        fake::fail_on = k % 2 ? "" : "launch_dof";
+        sgl_view v = view_of(64 + k, 48);
+        v.dof.enabled = 1, v.dof.max_radius = 4.0f;
+        const sgl_target t = target_of(64 + k, 48);
+        if ((sgl_dof(ctx, &v, &t, &t, 1, a) == SGL_OK) != (k % 2 == 1))
+            return 2;
+    }
+    fake::drain_all();
+    const long dof = fake::overwritten;
+    for (int k = 0; k < 16; k++) {
+        fake::fail_on = k < 12 ? (k % 2 ? "cudaGraphLaunch" : "launch_batch") : "";
+        if ((batch(id, a, k % 3 == 0, k % 2 != 0) == SGL_OK) != (k >= 12))
+            return 2;
+    }
+    fake::drain_all();
+    const long batches = fake::overwritten - dof;
+    // posed requests: the first fails when its sequence is launched
+    fake::auto_progress = true;
+    const sgl_serve_opts opts{0, 4, 1, 0};
+    sgl_server *srv = nullptr;
+    if (sgl_server_create(ctx, &opts, &srv) != SGL_OK)
+        return 2;
+    for (int k = 0; k < 4; k++) {
+        sgl_node_desc node{};
+        node.scale[0] = node.scale[1] = node.scale[2] = 1.0f;
+        node.parent = -1;
+        node.translation[0] = (float)k;
+        sgl_request req{};
+        req.scene_id = id, req.view = view_of(64, 48);
+        req.nodes = &node, req.n_nodes = 1;
+        uint64_t ticket = 0;
+        sgl_request_result res{};
+        fake::fail_on = k % 2 ? "" : "cudaGraphLaunch";
+        if (sgl_server_submit(srv, &req, &ticket) != SGL_OK || sgl_server_wait(srv, ticket, 60.0, &res) != SGL_OK ||
+            (res.status == SGL_OK) != (k % 2 == 1))
+            return 2;
+    }
+    sgl_server_destroy(srv);
+    fake::drain_all();
+    printf("%ld %ld %ld\n", dof, batches, fake::overwritten - dof - batches);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     if (sgl_create(&ctx, 0) != SGL_OK)
@@ -130,6 +181,8 @@ int main(int argc, char **argv)
         r = streams();
     else if (argc > 1 && !strcmp(argv[1], "ownership"))
         r = ownership();
+    else if (argc > 1 && !strcmp(argv[1], "failures"))
+        r = failures();
     fake::auto_progress = true;
     sgl_destroy(ctx);
     return r;

@@ -42,3 +42,8 @@ def test_calls_on_alternating_streams_are_ordered(exe):
 def test_only_own_streams_are_destroyed(exe):
     foreign, twice = run(exe, "ownership")
     assert foreign == 0 and twice == 0
+
+
+def test_staging_is_not_reused_before_its_copy_after_a_failed_call(exe):
+    dof, batches, posed = run(exe, "failures")
+    assert (dof, batches, posed) == (0, 0, 0)
