@@ -344,7 +344,8 @@ constexpr int kSeqDof = 1, kSeqShaders = 2, kSeqLayers = 4, kSeqFused = 8, kSeqS
 // kernel and its round trip through L2, at any size (winner records and shade,
 // tiled / list: 640 x 480 cube 16.8 / 13.9 us, 960 x 540 18.9 / 13.8, 1283 x
 // 719 flat 24.6 / 15.3).  Views below this many pixels do not count the list
-// in their scratch bytes: the allocation-free call uses it where it fits.
+// in their scratch bytes: the allocation-free call and the serving budget use
+// it where it fits.
 constexpr uint64_t kWinListCounted = 1u << 20;
 cudaError_t launch_batch(const BatchDev *b, int tile, int flags, cudaStream_t st, int *launches, Profiler *prof);
 // The device-side bounds checks of the checked build (-DSGL_BOUNDS_CHECK):

@@ -229,7 +229,7 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     }
     CUDA_TRY(prec.ensure(sizeof(float4) * std::max<uint64_t>(tp, 1)));
     // one view: the shade goes through a winner list
-    const bool win_list = n == 1 && e[0].view.layers == 0;
+    const bool win_list = n == 1 && e[0].view.layers == 0 && (small_lists || tp >= kWinListCounted);
     if (win_list)
         CUDA_TRY(wins.ensure(sizeof(uint2) * tp));
     CUDA_TRY(list.ensure(sizeof(uint2) * std::max<uint64_t>(tt, 1)));

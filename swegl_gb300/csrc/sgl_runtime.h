@@ -137,6 +137,7 @@ struct Lane {
                                            // general geometry pass's vertices and triangles; the fused
                                            // pass's group chunks, group items and the grouped items
     size_t frag_want = 0;            // fragments the pool must hold (grown after an overflow)
+    bool small_lists = true;  // single views below kWinListCounted pixels shade through a winner list
     bool heads_dirty = false; // the list heads may hold other than kFragEnd (failed launch)
     bool keys_dirty = false; // the key pool may hold other than kEmptyKey (debug, failed launch)
     cudaEvent_t last = nullptr; // recorded after the lane's newest work (a slot's `done` or `posed`)

@@ -95,6 +95,15 @@ static size_t request_bytes(const Scene *s, const sgl_view &v)
     return 8 * (size_t)v.w * v.h + view_scratch_bytes(s->n_vertices, s->n_triangles, v.w, v.h) + layers;
 }
 
+// Bytes of the winner list of a batch of one view beyond what request_bytes
+// counts: a list of a small view takes the place of the depth-of-field colour
+// and depth (8 B a pixel), of which a served view with depth of field uses 4.
+static size_t uncounted_list_bytes(const sgl_view &v)
+{
+    const size_t px = (size_t)v.w * v.h;
+    return v.dof.enabled && v.layers == 0 && px < kWinListCounted ? 4 * px : 0;
+}
+
 // Frame bytes of the next batch when n_free streams are free.  With copy-out
 // the copies of a batch can only run beside another batch's kernels, so what
 // is queued is spread over the free streams, a smaller part first (its copies
@@ -327,6 +336,16 @@ void Server::run()
                     pending.pop_front();
                     if (layered)
                         break;
+                }
+                // the list of a small view alone counts when it fits, else the view is shaded by tiles
+                free_lane->lane->small_lists = true;
+                if (batch.size() == 1) {
+                    const size_t list = uncounted_list_bytes(batch[0].req.view);
+                    free_lane->lane->small_lists = in_flight_bytes + list <= opts.budget_bytes;
+                    if (free_lane->lane->small_lists) {
+                        in_flight_bytes += list;
+                        batch[0].bytes += list;
+                    }
                 }
             }
             if (batch.empty()) {

@@ -172,6 +172,47 @@ static int failures()
     return 0;
 }
 
+// One request on a server whose budget is the least that admits it: the device
+// bytes that it allocates beyond the budget, without and with depth of field,
+// then with the budget of two and with four times as much.
+static int budget()
+{
+    const int id = upload();
+    fake::auto_progress = true;
+    for (int k = 0; k < 4; k++) {
+        sgl_request req{};
+        req.scene_id = id, req.view = view_of(1000, 1000);
+        req.view.dof.enabled = k > 0, req.view.dof.max_radius = 8.0f;
+        uint64_t lo = 0, hi = 1ull << 32; // refused, admitted
+        auto serve = [&](uint64_t bytes, long long *over) {
+            const sgl_serve_opts opts{bytes, 4, 1, 0};
+            sgl_server *srv = nullptr;
+            uint64_t ticket = 0;
+            sgl_request_result res{};
+            if (sgl_server_create(ctx, &opts, &srv) != SGL_OK)
+                exit(2);
+            const size_t before = fake::peak = fake::live;
+            const bool in = sgl_server_submit(srv, &req, &ticket) == SGL_OK;
+            if (in && over) {
+                if (sgl_server_wait(srv, ticket, 60.0, &res) != SGL_OK || res.status != SGL_OK)
+                    exit(2);
+                *over = (long long)(fake::peak - before) - (long long)bytes;
+            }
+            sgl_server_destroy(srv);
+            return in;
+        };
+        while (hi - lo > 1) {
+            const uint64_t mid = lo + (hi - lo) / 2;
+            (serve(mid, nullptr) ? hi : lo) = mid;
+        }
+        long long over = 0;
+        serve(k == 2 ? 2 * hi : (k == 3 ? 4 * hi : hi), &over);
+        printf("%lld ", over);
+    }
+    printf("\n");
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     if (sgl_create(&ctx, 0) != SGL_OK)
@@ -183,6 +224,8 @@ int main(int argc, char **argv)
         r = ownership();
     else if (argc > 1 && !strcmp(argv[1], "failures"))
         r = failures();
+    else if (argc > 1 && !strcmp(argv[1], "budget"))
+        r = budget();
     fake::auto_progress = true;
     sgl_destroy(ctx);
     return r;

@@ -47,3 +47,8 @@ def test_only_own_streams_are_destroyed(exe):
 def test_staging_is_not_reused_before_its_copy_after_a_failed_call(exe):
     dof, batches, posed = run(exe, "failures")
     assert (dof, batches, posed) == (0, 0, 0)
+
+
+def test_a_request_stays_within_the_budget_that_admits_it(exe):
+    over = run(exe, "budget")
+    assert len(over) == 4 and max(over) <= 0
