@@ -1811,27 +1811,34 @@ struct WalkShared {
     uint2 entry[4][32];
 };
 
-// Fragments of the lanes' triangles (fewer than 2^26 each, or counted at once)
-// added to the block's sums of the first kWalkItems items, the others' to
-// their counters.  An atomic on the item's counter per group of 32 triangles
-// met all the warps that were walking the same view: 98 us of the 64-view
-// batch's 589.  Every lane of the warp calls it.
+// Fragments of the lanes' triangles added to the block's sums of the first
+// kWalkItems items, the others' to their counters: one addition per item of the
+// warp, or one per lane where a triangle has 2^26 fragments and more.  Few
+// items' counters meet all the warps that walk the same view; more items'
+// spread over as many addresses (32 views of 512 x 384, of 200 spheres, take
+// 752 us in all with the sums and 812 with counters alone; from 64 views on the
+// walk is as long either way, 364 and 366 us, and sums of 256 or 1,024 items
+// change nothing at 96 to 4,096 views).  Additions by lane were what cost:
+// 96 views 1,950 us, 548 now.  Every lane of the warp calls it.
 constexpr int kWalkItems = 64;
 __device__ __forceinline__ void block_add(const BatchDev *b, uint32_t *sums, uint32_t item, uint32_t n)
 {
     const unsigned act = __ballot_sync(0xFFFFFFFFu, n != 0u);
     if (!n)
         return;
-    if (__any_sync(act, (n >> 26) || item >= (uint32_t)kWalkItems)) {
-        atomicAdd(b->item_counters + 2 * (size_t)item + 1, (unsigned long long)n);
+    unsigned long long *counter = b->item_counters + 2 * (size_t)item + 1;
+    if (__any_sync(act, n >> 26)) {
+        atomicAdd(counter, (unsigned long long)n);
         return;
     }
     const unsigned grp = __match_any_sync(act, item);
     const uint32_t sum = __reduce_add_sync(grp, n);
-    if ((threadIdx.x & 31) == __ffs(grp) - 1 && atomicAdd(sums + item, sum) >> 31) {
-        const uint32_t all = atomicExch(sums + item, 0u); // (well before it overflows)
-        atomicAdd(b->item_counters + 2 * (size_t)item + 1, (unsigned long long)all);
-    }
+    if ((threadIdx.x & 31) != __ffs(grp) - 1)
+        return;
+    if (item >= (uint32_t)kWalkItems)
+        atomicAdd(counter, (unsigned long long)sum);
+    else if (atomicAdd(sums + item, sum) >> 31) // (well before it overflows)
+        atomicAdd(counter, (unsigned long long)atomicExch(sums + item, 0u));
 }
 
 // Set-up and depth walk of the drawable triangles wholly in front of the near
@@ -1845,7 +1852,7 @@ template <bool FRAGS, bool STRIDED>
 __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(const BatchDev *b)
 {
     __shared__ WalkShared shared[kWalkWarps];
-    __shared__ uint32_t item_frags[kWalkItems]; // fragments of the batch's first items, walked by this block
+    __shared__ uint32_t item_frags[STRIDED ? 1 : kWalkItems]; // fragments of the batch's first items, walked by this block
     WalkShared &W = shared[threadIdx.x >> 5];
     WalkRow *S = W.S;
     const int lane = threadIdx.x & 31;
@@ -1883,8 +1890,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
             }
         }
     };
+    const int summed = min(b->n_items, kWalkItems);
     if (!STRIDED) {
-        for (int i = (int)threadIdx.x; i < kWalkItems; i += kWalkWarps * 32)
+        for (int i = (int)threadIdx.x; i < summed; i += kWalkWarps * 32)
             item_frags[i] = 0u;
         __syncthreads();
     }
@@ -2015,7 +2023,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, SGL_WALK_MIN_BLOCKS) k_walk(c
     walk_tall_all<FRAGS>(b, S);
     if (!STRIDED) {
         __syncthreads();
-        for (int i = (int)threadIdx.x; i < kWalkItems; i += kWalkWarps * 32)
+        for (int i = (int)threadIdx.x; i < summed; i += kWalkWarps * 32)
             if (item_frags[i])
                 atomicAdd(b->item_counters + 2 * (size_t)i + 1, (unsigned long long)item_frags[i]);
     }
