@@ -182,35 +182,40 @@ __global__ void __launch_bounds__(256) k_pose(const PoseDev *poses, int n, uint3
     }
 }
 
-// The AND of each texture's texels (blockIdx.y strides over the textures), and
-// the triangles of primitives whose texture or, without one, colour has an
-// alpha below 255.
-__global__ void __launch_bounds__(256) k_texture_alpha(SceneDev s)
-{
-    for (int t = (int)blockIdx.y; t < s.n_texs; t += (int)gridDim.y) {
-        const TexDesc d = s.texs[t];
-        const size_t n = (size_t)d.w * d.h;
-        uint32_t a = 0xFFFFFFFFu;
-        for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
-            a &= d.texels[i];
-        a = __reduce_and_sync(0xFFFFFFFFu, a);
-        if ((threadIdx.x & 31) == 0)
-            atomicAnd(s.alpha + t, a);
-    }
-}
+// Counts of kAlphaSamples points a triangle those with an alpha below 255: the
+// texels under its centroid and the points halfway from there to its corners,
+// found as the bilinear shader finds them, or its material's colour.  (By
+// triangles, not by texels: of a texture that many objects share, some may be
+// opaque and others not.)
 __global__ void __launch_bounds__(256) k_translucent(SceneDev s)
 {
-    const uint32_t q = blockIdx.x * 256 + threadIdx.x;
+    const uint32_t t = blockIdx.x * 256 + threadIdx.x;
     uint32_t n = 0;
-    if (q < s.n_prims) {
-        const int m = s.prims[q].material;
-        const MatDesc d = m >= 0 && m < s.n_mats ? s.mats[m] : s.default_mat;
-        const uint32_t a = d.texture >= 0 && d.texture < s.n_texs ? s.alpha[d.texture] : d.color;
-        n = (a >> 24) != 255u ? s.pgeo[q].w : 0u;
+    if (t < s.n_triangles) {
+        const uint4 tri = s.tris[t];
+        const PrimShade ps = s.pshade[tri.w];
+        if (!ps.tex) {
+            n = (ps.color >> 24) != 255u ? kAlphaSamples : 0u;
+        } else {
+            const V2 a = mk2(s.pos_u[tri.x].w, s.nrm_v[tri.x].w), b = mk2(s.pos_u[tri.y].w, s.nrm_v[tri.y].w),
+                     c = mk2(s.pos_u[tri.z].w, s.nrm_v[tri.z].w);
+            const V2 mid = mul2(add2(add2(a, b), c), 1.0f / 3.0f);
+            // floor(x) modulo `size`, 0 where it has none
+            auto wrap = [](float x, int size) {
+                const float f = (float)size, r = x - floorf(x / f) * f;
+                return r >= 0.0f && r < f ? min((int)r, size - 1) : 0;
+            };
+            static_assert(kAlphaSamples == 4, "the centroid and three points");
+            const V2 at[kAlphaSamples] = {mid, mul2(add2(mid, a), 0.5f), mul2(add2(mid, b), 0.5f), mul2(add2(mid, c), 0.5f)};
+#pragma unroll
+            for (int k = 0; k < (int)kAlphaSamples; k++)
+                n += (__ldg(ps.tex + (size_t)wrap(at[k].x * (float)ps.tw, ps.th) * ps.tw +
+                            wrap(at[k].y * (float)ps.th, ps.tw)) >> 24) != 255u;
+        }
     }
     n = __reduce_add_sync(0xFFFFFFFFu, n);
     if ((threadIdx.x & 31) == 0 && n)
-        atomicAdd(s.alpha + s.n_texs, n);
+        atomicAdd(s.translucent, (unsigned long long)n);
 }
 
 // The box of each primitive's world positions (a warp per primitive), for the
@@ -3278,17 +3283,29 @@ __device__ __forceinline__ uint32_t shade_frag(const BatchDev *b, const ItemDev 
 }
 
 // Whether fragments are shaded when their pixel is resolved, nearest first
-// until one is opaque, instead of all when they are linked: where less than
-// half of the scene's triangles can be translucent.  In the pool's order
-// neighbours share a triangle and every lane has a fragment; by pixel a warp
-// takes as many turns as its deepest pixel, each a chain of dependent loads.
-// Both passes on 1280 x 720 views of 200 spheres, linked / on demand: block
-// alpha at 0.4, 2.4, 3.1 and 5.8 fragments a pixel of the view 43 / 66, 142 /
-// 245, 129 / 231 and 229 / 361 us; all opaque at 2.4 and 3.1 (three to five a
-// covered pixel, one of them shaded on demand) 132 / 93 and 116 / 100 us.
-__device__ __forceinline__ bool frags_on_demand(const SceneDev &s)
+// until one is opaque, instead of all when they are linked.  In the pool's
+// order neighbours share a triangle and every lane has a fragment, but hidden
+// ones are shaded too; by pixel a warp takes as many turns as its deepest
+// pixel, each a chain of dependent loads.  So it depends on the view's
+// fragments a pixel, f, and on the share p of them that are translucent (of
+// the scene's samples): k_link + k_layers, linked / on demand, us:
+//   f 0.9  p 0: 61 / 62      .05: 61 / 84     .3: 65 / 109
+//   f 1.8  p 0: 109 / 90     .02: 109 / 109   .05: 110 / 119
+//   f 3.3  p 0: 196 / 123    .1: 202 / 177    .15: 204 / 196   .2: 205 / 211
+//   f 6.4  p 0: 384 / 188    .1: 409 / 249    .3: 418 / 353
+//   f 7.0  p 0: 78 / 46      .15: 84 / 80     .2: 84 / 88
+//   f 13.5 p 0: 267 / 95     .15: 282 / 132   .3: 284 / 175
+// (1280 x 720 but for 7.0 and 13.5).  The line f = 1.25 + 16 p lies between,
+// and f = 1 where none is translucent: a pixel then takes one turn, else a warp
+// takes those of its deepest (calls at 640 x 360, linked / on demand: f 1.0 to 1.25,
+// p 0 258 / 246 us; f 1.4, p .02 159 / 169).  From a half on they are linked: the
+// turns grow with the chain's length squared.
+__device__ __forceinline__ bool frags_on_demand(const BatchDev *b, const ItemDev &it)
 {
-    return 2u * (unsigned long long)__ldg(s.alpha + s.n_texs) < s.n_triangles;
+    const unsigned long long n = __ldg(it.s.translucent);
+    const float p = (float)n / ((float)kAlphaSamples * (float)it.s.n_triangles);
+    const float px = (float)it.v.w * (float)it.v.h;
+    return p < 0.5f && (float)*frag_counter(b) > px * (n ? 1.25f + 16.0f * p : 1.0f);
 }
 
 // Chains the stored fragments to their pixels: one thread per pool entry
@@ -3302,7 +3319,7 @@ __global__ void __launch_bounds__(256, SGL_SHADE_MIN_BLOCKS) k_link(const BatchD
         return;
     const uint32_t n = (uint32_t)*frag_counter(b);
     const ItemDev &it = b->items[0];
-    const bool on_demand = frags_on_demand(it.s);
+    const bool on_demand = frags_on_demand(b, it);
     uint32_t *head = it.frag_head;
     Frag *pool = b->frags;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -3503,7 +3520,7 @@ __global__ void __launch_bounds__(256, 4) k_layers(const BatchDev *b)
         return;
     const ItemDev &it = b->items[0];
     const uint32_t total = (uint32_t)it.v.w * (uint32_t)it.v.h;
-    if (!frags_on_demand(it.s)) {
+    if (!frags_on_demand(b, it)) {
         // (a pixel's list head is loaded two turns ahead and its first fragment
         // one, so that a turn waits for neither: 26.6 -> 23.5 us; four consecutive
         // pixels a thread, with 16-byte accesses, 41.6 us)
@@ -3642,17 +3659,13 @@ cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, ui
     return cudaGetLastError();
 }
 
-cudaError_t launch_alpha(const SceneDev &s, cudaStream_t st)
+cudaError_t launch_translucent(const SceneDev &s, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(s.alpha, 0xFF, sizeof(uint32_t) * (size_t)s.n_texs, st);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(s.alpha + s.n_texs, 0, sizeof(uint32_t), st);
+    const cudaError_t e = cudaMemsetAsync(s.translucent, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess)
         return e;
-    if (s.n_texs)
-        k_texture_alpha<<<dim3(16, (unsigned)std::min(s.n_texs, 65535)), 256, 0, st>>>(s);
-    if (s.n_prims)
-        k_translucent<<<grid_for(s.n_prims, 256), 256, 0, st>>>(s);
+    if (s.n_triangles)
+        k_translucent<<<grid_for(s.n_triangles, 256), 256, 0, st>>>(s);
     return cudaGetLastError();
 }
 

@@ -97,8 +97,7 @@ struct SceneDev {
     int n_mats;
     int n_texs;
     MatDesc default_mat;
-    uint32_t *alpha;         // per texture the AND of its texels, then the triangles whose material has an alpha
-                             // below 255 (k_texture_alpha, k_translucent: at upload)
+    unsigned long long *translucent; // of kAlphaSamples points a triangle those with an alpha below 255 (at upload)
 };
 
 struct ViewDev {
@@ -302,8 +301,9 @@ void prof_flush(Profiler *p);
 cudaError_t launch_world(const SceneDev &s, cudaStream_t st);
 // The boxes of the primitives' positions before any transform.
 cudaError_t launch_local_boxes(const SceneDev &s, float4 *lbox, cudaStream_t st);
-// Fills SceneDev::alpha (n_texs + 1 words).
-cudaError_t launch_alpha(const SceneDev &s, cudaStream_t st);
+// Fills SceneDev::translucent.
+constexpr uint32_t kAlphaSamples = 4;
+cudaError_t launch_translucent(const SceneDev &s, cudaStream_t st);
 // One posed view: the scene's arrays, the pose's node matrices (device) and
 // where its own world positions, normals and primitive boxes go (`pbox` may be
 // null); the scene's own arrays are not touched.

@@ -453,9 +453,9 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
                               d->default_material.double_sided, d->default_material.shininess};
     if (dev.default_mat.texture >= d->n_textures)
         dev.default_mat.texture = -1;
-    CUDA_TRY(d_alpha.ensure(sizeof(uint32_t) * ((size_t)d->n_textures + 1)));
-    dev.alpha = (uint32_t *)d_alpha.ptr;
-    CUDA_TRY(launch_alpha(dev, 0));
+    CUDA_TRY(d_translucent.ensure(sizeof(unsigned long long)));
+    dev.translucent = (unsigned long long *)d_translucent.ptr;
+    CUDA_TRY(launch_translucent(dev, 0));
     if (dev.fused)
         CUDA_TRY(launch_local_boxes(dev, (float4 *)d_lbox.ptr, 0));
     st = set_lights(ctx, d->ambient, d->sun_direction, d->sun_intensity, d->point_lights, d->n_point_lights);
@@ -465,7 +465,7 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     if (st != SGL_OK)
         return st;
     device_bytes = d_pos_u.bytes + d_nrm_v.bytes + d_vnode.bytes + d_tris.bytes + d_prims.bytes + d_mats.bytes +
-                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes + d_lbox.bytes + d_alpha.bytes;
+                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes + d_lbox.bytes + d_translucent.bytes;
     return SGL_OK;
 }
 

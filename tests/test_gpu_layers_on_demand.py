@@ -99,3 +99,35 @@ def test_both_ways_offset_on_a_surface_with_content(renderer, shader):
         frames.append(got[0].pixels)
         renderer.release(sid)
     assert np.array_equal(frames[0], frames[1])
+
+
+def test_one_translucent_texel_costs_an_opaque_scene_little(renderer):
+    """A deep stack of opaque sheets, and the same with one texel of the
+    texture translucent: about the same time in the layer passes (all of the
+    hidden fragments were shaded in the second once)."""
+    times = []
+    for clear in (0, 1):
+        s = S.Scene()
+        t = S.texture_uniform(31, 256, 256) | np.uint32(0xFF000000)
+        t[0, :clear] &= np.uint32(0x80FFFFFF)
+        s.textures.append(t)
+        s.materials.append((0xFFFFFFFF, 0, 1, 32))
+        q = np.array([[-3.0, -2.0, 0.0], [3.0, -2.0, 0.0], [3.0, 2.0, 0.0], [-3.0, 2.0, 0.0]], np.float32)
+        nq = np.tile(np.array([0.0, 0.0, 1.0], np.float32), (4, 1))
+        uq = np.array([[0.01, 0.01], [0.96, 0.01], [0.96, 0.97], [0.01, 0.97]], np.float32)
+        for k in range(100):
+            node = s.add_node(translation=(0.0, 0.0, -2.0 + 0.01 * k))
+            s.add_primitive(node, S.TRIANGLE_FAN, 0, q, nq, uq, np.arange(4, dtype=np.uint32))
+        s.point_lights = [(0.0, 1.0, 2.0, 2.0)]
+        sid = renderer.upload(s.finalize())
+        v = view(320, 240, 2)
+        best = 1e9
+        for _ in range(6):
+            renderer.profile(True)
+            renderer.render(sid, [v])
+            p = renderer.profile_read()
+            best = min(best, p["k_frags"]["total_ms"] + p["k_layers"]["total_ms"])
+        renderer.profile(False)
+        times.append(best)
+        renderer.release(sid)
+    assert times[1] < 1.25 * times[0], times
