@@ -182,42 +182,6 @@ __global__ void __launch_bounds__(256) k_pose(const PoseDev *poses, int n, uint3
     }
 }
 
-// Counts of kAlphaSamples points a triangle those with an alpha below 255: the
-// texels under its centroid and the points halfway from there to its corners,
-// found as the bilinear shader finds them, or its material's colour.  (By
-// triangles, not by texels: of a texture that many objects share, some may be
-// opaque and others not.)
-__global__ void __launch_bounds__(256) k_translucent(SceneDev s)
-{
-    const uint32_t t = blockIdx.x * 256 + threadIdx.x;
-    uint32_t n = 0;
-    if (t < s.n_triangles) {
-        const uint4 tri = s.tris[t];
-        const PrimShade ps = s.pshade[tri.w];
-        if (!ps.tex) {
-            n = (ps.color >> 24) != 255u ? kAlphaSamples : 0u;
-        } else {
-            const V2 a = mk2(s.pos_u[tri.x].w, s.nrm_v[tri.x].w), b = mk2(s.pos_u[tri.y].w, s.nrm_v[tri.y].w),
-                     c = mk2(s.pos_u[tri.z].w, s.nrm_v[tri.z].w);
-            const V2 mid = mul2(add2(add2(a, b), c), 1.0f / 3.0f);
-            // floor(x) modulo `size`, 0 where it has none
-            auto wrap = [](float x, int size) {
-                const float f = (float)size, r = x - floorf(x / f) * f;
-                return r >= 0.0f && r < f ? min((int)r, size - 1) : 0;
-            };
-            static_assert(kAlphaSamples == 4, "the centroid and three points");
-            const V2 at[kAlphaSamples] = {mid, mul2(add2(mid, a), 0.5f), mul2(add2(mid, b), 0.5f), mul2(add2(mid, c), 0.5f)};
-#pragma unroll
-            for (int k = 0; k < (int)kAlphaSamples; k++)
-                n += (__ldg(ps.tex + (size_t)wrap(at[k].x * (float)ps.tw, ps.th) * ps.tw +
-                            wrap(at[k].y * (float)ps.th, ps.tw)) >> 24) != 255u;
-        }
-    }
-    n = __reduce_add_sync(0xFFFFFFFFu, n);
-    if ((threadIdx.x & 31) == 0 && n)
-        atomicAdd(s.translucent, (unsigned long long)n);
-}
-
 // The box of each primitive's world positions (a warp per primitive), for the
 // fused pass's whole-primitive frustum test: pbox[2 q] = centre, pbox[2 q + 1]
 // = half extent.  NaN coordinates are left out (a triangle with one fails
@@ -251,11 +215,56 @@ __device__ __forceinline__ void primitive_box(uint4 gq, uint32_t n_vertices, con
         out[1] = h;
     }
 }
-__global__ void k_box(SceneDev s, const float4 *wpos, float4 *pbox)
+// Counts of kAlphaSamples points a triangle those with an alpha below 255: the
+// texels under its centroid and the points halfway from there to its corners,
+// found as the bilinear shader finds them, or its material's colour.  (By
+// triangles, not by texels: of a texture that many objects share, some may be
+// opaque and others not.)
+__device__ __forceinline__ void count_translucent(const SceneDev &s, uint32_t t)
 {
-    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (q < s.n_prims)
-        primitive_box(s.pgeo[q], s.n_vertices, wpos, pbox + 2 * q);
+    uint32_t n = 0;
+    if (t < s.n_triangles) {
+        const uint4 tri = s.tris[t];
+        const PrimShade ps = s.pshade[tri.w];
+        if (!ps.tex) {
+            n = (ps.color >> 24) != 255u ? kAlphaSamples : 0u;
+        } else {
+            const V2 a = mk2(s.pos_u[tri.x].w, s.nrm_v[tri.x].w), b = mk2(s.pos_u[tri.y].w, s.nrm_v[tri.y].w),
+                     c = mk2(s.pos_u[tri.z].w, s.nrm_v[tri.z].w);
+            const V2 mid = mul2(add2(add2(a, b), c), 1.0f / 3.0f);
+            // floor(x) modulo `size`, 0 where it has none
+            auto wrap = [](float x, int size) {
+                const float f = (float)size, r = x - floorf(x / f) * f;
+                return r >= 0.0f && r < f ? min((int)r, size - 1) : 0;
+            };
+            static_assert(kAlphaSamples == 4, "the centroid and three points");
+            const V2 at[kAlphaSamples] = {mid, mul2(add2(mid, a), 0.5f), mul2(add2(mid, b), 0.5f), mul2(add2(mid, c), 0.5f)};
+#pragma unroll
+            for (int k = 0; k < (int)kAlphaSamples; k++)
+                n += (__ldg(ps.tex + (size_t)wrap(at[k].x * (float)ps.tw, ps.th) * ps.tw +
+                            wrap(at[k].y * (float)ps.th, ps.tw)) >> 24) != 255u;
+        }
+    }
+    n = __reduce_add_sync(0xFFFFFFFFu, n);
+    if ((threadIdx.x & 31) == 0 && n)
+        atomicAdd(s.translucent, (unsigned long long)n);
+}
+
+// The boxes, and at upload those of the positions before any transform
+// (`lbox`) in the first `box_blocks` blocks, the translucent samples in the
+// others.  (Launches and arrays of their own cost a small scene's upload: the
+// textured cube 177 us, 149 so, 159 before there were samples and such boxes.)
+__global__ void __launch_bounds__(256) k_box(SceneDev s, float4 *lbox, uint32_t box_blocks)
+{
+    if (blockIdx.x >= box_blocks) {
+        count_translucent(s, (blockIdx.x - box_blocks) * 256 + threadIdx.x);
+        return;
+    }
+    const uint32_t w = (blockIdx.x * 256 + threadIdx.x) >> 5;
+    const bool local = w >= s.n_prims;
+    const uint32_t q = local ? w - s.n_prims : w;
+    if (q < s.n_prims && (!local || lbox))
+        primitive_box(s.pgeo[q], s.n_vertices, local ? s.pos_u : s.wpos, (local ? lbox : s.pbox) + 2 * q);
 }
 // world_to_camera_or_frustum (vertex_shaders.hpp:35-52): view, projection
 // (rows 0-2), x and y divided by |z'|; also clears the visibility flag.  The
@@ -3635,20 +3644,15 @@ static int sm_count()
     return n;
 }
 
-cudaError_t launch_world(const SceneDev &s, cudaStream_t st)
+cudaError_t launch_world(const SceneDev &s, bool uploaded, float4 *lbox, cudaStream_t st)
 {
     if (s.n_vertices == 0)
         return cudaSuccess;
     k_world<<<grid_for(s.n_vertices, 256), 256, 0, st>>>(s);
-    if (s.pbox && s.n_prims)
-        k_box<<<(s.n_prims + 7) / 8, 256, 0, st>>>(s, s.wpos, s.pbox);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_local_boxes(const SceneDev &s, float4 *lbox, cudaStream_t st)
-{
-    if (s.n_prims)
-        k_box<<<(s.n_prims + 7) / 8, 256, 0, st>>>(s, s.pos_u, lbox);
+    const unsigned boxes = s.pbox ? grid_for((uploaded ? 2ull : 1ull) * s.n_prims, 8) : 0u,
+                   samples = uploaded ? grid_for(s.n_triangles, 256) : 0u;
+    if (boxes + samples)
+        k_box<<<boxes + samples, 256, 0, st>>>(s, uploaded ? lbox : nullptr, boxes);
     return cudaGetLastError();
 }
 
@@ -3656,16 +3660,6 @@ cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, ui
 {
     if (vertex_blocks + prim_blocks)
         k_pose<<<vertex_blocks + prim_blocks, 256, 0, st>>>(poses, n, vertex_blocks);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_translucent(const SceneDev &s, cudaStream_t st)
-{
-    const cudaError_t e = cudaMemsetAsync(s.translucent, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess)
-        return e;
-    if (s.n_triangles)
-        k_translucent<<<grid_for(s.n_triangles, 256), 256, 0, st>>>(s);
     return cudaGetLastError();
 }
 

@@ -77,7 +77,6 @@ struct SceneDev {
     const uint4 *tris;       // draw-order triangles: 3 global vertex indices + draw-order primitive
     const PrimDesc *prims;   // draw-order primitives
     const MatDesc *mats;
-    const TexDesc *texs;
     const float *node_world; // 16 floats per node
     const float *node_rs;    // 16 floats per node
     const LightsDev *lights;
@@ -95,9 +94,7 @@ struct SceneDev {
     float4 *pbox;            // fused: per draw-order primitive, the centre then the half extent of the box of its
                              // world positions (k_box, after k_world); the fused pass's whole-primitive frustum test
     int n_mats;
-    int n_texs;
-    MatDesc default_mat;
-    unsigned long long *translucent; // of kAlphaSamples points a triangle those with an alpha below 255 (at upload)
+    unsigned long long *translucent; // of kAlphaSamples points a triangle those with an alpha below 255 (at upload; behind pgeo)
 };
 
 struct ViewDev {
@@ -298,12 +295,11 @@ const char *prof_kernel_name(int k);
 void prof_flush(Profiler *p);
 
 // kernel launchers (raster.cu)
-cudaError_t launch_world(const SceneDev &s, cudaStream_t st);
-// The boxes of the primitives' positions before any transform.
-cudaError_t launch_local_boxes(const SceneDev &s, float4 *lbox, cudaStream_t st);
-// Fills SceneDev::translucent.
+// World positions, normals and boxes; when `uploaded` also the boxes of the
+// primitives' positions before any transform (into `lbox`, unless null) and
+// SceneDev::translucent (added to).
 constexpr uint32_t kAlphaSamples = 4;
-cudaError_t launch_translucent(const SceneDev &s, cudaStream_t st);
+cudaError_t launch_world(const SceneDev &s, bool uploaded, float4 *lbox, cudaStream_t st);
 // One posed view: the scene's arrays, the pose's node matrices (device) and
 // where its own world positions, normals and primitive boxes go (`pbox` may be
 // null); the scene's own arrays are not touched.

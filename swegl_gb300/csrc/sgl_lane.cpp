@@ -411,7 +411,7 @@ sgl_status pose_views(Ctx *ctx, DevBuf &dev, HostBuf &host, const std::vector<Po
             e.pbox = (float4 *)(d + arrays);
             arrays += align_up(2 * sizeof(float4) * s.dev.n_prims, 256);
         }
-        const PoseDev p{s.dev.pos_u, s.dev.nrm_v, s.dev.vnode, s.dev.pgeo, (const float4 *)s.d_lbox.ptr,
+        const PoseDev p{s.dev.pos_u, s.dev.nrm_v, s.dev.vnode, s.dev.pgeo, s.lbox,
                         e.node_world, e.node_rs, e.wpos, e.wnrm,
                         e.pbox, s.n_vertices, s.dev.n_prims, (uint32_t)vb, (uint32_t)pb};
         memcpy(h + sizeof(PoseDev) * i, &p, sizeof p);

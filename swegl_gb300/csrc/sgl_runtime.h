@@ -52,9 +52,10 @@ struct Ctx;
 
 // A scene resident in device memory.
 struct Scene {
-    DevBuf d_pos_u, d_nrm_v, d_vnode, d_tris, d_prims, d_mats, d_texs, d_texels, d_wpos, d_wnrm,
-        d_node_world, d_node_rs, d_lights, d_pgeo, d_pshade, d_psmall, d_vsmall, d_pbox, d_lbox, d_translucent;
+    DevBuf d_pos_u, d_nrm_v, d_vnode, d_tris, d_prims, d_mats, d_texels, d_wpos, d_wnrm,
+        d_node_world, d_node_rs, d_lights, d_pgeo, d_pshade, d_psmall, d_vsmall, d_pbox;
     SceneDev dev{};
+    float4 *lbox = nullptr; // the primitives' boxes before any transform, for poses (behind dev.pbox)
     LightsDev lights{};
     std::vector<sgl_node_desc> nodes;
     uint32_t n_vertices = 0;
@@ -62,7 +63,7 @@ struct Scene {
     size_t device_bytes = 0;
 
     sgl_status upload_desc(Ctx *ctx, const sgl_scene_desc *d);
-    sgl_status refresh_nodes(Ctx *ctx);
+    sgl_status refresh_nodes(Ctx *ctx, bool uploaded = false); // `uploaded`: the scene's other arrays too
     sgl_status set_lights(Ctx *ctx, float ambient, const float *sun, float sun_intensity, const sgl_point_light *pl,
                           int n);
 };

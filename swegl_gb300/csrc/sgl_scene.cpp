@@ -155,7 +155,7 @@ static cudaError_t upload(DevBuf &b, const T *src, size_t n)
 
 // --------------------------------------------------------------- scenes --
 
-sgl_status Scene::refresh_nodes(Ctx *ctx)
+sgl_status Scene::refresh_nodes(Ctx *ctx, bool uploaded)
 {
     std::vector<float> world, rs;
     if (!node_matrices(nodes, world, rs)) {
@@ -167,7 +167,7 @@ sgl_status Scene::refresh_nodes(Ctx *ctx)
     dev.node_world = (const float *)d_node_world.ptr;
     dev.node_rs = (const float *)d_node_rs.ptr;
     CUDA_TRY(cudaDeviceSynchronize()); // in-flight frames read the world positions
-    CUDA_TRY(launch_world(dev, 0));
+    CUDA_TRY(launch_world(dev, uploaded, lbox, 0));
     CUDA_TRY(cudaStreamSynchronize(0));
     return SGL_OK;
 }
@@ -305,7 +305,7 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
             order.insert(order.end(), v.begin(), v.end());
     }
     std::vector<PrimDesc> prims(order.size());
-    std::vector<uint4> pgeo(order.size());
+    std::vector<uint4> pgeo(order.size() + 1); // the last: the count of translucent samples, zero
     std::vector<uint8_t> psmall(std::max<size_t>(order.size(), 1), 0);
     bool any_small = false, any_big = false;
     std::vector<uint4> tris;
@@ -379,7 +379,6 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     CUDA_TRY(upload(d_prims, prims.data(), prims.size()));
     CUDA_TRY(upload(d_pgeo, pgeo.data(), pgeo.size()));
     CUDA_TRY(upload(d_mats, mats.data(), mats.size()));
-    CUDA_TRY(upload(d_texs, texs.data(), texs.size()));
     // per draw-order primitive: the material and texture the pixel shader binds
     const MatDesc def_mat{d->default_material.color,
                           d->default_material.texture < d->n_textures ? d->default_material.texture : -1,
@@ -413,12 +412,12 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     dev.tris = (const uint4 *)d_tris.ptr;
     dev.prims = (const PrimDesc *)d_prims.ptr;
     dev.mats = (const MatDesc *)d_mats.ptr;
-    dev.texs = (const TexDesc *)d_texs.ptr;
     dev.wpos = (float4 *)d_wpos.ptr;
     dev.wnrm = (float4 *)d_wnrm.ptr;
     dev.pgeo = (const uint4 *)d_pgeo.ptr;
     dev.pshade = (const PrimShade *)d_pshade.ptr;
-    dev.n_prims = (uint32_t)pgeo.size();
+    dev.n_prims = (uint32_t)order.size();
+    dev.translucent = (unsigned long long *)((uint4 *)d_pgeo.ptr + order.size());
     // Primitives within kFuseVerts / kFuseTris take the fused geometry pass.
     // A scene that also has larger ones runs the general passes as well, and
     // each pass skips the other's primitives: the general passes skip the
@@ -429,10 +428,10 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
     dev.mixed = any_small && any_big ? 1 : 0;
     if (dev.mixed) {
         std::vector<uint8_t> vsmall(std::max<uint32_t>(n_vertices, 1), 0);
-        for (size_t q = 0; q < pgeo.size(); q++)
+        for (size_t q = 0; q < order.size(); q++)
             if (psmall[q])
                 std::fill(vsmall.begin() + pgeo[q].x, vsmall.begin() + pgeo[q].x + pgeo[q].y, (uint8_t)1);
-        for (size_t q = 0; q < pgeo.size(); q++)
+        for (size_t q = 0; q < order.size(); q++)
             if (!psmall[q])
                 std::fill(vsmall.begin() + pgeo[q].x, vsmall.begin() + pgeo[q].x + pgeo[q].y, (uint8_t)0);
         CUDA_TRY(upload(d_psmall, psmall.data(), psmall.size()));
@@ -440,32 +439,22 @@ sgl_status Scene::upload_desc(Ctx *ctx, const sgl_scene_desc *d)
         dev.psmall = (const uint8_t *)d_psmall.ptr;
         dev.vsmall = (const uint8_t *)d_vsmall.ptr;
     }
-    if (dev.fused) { // the primitives' boxes, written with the world positions
-        CUDA_TRY(d_pbox.ensure(2 * sizeof(float4) * pgeo.size()));
+    if (dev.fused) { // the primitives' boxes, written with the world positions, and before any transform
+        CUDA_TRY(d_pbox.ensure(4 * sizeof(float4) * order.size()));
         dev.pbox = (float4 *)d_pbox.ptr;
-        CUDA_TRY(d_lbox.ensure(2 * sizeof(float4) * pgeo.size())); // ... and before any transform, for poses
+        lbox = dev.pbox + 2 * order.size();
     }
     dev.n_vertices = n_vertices;
     dev.n_triangles = n_triangles;
     dev.n_mats = d->n_materials;
-    dev.n_texs = d->n_textures;
-    dev.default_mat = MatDesc{d->default_material.color, d->default_material.texture,
-                              d->default_material.double_sided, d->default_material.shininess};
-    if (dev.default_mat.texture >= d->n_textures)
-        dev.default_mat.texture = -1;
-    CUDA_TRY(d_translucent.ensure(sizeof(unsigned long long)));
-    dev.translucent = (unsigned long long *)d_translucent.ptr;
-    CUDA_TRY(launch_translucent(dev, 0));
-    if (dev.fused)
-        CUDA_TRY(launch_local_boxes(dev, (float4 *)d_lbox.ptr, 0));
     st = set_lights(ctx, d->ambient, d->sun_direction, d->sun_intensity, d->point_lights, d->n_point_lights);
     if (st != SGL_OK)
         return st;
-    st = refresh_nodes(ctx);
+    st = refresh_nodes(ctx, true);
     if (st != SGL_OK)
         return st;
     device_bytes = d_pos_u.bytes + d_nrm_v.bytes + d_vnode.bytes + d_tris.bytes + d_prims.bytes + d_mats.bytes +
-                   d_texs.bytes + d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes + d_lbox.bytes + d_translucent.bytes;
+                   d_texels.bytes + d_wpos.bytes + d_wnrm.bytes + d_node_world.bytes + d_node_rs.bytes + d_lights.bytes + d_pgeo.bytes + d_pshade.bytes + d_psmall.bytes + d_vsmall.bytes + d_pbox.bytes;
     return SGL_OK;
 }
 

@@ -293,9 +293,7 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s) { return launch("cu
 } // extern "C"
 
 namespace sgl {
-cudaError_t launch_world(const SceneDev &, cudaStream_t st) { return launch("launch_world", st); }
-cudaError_t launch_local_boxes(const SceneDev &, float4 *, cudaStream_t st) { return launch("launch_local_boxes", st); }
-cudaError_t launch_translucent(const SceneDev &, cudaStream_t st) { return launch("launch_translucent", st); }
+cudaError_t launch_world(const SceneDev &, bool, float4 *, cudaStream_t st) { return launch("launch_world", st); }
 cudaError_t launch_poses(const PoseDev *, int, uint32_t, uint32_t, cudaStream_t st) { return launch("launch_poses", st); }
 cudaError_t launch_batch(const BatchDev *, int, int, cudaStream_t st, int *, Profiler *)
 {

@@ -213,6 +213,17 @@ static int budget()
     return 0;
 }
 
+// Device allocations, copies and launches of an upload (a launch_* call counts
+// once).
+static int uploads()
+{
+    upload();
+    const long before = fake::device_calls;
+    upload();
+    printf("%ld\n", fake::device_calls - before);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     if (sgl_create(&ctx, 0) != SGL_OK)
@@ -226,6 +237,8 @@ int main(int argc, char **argv)
         r = failures();
     else if (argc > 1 && !strcmp(argv[1], "budget"))
         r = budget();
+    else if (argc > 1 && !strcmp(argv[1], "uploads"))
+        r = uploads();
     fake::auto_progress = true;
     sgl_destroy(ctx);
     return r;

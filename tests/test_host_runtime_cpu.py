@@ -52,3 +52,9 @@ def test_staging_is_not_reused_before_its_copy_after_a_failed_call(exe):
 def test_a_request_stays_within_the_budget_that_admits_it(exe):
     over = run(exe, "budget")
     assert len(over) == 4 and max(over) <= 0
+
+
+def test_upload_allocates_and_launches_no_more_than_it_needs(exe):
+    """15 arrays, 12 copies, one launch sequence."""
+    (calls,) = run(exe, "uploads")
+    assert calls <= 28
