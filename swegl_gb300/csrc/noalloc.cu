@@ -15,13 +15,13 @@
 // until the process exits.  Views whose scratch does not fit are refused with
 // SGL_ERR_BUDGET and a message giving the bytes needed.  The call makes no
 // cudaMalloc, cudaFree or other allocating call.  Its descriptors are passed
-// by value to a one-block kernel that writes them into the array (kernel
-// arguments are copied at launch, so no host buffer has to outlive the call).
+// by value to a kernel whose first block writes them into the array, while all
+// of its blocks empty the depth keys (kernel arguments are copied at launch, so
+// no host buffer has to outlive the call).
 //
 // The array is shared by every call in a CUDA context and keeps the last
-// call's contents; each call clears what must start cleared (the counters in
-// the descriptor kernel, the depth keys to all ones there too; the
-// visibility flags are cleared by the kernels).  Calls that overlap on the
+// call's contents; each call clears what must start cleared (the counters and
+// the depth keys in that kernel, the visibility flags in the geometry passes).  Calls that overlap on the
 // GPU in one context (on different streams, or from different host threads)
 // race on the array: the caller must order them.  Each CUDA context has its
 // own copy of the array, so calls in different contexts do not share it.
@@ -283,7 +283,6 @@ SGL_API sgl_status sgl_render_noalloc(sgl_ctx *c, int scene_id, const sgl_view *
     b.items = (const ItemDev *)(base + o_item);
     const uint32_t *bp = (const uint32_t *)(base + o_bases);
     b.tri_base = bp + 2;
-    b.px_base = bp + 4;
     b.tile_base = bp + 6;
     b.dof_base = bp + 8;
     b.g_vtx_base = bp + 10;

@@ -35,7 +35,6 @@
 // shaded with; spans too long to replay cheaply have them recorded by the
 // span kernels instead.  The depth keys start every launch sequence empty:
 // new key pools are filled once and the shade kernel empties what it reads.
-#include <algorithm>
 #include <cstdint>
 
 #include "sgl_cull.h"
@@ -1197,7 +1196,6 @@ struct DepthVisitor {
     uint32_t item;
     uint32_t slot;
     int inline_span;
-    bool bin_all; // tall triangle: every span goes to the bins
     uint32_t drawn_n;
     unsigned long long fragments;
 
@@ -1211,7 +1209,7 @@ struct DepthVisitor {
     __device__ __forceinline__ void span(int y, int x1, int x2, const Side &Ls, const Side &Rs, uint32_t bits)
     {
         fragments += (unsigned long long)(x2 - x1);
-        if ((bin_all || x2 - x1 > inline_span) && bin_span(b, item, slot, y, x1, x2, Ls, Rs, bits))
+        if (x2 - x1 > inline_span && bin_span(b, item, slot, y, x1, x2, Ls, Rs, bits))
             return;
         const ViewDev &v = it->v;
         unsigned long long *row = it->key + ((long long)(y - v.y) * v.w - v.x);
@@ -2153,7 +2151,7 @@ __device__ __noinline__ void walk_clip_depth(const BatchDev *b)
     for (uint32_t i0 = 32 * gw; i0 < n; i0 += 32 * n_warps) {
         const uint32_t i = i0 + lane;
         const bool valid = i < n;
-        DepthVisitor dvis{b, nullptr, 0u, 0u, b->inline_span, false, 0u, 0ull};
+        DepthVisitor dvis{b, nullptr, 0u, 0u, b->inline_span, 0u, 0ull};
         if (valid) {
             const uint2 e = b->clip[b->clip_cap - 1 - i];
             const ItemDev &it = b->items[e.y];
@@ -2796,9 +2794,9 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr)
 //
 // Bound by integer issue (two ALU instructions and a shared-memory read a
 // pixel and tap); before, staging took a quarter of the instructions a word at
-// a time and its latency was the main stall (3840 x 2160, radius 16: 64.2 M
-// instructions and 92 us, now 55.7 M and 71 us; 2560 x 1440 of unlike radii up
-// to 24: 64 -> 55 us).
+// a time and its latency was the main stall (a 3840 x 2160 frame of the spheres,
+// radius 16: 60.9 M instructions and 87.4 us, now 52.0 M and 65.6 us; 2560 x
+// 1440 of unlike radii up to 24: 64 -> 55 us).
 constexpr int kDofBlocks = 5; // resident blocks per SM (shared memory: 37 KB each)
 constexpr int kDofNear = 16;  // halo whose tiles are staged ahead
 constexpr int kDofNearPitch = kDofTile + 2 * kDofNear;
@@ -3119,9 +3117,9 @@ __global__ void __launch_bounds__(256) k_dof_source(const BatchDev *b)
 //    front of it, nearer meaning a smaller depth or, at equal depth, drawn
 //    later (an insertion goes in front of the equal depths already there,
 //    and when every layer is used the farthest is dropped).
-// The capture walk chains every fragment of a pixel; the resolve takes a
-// pixel's chain in (depth, draw order), shading fragments up to the first
-// opaque one.  The flatten and copy passes follow viewport_t::flatten
+// The capture stores every fragment, the linking chains those of a pixel (and
+// shades them, or leaves that to the resolve: frags_on_demand), and the resolve
+// takes a pixel's chain to that outcome.  The flatten and copy passes follow viewport_t::flatten
 // (viewport.cpp:43-86) and post_shader_t's copy of the first layer to the
 // screen (post_shaders.hpp:22-47).  A layered batch holds one view.
 

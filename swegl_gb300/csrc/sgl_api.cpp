@@ -720,11 +720,11 @@ SGL_API sgl_status sgl_dof(sgl_ctx *c, const sgl_view *view, const sgl_target *i
     it.dof_halo = dof_halo_of(v.dof.max_radius);
     it.dof_tiles_x = (v.w + kDofTile - 1) / kDofTile;
     const uint32_t dof_tiles = (uint32_t)it.dof_tiles_x * (uint32_t)((v.h + kDofTile - 1) / kDofTile);
-    // the item, the batch, the prefixes and the (zero) counters in one
+    // the item, the batch, the prefix of tiles and the (zero) counters in one
     // page-locked block and one copy (the call waits before it returns, also
     // when it fails, so the block is free again)
     const size_t b_at = sizeof(ItemDev), base_at = b_at + sizeof(BatchDev),
-                 counters_at = (base_at + 4 * sizeof(uint32_t) + 15) & ~(size_t)15,
+                 counters_at = (base_at + 2 * sizeof(uint32_t) + 15) & ~(size_t)15,
                  desc_bytes = counters_at + sizeof(unsigned long long) * kCounterWords;
     CUDA_TRY(ctx->dof_desc.ensure(desc_bytes));
     CUDA_TRY(ctx->dof_host.ensure(desc_bytes));
@@ -734,12 +734,11 @@ SGL_API sgl_status sgl_dof(sgl_ctx *c, const sgl_view *view, const sgl_target *i
     BatchDev b{};
     b.items = (const ItemDev *)dd;
     b.counters = (unsigned long long *)(dd + counters_at); // the gather's tile counter
-    b.px_base = d_base;
-    b.dof_base = d_base + 2;
+    b.dof_base = d_base;
     b.n_items = 1;
     b.total_px = (uint32_t)px;
     b.total_dof_tiles = dof_tiles;
-    const uint32_t base[4] = {0u, (uint32_t)px, 0u, dof_tiles};
+    const uint32_t base[2] = {0u, dof_tiles};
     memset(hd, 0, desc_bytes);
     memcpy(hd, &it, sizeof it);
     memcpy(hd + b_at, &b, sizeof b);

@@ -69,7 +69,10 @@ struct LightsDev {
     float4 pl[kMaxPointLights]; // x, y, z, intensity
 };
 
-// Device-resident scene (all pointers are device memory).
+// Device-resident scene (all pointers are device memory).  The tiled shade loads
+// `wpos` and `wnrm` as one 16-byte word; `lights` shares no such word with
+// `pshade`, or it would be loaded with it and held from there on (64 views: 425 us
+// so, 434 with the positions' word split, 436 with lights beside pshade).
 struct SceneDev {
     const float4 *pos_u;     // (x, y, z, u)
     const float4 *nrm_v;     // (nx, ny, nz, v)
@@ -80,9 +83,9 @@ struct SceneDev {
     const float *node_world; // 16 floats per node
     const float *node_rs;    // 16 floats per node
     const LightsDev *lights;
+    const uint4 *pgeo;       // draw-order primitives: first vertex, vertex count, first triangle, triangle count
     float4 *wpos;            // v_world, and tex_coords u in w
     float4 *wnrm;            // normal_world, and tex_coords v in w
-    const uint4 *pgeo;       // draw-order primitives: first vertex, vertex count, first triangle, triangle count
     const PrimShade *pshade; // draw-order primitives: material and texture as the pixel shader binds them
     uint32_t n_vertices;
     uint32_t n_triangles;
@@ -96,6 +99,8 @@ struct SceneDev {
     int n_mats;
     unsigned long long *translucent; // of kAlphaSamples points a triangle those with an alpha below 255 (at upload; behind pgeo)
 };
+static_assert(offsetof(SceneDev, wpos) % 16 == 0 && offsetof(SceneDev, wnrm) == offsetof(SceneDev, wpos) + 8,
+              "one word of the shade");
 
 struct ViewDev {
     int x, y, w, h;
@@ -241,7 +246,7 @@ constexpr int kCounterWords = (C_SHADE_Q + 32 * kQueues) / 2; // 64-bit words
 struct BatchDev {
     const ItemDev *items;
     const uint32_t *tri_base;  // n_items + 1 prefix of triangle counts
-    const uint32_t *px_base;   // n_items + 1 prefix of pixel counts
+    uint8_t *slot_flags;       // debug, single-item batches: slot reached scanline setup
     const uint32_t *tile_base; // n_items + 1 prefix of shade-tile counts
     const uint32_t *dof_base;  // n_items + 1 prefix of depth-of-field tile counts (0 for items without)
     // the geometry passes: items of fused scenes in groups that read the same
@@ -265,13 +270,12 @@ struct BatchDev {
                                // triangle with fragments, or flags kRecClip for a near-clipped one (others: stale)
     uint32_t *tall;            // batch triangles walked a warp each (list_cap entries; not in `list`)
     int keep_keys;             // leave the depth keys for the caller (debug); else the shade resets them
-    unsigned long long *key_pool; // the items' depth keys: batch pixel px_base[item] + i at key_pool[...]
+    unsigned long long *key_pool; // the items' depth keys, one item's after the other's
     uint2 *wins;               // kSeqWinList: pixels with a winner {batch pixel, draw slot}, in pixel order
     void *spans;               // long-span bins (span_cap spans of kSpanBytes)
     uint32_t span_cap;
     unsigned long long *counters;      // kCounterWords words
     unsigned long long *item_counters; // per item: drawn, fragments
-    uint8_t *slot_flags;       // debug, single-item batches: slot reached scanline setup
     Frag *frags;               // fragment pool of the views with transparency layers
     uint32_t frag_cap;
 };
@@ -328,7 +332,7 @@ cudaError_t launch_poses(const PoseDev *poses, int n, uint32_t vertex_blocks, ui
 // untouched and the host renders again with a bigger pool.
 // kSeqFused: items of fused scenes (k_geom); kSeqSplit: other items (k_vertex,
 // k_flags, k_compact).  kSeqWinList shades through a winner list (k_classify
-// then k_shade_wins, for a batch of one large view) instead of the tiled
+// then k_shade_wins, for a batch of one view) instead of the tiled
 // k_shade; BatchDev::wins must then hold total_px entries.  kSeqOne: the
 // batch has one view (the walk deals its list entries strided over groups).
 // kSeqOrigin: a layered view at the surface's top left, whose flatten and copy

@@ -329,7 +329,6 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
     bd.items = (const ItemDev *)(ds + at.items);
     const uint32_t *db = (const uint32_t *)(ds + at.bases);
     bd.tri_base = db + (n + 1); // (db[0 .. n]: the vertex prefix, read by nothing on the device)
-    bd.px_base = db + 2 * (n + 1);
     bd.tile_base = db + 3 * (n + 1);
     bd.dof_base = db + 4 * (n + 1);
     bd.g_vtx_base = db + 5 * (n + 1);

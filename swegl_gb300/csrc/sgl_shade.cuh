@@ -140,7 +140,7 @@ __host__ __device__ __forceinline__ float light_sum(const LightsDev &L, V3 cente
         const V3 reflection = add3(ld, mul3(normal, alignment * 2.0f));
         float specular = dot3(reflection, camvec);
         const bool unseen =
-            (uint32_t)shininess <= 1024u && fp * log2_approx(specular) < log2_approx(diffuse * d2) - 36.0f;
+            fp * log2_approx(specular) < log2_approx(diffuse * d2) - 36.0f && (uint32_t)shininess <= 1024u;
         if (specular > 0.0f && !unseen) {
             specular = spec_pow(specular, shininess);
             specular = specular * fp / 2.0f;
