@@ -1824,8 +1824,8 @@ struct WalkShared {
 };
 
 // Fragments of the lanes' triangles added to the block's sums of the first
-// kWalkItems items, the others' to their counters: one addition per item of the
-// warp, or one per lane where a triangle has 2^26 fragments and more.  Few
+// kWalkItems items, or (when the warp holds another, or a triangle of 2^26
+// fragments) to the items' counters: one addition per item of the warp.  Few
 // items' counters meet all the warps that walk the same view; more items'
 // spread over as many addresses (32 views of 512 x 384, of 200 spheres, take
 // 752 us in all with the sums and 812 with counters alone; from 64 views on the
@@ -1835,22 +1835,19 @@ struct WalkShared {
 constexpr int kWalkItems = 64;
 __device__ __forceinline__ void block_add(const BatchDev *b, uint32_t *sums, uint32_t item, uint32_t n)
 {
+    if (__any_sync(0xFFFFFFFFu, n && ((n >> 26) || item >= (uint32_t)kWalkItems))) {
+        item_add(b, 1, item, n, true);
+        return;
+    }
     const unsigned act = __ballot_sync(0xFFFFFFFFu, n != 0u);
     if (!n)
         return;
-    unsigned long long *counter = b->item_counters + 2 * (size_t)item + 1;
-    if (__any_sync(act, n >> 26)) {
-        atomicAdd(counter, (unsigned long long)n);
-        return;
-    }
     const unsigned grp = __match_any_sync(act, item);
     const uint32_t sum = __reduce_add_sync(grp, n);
-    if ((threadIdx.x & 31) != __ffs(grp) - 1)
-        return;
-    if (item >= (uint32_t)kWalkItems)
-        atomicAdd(counter, (unsigned long long)sum);
-    else if (atomicAdd(sums + item, sum) >> 31) // (well before it overflows)
-        atomicAdd(counter, (unsigned long long)atomicExch(sums + item, 0u));
+    if ((threadIdx.x & 31) == __ffs(grp) - 1 && atomicAdd(sums + item, sum) >> 31) {
+        const uint32_t all = atomicExch(sums + item, 0u); // (well before it overflows)
+        atomicAdd(b->item_counters + 2 * (size_t)item + 1, (unsigned long long)all);
+    }
 }
 
 // Set-up and depth walk of the drawable triangles wholly in front of the near
