@@ -535,7 +535,7 @@ static sgl_status pose_items(Ctx *ctx, Lane *lane, const sgl_batch_item *items, 
     CUDA_TRY(cudaEventSynchronize(sl.posed)); // its staging is free again
     const sgl_status r = pose_views(ctx, lane->poses, sl.h_pose, posed, lane->stream);
     CUDA_TRY(cudaEventRecord(sl.posed, lane->stream));
-    lane->last = sl.posed;
+    lane->recorded(sl.posed);
     return r;
 }
 

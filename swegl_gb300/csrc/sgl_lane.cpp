@@ -100,20 +100,33 @@ sgl_status Lane::init(Ctx *ctx, int max_items_, const cudaStream_t *external, bo
     return SGL_OK;
 }
 
+// Whether `st` is under capture (or cannot be asked, as the legacy default
+// stream beside one).
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) == cudaSuccess)
+        return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+void Lane::recorded(cudaEvent_t event)
+{
+    if (capturing(stream))
+        return; // nothing outside the graph can wait for it
+    last = event;
+    last_on = stream;
+}
+
 sgl_status Lane::move_to(Ctx *ctx, cudaStream_t st)
 {
-    if (st == stream)
-        return SGL_OK;
-    // (the event was recorded with the work: the old stream may be gone.  A
-    // stream under capture cannot wait for work outside its graph; ordering
-    // the graph's launches is then the caller's.)
-    if (last && cudaEventQuery(last) == cudaErrorNotReady) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
-            CUDA_TRY(cudaStreamWaitEvent(st, last, 0));
-    }
-    cudaGetLastError();
     stream = st;
+    // (the event was recorded with the work: its stream may be gone; a stream
+    // under capture cannot wait for work outside its graph, whose order is the
+    // caller's)
+    if (last && last_on != st && !capturing(st))
+        CUDA_TRY(cudaStreamWaitEvent(st, last, 0));
     return SGL_OK;
 }
 
@@ -485,7 +498,7 @@ sgl_status Lane::enqueue(Ctx *ctx, int si, int tile, bool use_graph, bool counte
         CUDA_TRY(cudaMemcpyAsync(hc + C_FRAGS / 2, ds + at.counters + sizeof(unsigned long long) * (C_FRAGS / 2),
                                  sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaEventRecord(sl.done, stream));
-    last = sl.done;
+    recorded(sl.done);
     return SGL_OK;
 }
 

@@ -142,6 +142,7 @@ struct Lane {
     bool heads_dirty = false; // the list heads may hold other than kFragEnd (failed launch)
     bool keys_dirty = false; // the key pool may hold other than kEmptyKey (debug, failed launch)
     cudaEvent_t last = nullptr; // recorded after the lane's newest work (a slot's `done` or `posed`)
+    cudaStream_t last_on = nullptr; // ... on this stream
     ~Lane();
 
     // external: the caller's stream; nullptr: own stream, blocking (ordered with the legacy default stream) or not
@@ -150,6 +151,7 @@ struct Lane {
     // all of it uses the lane's pools, and some of it leaves state in them
     // (empty depth keys and list heads) that the next sequence starts from.
     sgl_status move_to(Ctx *ctx, cudaStream_t st);
+    void recorded(cudaEvent_t event); // `event` was recorded after the lane's newest work
     // Stage and copy the descriptors of a batch into a free slot; returns its index.
     sgl_status prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inline_span, uint8_t *slot_flags,
                        int *slot_out);

@@ -42,3 +42,36 @@ def test_alternating_streams_equal_single_frames(batched):
         assert np.array_equal(pix.cpu().numpy().view(np.uint32), f.pixels)
         assert np.array_equal(z.cpu().numpy().view(np.uint32), f.zbuffer.view(np.uint32))
     r.close()
+
+
+def test_calls_after_a_captured_batch():
+    """A batch captured into a caller's graph (direct launches) between calls
+    on other streams: those go on as before, and the replay draws the frame."""
+    import torch
+
+    from swegl_gb300.runtime import Renderer
+
+    r = Renderer(0)
+    sid = r.upload(S.cube_scene())
+    v = S.cube_view(320, 240)
+    pix = torch.zeros((240, 320), dtype=torch.int32, device="cuda")
+    z = torch.zeros((240, 320), dtype=torch.float32, device="cuda")
+    t = abi.Target(pix.data_ptr(), 1280, 320, 240, C.cast(C.c_void_p(z.data_ptr()), C.POINTER(C.c_float)))
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    r.render_batch([(sid, v, t)], use_graph=False, stream=a.cuda_stream)
+    torch.cuda.synchronize()
+    expect = pix.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=b, capture_error_mode="thread_local"):
+        r.render_batch([(sid, v, t)], use_graph=False, stream=b.cuda_stream)
+    pix.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(pix, expect)
+    for stream in (a, b):
+        pix.zero_()
+        torch.cuda.synchronize()
+        r.render_batch([(sid, v, t)], use_graph=False, stream=stream.cuda_stream)
+        torch.cuda.synchronize()
+        assert torch.equal(pix, expect)
+    r.close()
