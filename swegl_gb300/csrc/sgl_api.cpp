@@ -531,11 +531,15 @@ static sgl_status pose_items(Ctx *ctx, Lane *lane, const sgl_batch_item *items, 
     }
     if (posed.empty())
         return SGL_OK;
-    Lane::Slot &sl = lane->slots[lane->next]; // (the batch takes this slot next)
-    CUDA_TRY(cudaEventSynchronize(sl.posed)); // its staging is free again
+    const int si = lane->free_slot(); // (the batch takes it next)
+    if (si < 0)
+        return SGL_OK; // (and says that there is none)
+    Lane::Slot &sl = lane->slots[si];
+    if (sl.pose_used)
+        CUDA_TRY(cudaEventSynchronize(sl.posed)); // its staging is free again
     const sgl_status r = pose_views(ctx, lane->poses, sl.h_pose, posed, lane->stream);
     CUDA_TRY(cudaEventRecord(sl.posed, lane->stream));
-    lane->recorded(sl.posed);
+    sl.pose_used = lane->recorded(sl.posed);
     return r;
 }
 

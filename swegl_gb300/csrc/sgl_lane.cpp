@@ -111,12 +111,21 @@ static bool capturing(cudaStream_t st)
     return true;
 }
 
-void Lane::recorded(cudaEvent_t event)
+bool Lane::recorded(cudaEvent_t event)
 {
     if (capturing(stream))
-        return; // nothing outside the graph can wait for it
+        return false;
     last = event;
     last_on = stream;
+    return true;
+}
+
+int Lane::free_slot() const
+{
+    for (int k = 0; k < kSlots; k++)
+        if (!slots[(next + k) % kSlots].captured)
+            return (next + k) % kSlots;
+    return -1;
 }
 
 sgl_status Lane::move_to(Ctx *ctx, cudaStream_t st)
@@ -137,8 +146,12 @@ sgl_status Lane::prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inl
         ctx->fail("batch of %d views; this lane takes 1..%d", n, max_items);
         return SGL_ERR_INVALID;
     }
-    const int si = next;
-    next = (next + 1) % kSlots;
+    const int si = free_slot();
+    if (si < 0) {
+        ctx->fail("captured graphs hold every staging slot of this context");
+        return SGL_ERR_UNSUPPORTED;
+    }
+    next = (si + 1) % kSlots;
     Slot &sl = slots[si];
     if (sl.used)
         CUDA_TRY(cudaEventSynchronize(sl.done)); // its staging buffers are free again
@@ -498,7 +511,7 @@ sgl_status Lane::enqueue(Ctx *ctx, int si, int tile, bool use_graph, bool counte
         CUDA_TRY(cudaMemcpyAsync(hc + C_FRAGS / 2, ds + at.counters + sizeof(unsigned long long) * (C_FRAGS / 2),
                                  sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaEventRecord(sl.done, stream));
-    recorded(sl.done);
+    sl.captured = !recorded(sl.done);
     return SGL_OK;
 }
 

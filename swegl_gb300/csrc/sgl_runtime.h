@@ -122,8 +122,10 @@ struct Lane {
         HostBuf h_stage, h_counters;
         HostBuf h_pose;              // the batch's posed items: descriptors and matrices
         cudaEvent_t posed = nullptr; // ... copied
+        bool pose_used = false;      // (`posed` can be waited for)
         cudaEvent_t done = nullptr; // launch sequence of this slot done
         bool used = false;
+        bool captured = false;      // its staging is read by a graph that a caller captured: not taken again
         cudaGraphExec_t graph[3][kSeqVariants] = {}; // per tile 8/16/32 and sequence flags (kSeq*)
         int graph_kernels[3][kSeqVariants] = {};     // kernels in each graph
         int n_items = 0;
@@ -151,7 +153,11 @@ struct Lane {
     // all of it uses the lane's pools, and some of it leaves state in them
     // (empty depth keys and list heads) that the next sequence starts from.
     sgl_status move_to(Ctx *ctx, cudaStream_t st);
-    void recorded(cudaEvent_t event); // `event` was recorded after the lane's newest work
+    // `event` was recorded after the lane's newest work; false under capture,
+    // where nothing outside the graph can wait for it.
+    bool recorded(cudaEvent_t event);
+    // The slot that the next prepare takes, -1 when graphs hold them all.
+    int free_slot() const;
     // Stage and copy the descriptors of a batch into a free slot; returns its index.
     sgl_status prepare(Ctx *ctx, const BatchEntry *e, int n, int tile, int inline_span, uint8_t *slot_flags,
                        int *slot_out);

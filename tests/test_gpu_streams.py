@@ -44,34 +44,43 @@ def test_alternating_streams_equal_single_frames(batched):
     r.close()
 
 
-def test_calls_after_a_captured_batch():
+@pytest.mark.parametrize("posed", [False, True])
+def test_calls_after_a_captured_batch(posed):
     """A batch captured into a caller's graph (direct launches) between calls
-    on other streams: those go on as before, and the replay draws the frame."""
+    on other streams: those go on as before, however many, and the replay
+    draws the frame, also after them."""
     import torch
 
     from swegl_gb300.runtime import Renderer
 
     r = Renderer(0)
-    sid = r.upload(S.cube_scene())
-    v = S.cube_view(320, 240)
+    scene = S.cube_scene()
+    sid = r.upload(scene)
+    v, other = S.cube_view(320, 240), S.cube_view(320, 240)
+    m, c = S.look_at((2.0, 1.5, 3.0), (0.0, 0.0, 0.0))
+    other.view, other.camera_pos = m, c
+    nodes = abi.SceneDescHolder(scene).nodes if posed else None
     pix = torch.zeros((240, 320), dtype=torch.int32, device="cuda")
     z = torch.zeros((240, 320), dtype=torch.float32, device="cuda")
     t = abi.Target(pix.data_ptr(), 1280, 320, 240, C.cast(C.c_void_p(z.data_ptr()), C.POINTER(C.c_float)))
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
-    r.render_batch([(sid, v, t)], use_graph=False, stream=a.cuda_stream)
-    torch.cuda.synchronize()
-    expect = pix.clone()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph, stream=b, capture_error_mode="thread_local"):
-        r.render_batch([(sid, v, t)], use_graph=False, stream=b.cuda_stream)
-    pix.zero_()
-    graph.replay()
-    torch.cuda.synchronize()
-    assert torch.equal(pix, expect)
-    for stream in (a, b):
+
+    def frame(view, stream):
         pix.zero_()
         torch.cuda.synchronize()
-        r.render_batch([(sid, v, t)], use_graph=False, stream=stream.cuda_stream)
+        r.render_batch([(sid, view, t, nodes)], use_graph=False, stream=stream.cuda_stream)
         torch.cuda.synchronize()
-        assert torch.equal(pix, expect)
+        return pix.clone()
+
+    expect, expect_other = frame(v, a), frame(other, a)
+    graph = torch.cuda.CUDAGraph()
+    # (a slot's first poses allocate their staging)
+    with torch.cuda.graph(graph, stream=b, capture_error_mode="relaxed" if posed else "thread_local"):
+        r.render_batch([(sid, v, t, nodes)], use_graph=False, stream=b.cuda_stream)
+    for k in range(10):
+        pix.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(pix, expect), k
+        assert torch.equal(frame(other, (a, b)[k % 2]), expect_other), k
     r.close()
